@@ -34,7 +34,7 @@ def _nvcc() -> str:
 
 
 def _headers() -> list[str]:
-    return glob.glob(os.path.join(CSRC, '*.h')) + glob.glob(os.path.join(INCLUDE, '*.h'))
+    return [h for pattern in ('*.h', '*.cuh') for h in glob.glob(os.path.join(CSRC, pattern))] + glob.glob(os.path.join(INCLUDE, '*.h'))
 
 
 def _command(source: str, obj: str) -> list[str]:

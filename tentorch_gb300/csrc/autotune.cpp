@@ -108,7 +108,7 @@ namespace ttg
     bool tensor = false;
     if (precision > 0 && !complex)
       for (const Op &op : p.ops)
-        if (op.kind == OpKind::gemm && split_tc_suits(p, op, precision)) tensor = true;
+        if (op.kind == OpKind::gemm && split_tc_large(p, op, precision)) tensor = true;
     if (tensor)
     {
       const size_t n = out.size();

@@ -72,19 +72,17 @@ namespace ttg
       int32_t *cta_begin = nullptr;  // per CTA, the start of its list of items (n_ctas + 1 entries)
       int32_t n_ctas = 0;
       int64_t longest = 0;
-      void *items = nullptr, *pairs = nullptr, *lines = nullptr;
+      void *items = nullptr, *pairs = nullptr, *groups = nullptr;
       GemmReduce *reduces = nullptr;
-      int64_t n_items = 0, n_reduces = 0, n_lines_a = 0, n_lines_b = 0, slice_a = 0, slice_b = 0, exps_a = 0, exps = 0,
-              slots = 0;
+      int64_t n_items = 0, n_reduces = 0, n_groups_a = 0, n_groups_b = 0, slice_a = 0, slice_b = 0, exps_a = 0, exps = 0,
+              slots = 0, partial_bytes = 0, longest_line = 0;
     };
-    // the tile lists of split products on the tensor cores (split_tc.cu), built on first use
+    // the tile lists of split products on the tensor cores (split_tc.cu), in the split tables' allocation
     struct TcTables
     {
-      bool ready = false;
-      void *base = nullptr;
       void *items = nullptr;
-      int32_t *cta_begin = nullptr;
-      int32_t n_ctas = 0;
+      GemmReduce *reduces = nullptr;
+      int32_t n_ctas = 0, longest = 0, n = 0;
     };
     std::vector<GemmTables> gemm;
     std::vector<SplitTables> split;
@@ -188,13 +186,14 @@ namespace ttg
   };
   cudaError_t launch_chain_batch(const std::vector<ChainBatchEntry> &entries, cudaStream_t stream, bool *used);
   void clear_chain_batches();
-  // Split products on the tensor cores (split_tc.cu): whether an op's blocks fill its 128 x 64 tiles
-  // well enough, and the launch (slices and exponents as launch_gemm_split lays them out; `error`
-  // an int of the workspace's ticket region, raised when a wait gives up).
-  bool split_tc_suits(const Program &p, const Op &op, int32_t slices);
-  cudaError_t launch_split_tc(const Program &p, const Op &op, DeviceTables &t, size_t op_index, int32_t slices,
+  // Split products on the tensor cores (split_tc.cu): whether an op's blocks are large enough that the
+  // autotuner times them on mma.sync too, and the launch (slices and exponents as launch_gemm_split
+  // lays them out; partial tiles in `partial`, tickets and at their end an error flag, raised when a
+  // wait gives up, in `tickets`).
+  bool split_tc_large(const Program &p, const Op &op, int32_t slices);
+  cudaError_t launch_split_tc(const DeviceTables &t, size_t op_index, int32_t slices,
                               const uint16_t *sa, const uint16_t *sb, const int16_t *exps_a, const int16_t *exps_b,
-                              int64_t stride_a, int64_t stride_b, const void *spairs, double *C, int *error,
+                              const void *spairs, double *C, double *partial, int *tickets, const int32_t *relabel,
                               cudaStream_t stream);
   // The plain per-block form (per_block.cu): one cuBLAS call per block pair.
   cudaError_t launch_gemm_per_block(const Program &p, const Op &op, const void *A, const void *B, void *C, bool complex,

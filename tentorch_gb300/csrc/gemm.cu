@@ -169,11 +169,24 @@ namespace ttg
   {
     SplitSchedule s;
     if (full) s.pairs.assign(p.gemm_pairs.size(), SplitPair{0, 0, 0, 0, 0, 0});
-    // slices: every distinct left block as rows of K padded to 32, every distinct right block
-    // transposed the same way; exponents: one per row of A, one per column of B
+    // slices: every distinct left block's rows, every distinct right block's columns, in the layout of
+    // SplitPair; exponents: one per row of A, one per column of B
     std::map<int64_t, std::pair<int64_t, int32_t>> a_at, b_at;  // arena offset -> (slice offset, exponent base)
     const auto pad32 = [](int64_t k) { return (k + kSplitStepK - 1) / kSplitStepK * kSplitStepK; };
-    std::vector<SplitLine> b_lines;
+    std::vector<SplitGroup> b_groups;
+    const auto cut = [full](std::vector<SplitGroup> &out, int64_t src, int64_t base, int32_t lines, int32_t len, int32_t line_step,
+                            int32_t entry_step, int32_t tile, int32_t exp)
+    {
+      const int32_t ksteps = (len + kSplitStepK - 1) / kSplitStepK;
+      for (int32_t l = 0; full && l < lines; l += 8)
+      {
+        SplitGroup g{src + static_cast<int64_t>(l) * line_step, 0, len, line_step, entry_step, std::min(8, lines - l), exp + l, 0, 0, 0};
+        g.dst = slice_place(base, lines, ksteps, tile, l, 0, g.slice_stride);
+        g.step_stride = kMaxSlices * g.slice_stride;
+        out.push_back(g);
+      }
+      return static_cast<int64_t>((lines + 7) / 8) * ksteps * kMaxSlices * kSliceGroup;
+    };
     for (int64_t bi = op.begin; bi < op.begin + op.count; ++bi)
     {
       const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(bi)];
@@ -181,40 +194,34 @@ namespace ttg
       {
         const size_t pi = static_cast<size_t>(blk.pair_begin + k);
         const GemmPair &pr = p.gemm_pairs[pi];
-        const int64_t kp = pad32(pr.k);
+        s.longest_line = std::max<int64_t>(s.longest_line, pr.k);
         auto fa = a_at.find(pr.a);
         if (fa == a_at.end())
         {
           fa = a_at.emplace(pr.a, std::make_pair(s.slice_a, static_cast<int32_t>(s.exps_a))).first;
-          for (int32_t r = 0; full && r < blk.m; ++r)
-            s.lines.push_back({pr.a + static_cast<int64_t>(r) * pr.k, s.slice_a + r * kp, pr.k, 1, static_cast<int32_t>(kp),
-                               static_cast<int32_t>(s.exps_a + r)});
-          s.slice_a += (blk.m * kp + 63) / 64 * 64;
+          s.slice_a += cut(s.groups, pr.a, s.slice_a, blk.m, pr.k, pr.k, 1, kSliceTileA, static_cast<int32_t>(s.exps_a));
           s.exps_a += blk.m;
         }
         auto fb = b_at.find(pr.b);
         if (fb == b_at.end())
         {
           fb = b_at.emplace(pr.b, std::make_pair(s.slice_b, static_cast<int32_t>(s.exps_b))).first;
-          for (int32_t c = 0; full && c < blk.n; ++c)
-            b_lines.push_back({pr.b + c, s.slice_b + c * kp, pr.k, blk.n, static_cast<int32_t>(kp),
-                               static_cast<int32_t>(s.exps_b + c)});
-          s.slice_b += (blk.n * kp + 63) / 64 * 64;
+          s.slice_b += cut(b_groups, pr.b, s.slice_b, blk.n, pr.k, 1, blk.n, kSliceTileB, static_cast<int32_t>(s.exps_b));
           s.exps_b += blk.n;
         }
         if (full)
-          s.pairs[pi] = SplitPair{fa->second.first, fb->second.first, static_cast<int32_t>(kp), fa->second.second,
-                                  fb->second.second, 0};
+          s.pairs[pi] = SplitPair{fa->second.first, fb->second.first, static_cast<int32_t>(pad32(pr.k) / kSplitStepK),
+                                  fa->second.second, fb->second.second, 0};
       }
     }
     s.exps = s.exps_a + s.exps_b;
-    s.lines_a = static_cast<int64_t>(s.lines.size());
-    s.lines.insert(s.lines.end(), b_lines.begin(), b_lines.end());
+    s.groups_a = static_cast<int64_t>(s.groups.size());
+    s.groups.insert(s.groups.end(), b_groups.begin(), b_groups.end());
     // items: one pair's K range each (a multiple of 32), about two per worker, never below a tile
     // over 256 of K (one exact level chunk: smaller items cost more in folds and partial tiles than
     // they gain in spread; at bond 512 the split matvec took 147 us with 128 and 123 us with 256)
     const double target =
-      std::max(op_work(p, op) / (p.ctas * kSplitWorkers * 2.0), static_cast<double>(kSplitTileM) * kSplitTileN * kExactChunk);
+      std::max(op_work(p, op) / (p.ctas * kSplitWorkers * 2.0), static_cast<double>(kSplitTileM) * kSplitTileN * kSplitChunk);
     struct Sized
     {
       SplitItem item;
@@ -231,7 +238,7 @@ namespace ttg
           // a warp's 16 x 16 quarter outside the block skips its products
           const double quarters = std::ceil(rows / 16.0) * std::ceil(cols / 16.0);
           const auto cost = [quarters](double k)
-          { return quarters * 256.0 * (std::ceil(k / kSplitStepK) * kSplitStepK + 2.0 * kSplitStepK * (std::ceil(k / kExactChunk) + 1.0)); };
+          { return quarters * 256.0 * (std::ceil(k / kSplitStepK) * kSplitStepK + 2.0 * kSplitStepK * (std::ceil(k / kSplitChunk) + 1.0)); };
           tile.clear();
           for (int32_t k = 0; k < blk.pair_count; ++k)
           {
@@ -299,11 +306,16 @@ namespace ttg
 
   namespace
   {
-    // bytes of split scratch: slices of A and of B (bf16), exponents (int16), partial tiles, tickets
-    int64_t split_bytes(const SplitSchedule &s, int slices)
+    // bytes of the partial tiles of either form of the split products
+    int64_t split_partial_bytes(const SplitSchedule &s, const TcSchedule &tc)
     {
-      return up256(2 * slices * s.slice_a) + up256(2 * slices * s.slice_b) + up256(2 * s.exps) +
-             up256(s.slots * kSplitTileM * kSplitTileN * 8) + up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
+      return up256(std::max<int64_t>(s.slots * kSplitTileM * kSplitTileN * 8, tc.slots * kSliceTileA * tc.n * 8));
+    }
+    // bytes of split scratch: slices of A and of B (bf16), exponents (int16), partial tiles, tickets
+    int64_t split_bytes(const SplitSchedule &s, const TcSchedule &tc)
+    {
+      return up256(2 * s.slice_a) + up256(2 * s.slice_b) + up256(2 * s.exps) + split_partial_bytes(s, tc) +
+             up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
     }
     // bytes of FP64 scratch: partial tiles (two doubles an entry for complex), tickets
     int64_t f64_bytes(const GemmSchedule &s)
@@ -357,7 +369,7 @@ namespace ttg
         need = std::max(need, (up256(p.chain_slots * kF64TileM * kF64TileN * 8) + 7) / 8);
       }
       const SplitSchedule sizes = schedule_split(p, op, false);
-      need = std::max(need, (split_bytes(sizes, kMaxSlices) + 7) / 8);
+      need = std::max(need, (split_bytes(sizes, schedule_tc(p, op)) + 7) / 8);
       // the slices of a prepared operand's value go into its arena
       for (int side = 0; side < 2; ++side)
       {
@@ -378,8 +390,8 @@ namespace ttg
         c.operand = operand;
         c.offset = plans->prepared_bytes[static_cast<size_t>(operand)];
         const int64_t slice = side == 0 ? sizes.slice_a : sizes.slice_b, exps = side == 0 ? sizes.exps_a : sizes.exps_b;
-        c.exps_offset = c.offset + up256(2 * kMaxSlices * slice);
-        c.bytes = up256(2 * kMaxSlices * slice) + up256(2 * exps);
+        c.exps_offset = c.offset + up256(2 * slice);
+        c.bytes = up256(2 * slice) + up256(2 * exps);
         plans->prepared_bytes[static_cast<size_t>(operand)] += c.bytes;
         (side == 0 ? plans->cache_a : plans->cache_b)[i] = static_cast<int32_t>(plans->caches.size());
         plans->caches.push_back(c);
@@ -398,9 +410,16 @@ namespace ttg
     // After a worker has written a partial tile: take the tile's ticket; the worker holding the last
     // ticket sums every partial of the tile in slot order into C.  The fences order the partial
     // writes before the ticket and the ticket before the reads (reads bypass L1).
-    template <typename T, int BM, int BN>
+    // `scale` gives an entry of the tile from its sum.
+    struct Unscaled
+    {
+      template <typename T>
+      __device__ T operator()(T v, const DevBlock &, int, int) const { return v; }
+    };
+    template <typename T, int BM, int BN, typename Scale = Unscaled>
     __device__ void finish_partial(int worker, int lt, int *flag, int *tickets, const GemmReduce *reduces, int reduce,
-                                   const DevBlock *blocks, const T *partial, T *C, const int32_t *relabel = nullptr)
+                                   const DevBlock *blocks, const T *partial, T *C, const int32_t *relabel = nullptr,
+                                   Scale scale = Scale())
     {
       __threadfence();
       worker_sync(worker);
@@ -445,10 +464,11 @@ namespace ttg
         const int gm = r.m0 + e / BN, gn = r.n0 + e % BN;
         if (gm >= blk.m || gn >= blk.n) continue;
         const int64_t at = blk.c + static_cast<int64_t>(gm) * blk.n + gn;
+        const T value = scale(sum[k], blk, gm, gn);
         if (!relabel)
-          C[at] = sum[k];
+          C[at] = value;
         else if (relabel[at] >= 0)
-          C[relabel[at]] = sum[k];  // straight to its place after the leg move that follows
+          C[relabel[at]] = value;  // straight to its place after the leg move that follows
       }
       const int64_t entries = static_cast<int64_t>(blk.m) * blk.n;
       if (!relabel && lt == 0 && r.m0 + BM >= blk.m && r.n0 + BN >= blk.n && (entries & 1)) C[blk.c + entries] = zero_t<T>();
@@ -700,116 +720,110 @@ namespace ttg
     // split precision
     // ---------------------------------------------------------------------------------------
 
-    // One warp per line (a row of A or a column of B), lines of A from `a` and lines of B from `b`:
-    // the power of two 2^e that bounds the line, then each entry as the integer round(x 2^(56-e))
-    // cut into `slices` balanced 7-bit digits (|q_1| <= 128, |q_t| <= 64 after it), exact in bf16,
-    // written to a row padded with zeros to a multiple of 32.  Loads are issued eight at a time.
-    constexpr int kLineHeld = 16;  // entries a lane holds of a line sliced in one pass (lines <= 512)
+    // One CTA per group of eight lines (rows of A, columns of B): the power of two 2^e that bounds each
+    // line, then each entry as the integer round(x 2^(56-e)) cut into `slices` balanced 7-bit digits
+    // (|q_1| <= 128, |q_t| <= 64 after it), exact in bf16, into the layout of SplitPair, zeros past the
+    // line's end.  A thread takes eight consecutive entries of one line, so that it writes 16 bytes a
+    // slice, a warp 512 contiguous ones; consecutive threads are consecutive lines, so that the columns
+    // of B, neighbours in memory, are read in runs of 64 bytes.  The first kHeld runs of a thread stay in
+    // registers between the maximum and the cut (lines of up to 512 with 256 threads); the rest are read
+    // again.  Bound by the bytes it reads and writes.
+    constexpr int kHeld = 2;
 
-    __global__ void split_lines_kernel(const double *__restrict__ a, const double *__restrict__ b,
-                                       uint16_t *__restrict__ slices_a, uint16_t *__restrict__ slices_b,
-                                       int16_t *__restrict__ exps_a, int16_t *__restrict__ exps_b, int64_t stride_a,
-                                       int64_t stride_b, const SplitLine *__restrict__ lines, int64_t lines_a,
-                                       int64_t line_begin, int64_t line_end, int slices_n)
+    __global__ void __launch_bounds__(256)
+      split_groups_kernel(const double *__restrict__ a, const double *__restrict__ b, uint16_t *__restrict__ slices_a,
+                          uint16_t *__restrict__ slices_b, int16_t *__restrict__ exps_a, int16_t *__restrict__ exps_b,
+                          const SplitGroup *__restrict__ groups, int64_t groups_a, int64_t group_begin, int slices_n)
     {
+      __shared__ unsigned long long most[8][8];
+      // the table is read while the kernel before still runs
+      const int64_t at = group_begin + blockIdx.x;
+      const SplitGroup g = groups[at];
       dependent_entry();
-      const int lane = threadIdx.x & 31;
-      const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-      const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-      for (int64_t l = line_begin + warp; l < line_end; l += warps)
+      const bool left = at < groups_a;
+      const int line = threadIdx.x & 7, first = threadIdx.x >> 3, runs = blockDim.x >> 3;
+      const bool live = line < g.lines;
+      const double *src = (left ? a : b) + g.src + static_cast<int64_t>(line) * g.line_step;
+      uint16_t *dst = (left ? slices_a : slices_b) + g.dst + line * 8;
+      const int total = (g.len + kSplitStepK - 1) / kSplitStepK * (kSplitStepK / 8);  // runs of a line, padding among them
+      const auto read = [&](int run, double (&x)[8])
       {
-        const SplitLine line = lines[l];
-        const bool left = l < lines_a;
-        const double *src = (left ? a : b) + line.src;
-        uint16_t *dst = (left ? slices_a : slices_b) + line.dst;
-        int16_t *exps = left ? exps_a : exps_b;
-        const int64_t stride = left ? stride_a : stride_b;
-        const auto cut = [&](int i, long long r)
-        {
-          for (int t = 0; t < slices_n; ++t)
-          {
-            const int shift = 49 - 7 * t;  // digit t weighs 2^(49 - 7t) of the 2^56 scale
-            long long q;
-            if (shift > 0)
-            {
-              q = (r + (1ll << (shift - 1))) >> shift;  // nearest integer, halves up
-              r -= q << shift;
-            }
-            else
-              q = r;
-            // |q| <= 128: exact in bf16, converted through int32 and fp32
-            dst[t * stride + i] = __bfloat16_as_ushort(__float2bfloat16_rn(__int2float_rn(static_cast<int>(q))));
-          }
-        };
-        if (line.padded <= 32 * kLineHeld)
-        {
-          // the whole line in registers, all its loads in flight at once: one round trip to memory
-          // for the maximum and the digits together
-          double v[kLineHeld];
-          unsigned long long big = 0;
 #pragma unroll
-          for (int u = 0; u < kLineHeld; ++u)
-          {
-            const int i = u * 32 + lane;
-            v[u] = i < line.len ? src[static_cast<int64_t>(i) * line.src_stride] : 0.0;
-            const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v[u])) & 0x7fffffffffffffffull;
-            big = bits > big ? bits : big;
-          }
-          for (int off = 16; off > 0; off >>= 1)
-          {
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, big, off);
-            big = o > big ? o : big;
-          }
-          const int e = frexp_exponent(big);
-          if (lane == 0) exps[line.exp] = static_cast<int16_t>(e);
-#pragma unroll
-          for (int u = 0; u < kLineHeld; ++u)
-          {
-            const int i = u * 32 + lane;
-            if (i < line.padded) cut(i, i < line.len ? scaled_integer(v[u], 56 - e) : 0ll);
-          }
-          continue;
+        for (int j = 0; j < 8; ++j)
+        {
+          const int k = run * 8 + j;
+          x[j] = live && k < g.len ? src[static_cast<int64_t>(k) * g.entry_step] : 0.0;
         }
-        // the largest |entry| by its bits (positive doubles order as integers), then its frexp
-        // exponent e: every |entry| < 2^e
-        unsigned long long big = 0;
-        for (int i0 = 0; i0 < line.len; i0 += 256)
+      };
+      unsigned long long big = 0;
+      const auto larger = [&](const double (&x)[8])
+      {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
         {
-          unsigned long long v[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-          {
-            const int i = i0 + u * 32 + lane;
-            v[u] = i < line.len ? (static_cast<unsigned long long>(__double_as_longlong(src[static_cast<int64_t>(i) * line.src_stride])) &
-                                   0x7fffffffffffffffull)
-                                : 0ull;
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u) big = v[u] > big ? v[u] : big;
+          // the largest |entry| by its bits (positive doubles order as integers)
+          const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(x[j])) & 0x7fffffffffffffffull;
+          big = bits > big ? bits : big;
         }
-        for (int off = 16; off > 0; off >>= 1)
+      };
+      // (zeros, and no reads, past the line's end: every read of the thread is in flight together)
+      double held[kHeld][8];
+#pragma unroll
+      for (int h = 0; h < kHeld; ++h) read(first + h * runs, held[h]);
+#pragma unroll
+      for (int h = 0; h < kHeld; ++h) larger(held[h]);
+      for (int run = first + kHeld * runs; run < total; run += runs)
+      {
+        double x[8];
+        read(run, x);
+        larger(x);
+      }
+#pragma unroll
+      for (int off = 8; off < 32; off <<= 1)
+      {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, big, off);
+        big = o > big ? o : big;
+      }
+      if ((threadIdx.x & 31) < 8) most[threadIdx.x >> 5][line] = big;
+      __syncthreads();
+      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) big = most[w][line] > big ? most[w][line] : big;
+      // its frexp exponent e: every |entry| < 2^e
+      const int e = frexp_exponent(big);
+      if (live && first == 0) (left ? exps_a : exps_b)[g.exp + line] = static_cast<int16_t>(e);
+      const auto cut = [&](int run, const double (&x)[8])
+      {
+        // the integer plus half a unit of each of the eight digits: digit t is then a field of seven bits,
+        // 64 too large but for the first (balanced digits with all their carries taken at once)
+        constexpr long long half = 0x0001020408102040ll;  // sum over t < 7 of 2^(48 - 7 t)
+        long long r[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) r[j] = scaled_integer(x[j], 56 - e) + half;
+        uint16_t *out = dst + static_cast<int64_t>(run >> 2) * g.step_stride + (run & 3) * 64;
+#pragma unroll
+        for (int t = 0; t < kMaxSlices; ++t)
         {
-          const unsigned long long o = __shfl_xor_sync(0xffffffffu, big, off);
-          big = o > big ? o : big;
-        }
-        const int e = frexp_exponent(big);
-        if (lane == 0) exps[line.exp] = static_cast<int16_t>(e);
-        for (int i0 = 0; i0 < line.padded; i0 += 128)
-        {
-          long long x[4];
+          if (t >= slices_n) break;
+          uint32_t word[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
+          for (int j = 0; j < 8; ++j)
           {
-            const int i = i0 + u * 32 + lane;
-            x[u] = i < line.len ? scaled_integer(src[static_cast<int64_t>(i) * line.src_stride], 56 - e) : 0ll;
+            const int q = t == 0 ? static_cast<int>(r[j] >> 49) : static_cast<int>((r[j] >> (49 - 7 * t)) & 127) - 64;
+            // |q| <= 128: the fp32 of 12582912 + q holds q in its last bits, and q is exact in bf16
+            const uint32_t f = __float_as_uint(__int_as_float(0x4b400000 + q) - 12582912.0f) >> 16;
+            word[j >> 1] = j & 1 ? word[j >> 1] | f << 16 : f;
           }
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-          {
-            const int i = i0 + u * 32 + lane;
-            if (i < line.padded) cut(i, x[u]);
-          }
+          *reinterpret_cast<uint4 *>(out + static_cast<int64_t>(t) * g.slice_stride) = make_uint4(word[0], word[1], word[2], word[3]);
         }
+      };
+      if (!live) return;
+#pragma unroll
+      for (int h = 0; h < kHeld; ++h)
+        if (first + h * runs < total) cut(first + h * runs, held[h]);
+      for (int run = first + kHeld * runs; run < total; run += runs)
+      {
+        double x[8];
+        read(run, x);
+        cut(run, x);
       }
     }
 
@@ -825,8 +839,7 @@ namespace ttg
     template <int S>
     __global__ void __launch_bounds__(kSplitWorkers * kWorkerThreads, 1)
       gemm_split_kernel(const uint16_t *__restrict__ sa_all, const uint16_t *__restrict__ sb_all,
-                        const int16_t *__restrict__ exps_a, const int16_t *__restrict__ exps_b, int64_t stride_a,
-                        int64_t stride_b, double *__restrict__ C,
+                        const int16_t *__restrict__ exps_a, const int16_t *__restrict__ exps_b, double *__restrict__ C,
                         const DevBlock *__restrict__ blocks, const DevSplitPair *__restrict__ spairs,
                         const SplitItem *__restrict__ items, const int32_t *__restrict__ cta_begin, const GemmReduce *__restrict__ reduces,
                         int64_t n_reduces, double *__restrict__ partial, int *__restrict__ tickets,
@@ -859,22 +872,24 @@ namespace ttg
         {
           const DevSplitPair sp = spairs[it.pair];
           const int rows = min(kSplitTileM, blk.m - it.m0), cols = min(kSplitTileN, blk.n - it.n0);
-          const uint16_t *ga = sa_all + sp.sa + static_cast<int64_t>(it.m0) * sp.kp;
-          const uint16_t *gb = sb_all + sp.sb + static_cast<int64_t>(it.n0) * sp.kp;
           const auto load = [&](int stage, int k) {
+            int32_t stride_a, stride_b;
+            const uint16_t *ga = sa_all + slice_place(sp.sa, blk.m, sp.ksteps, kSliceTileA, it.m0, k / kSplitStepK, stride_a);
+            const uint16_t *gb = sb_all + slice_place(sp.sb, blk.n, sp.ksteps, kSliceTileB, it.n0, k / kSplitStepK, stride_b);
+            const auto piece = [](int r, int q) { return (r >> 3) * kSliceGroup + q * 64 + (r & 7) * 8; };
             for (int c = lt; c < S * kSplitTileM * 4; c += kWorkerThreads)
             {
               const int t = c / (kSplitTileM * 4), r = (c / 4) % kSplitTileM, q = c % 4;
               const bool ok = r < rows;
-              cp_async16(sA + ((stage * S + t) * kSplitTileM + r) * kRow + q * 8,
-                         ga + t * stride_a + static_cast<int64_t>(ok ? r : 0) * sp.kp + k + q * 8, ok ? 16 : 0);
+              cp_async16(sA + ((stage * S + t) * kSplitTileM + r) * kRow + q * 8, ga + (ok ? t * stride_a + piece(r, q) : 0),
+                         ok ? 16 : 0);
             }
             for (int c = lt; c < S * kSplitTileN * 4; c += kWorkerThreads)
             {
               const int u = c / (kSplitTileN * 4), r = (c / 4) % kSplitTileN, q = c % 4;
               const bool ok = r < cols;
-              cp_async16(sB + ((stage * S + u) * kSplitTileN + r) * kRow + q * 8,
-                         gb + u * stride_b + static_cast<int64_t>(ok ? r : 0) * sp.kp + k + q * 8, ok ? 16 : 0);
+              cp_async16(sB + ((stage * S + u) * kSplitTileN + r) * kRow + q * 8, gb + (ok ? u * stride_b + piece(r, q) : 0),
+                         ok ? 16 : 0);
             }
             cp_async_commit();
           };
@@ -928,7 +943,7 @@ namespace ttg
                 }
             }
             worker_sync(worker);
-            if ((step + 1) % (kExactChunk / kSplitStepK) == 0 || step + 1 == steps)
+            if ((step + 1) % (kSplitChunk / kSplitStepK) == 0 || step + 1 == steps)
             {
               // the four leading levels are exact integers (below 2^24 over a chunk of <= 256 of K):
               // combined exactly in int64 as sum_l lev_l 2^(7 (3 - l)); the rest in fp32
@@ -951,15 +966,16 @@ namespace ttg
                 }
             }
           }
-          // one FP64 step per entry: head 2^-35 + tail 2^-42, times the row and column scales
+          // one FP64 step per entry, and the row and column scales unless several items share the K of
+          // the block's only pair
+          const bool last = it.slot < 0 || blk.pair_count != 1;
 #pragma unroll
           for (int ns = 0; ns < 2; ++ns)
 #pragma unroll
             for (int q = 0; q < 4; ++q)
             {
-              const int ex = (q < 2 ? er0 : er1) + ec[ns][q & 1];
-              acc[ns][q] = fma(static_cast<double>(acc_int[ns][q]), pow2(ex - 35),
-                               static_cast<double>(acc_tail[ns][q]) * pow2(ex - 42));
+              const double x = level_sum(acc_int[ns][q], acc_tail[ns][q]);
+              acc[ns][q] = last ? scaled(x, (q < 2 ? er0 : er1) + ec[ns][q & 1]) : x;
             }
         }
         if (it.slot >= 0)
@@ -970,8 +986,13 @@ namespace ttg
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               out[(wm * 16 + g + (q >= 2 ? 8 : 0)) * kSplitTileN + wn * 16 + ns * 8 + tig * 2 + (q & 1)] = acc[ns][q];
-          finish_partial<double, kSplitTileM, kSplitTileN>(worker, lt, flags + worker, tickets, reduces, it.reduce, blocks,
-                                                           partial, C, relabel);
+          finish_partial<double, kSplitTileM, kSplitTileN>(
+            worker, lt, flags + worker, tickets, reduces, it.reduce, blocks, partial, C, relabel,
+            [&](double v, const DevBlock &b, int gm, int gn) {
+              if (b.pair_count != 1) return v;
+              const DevSplitPair sp = spairs[b.pair_begin];
+              return scaled(v, exps_a[sp.ea + gm] + exps_b[sp.eb + gn]);
+            });
           continue;
         }
 #pragma unroll
@@ -1006,8 +1027,7 @@ namespace ttg
     }
 
     template <int S>
-    cudaError_t launch_split_s(const uint16_t *sa, const uint16_t *sb, const int16_t *exps_a, const int16_t *exps_b,
-                               int64_t stride_a, int64_t stride_b, double *C, const DevBlock *blocks, const DevSplitPair *spairs,
+    cudaError_t launch_split_s(const uint16_t *sa, const uint16_t *sb, const int16_t *exps_a, const int16_t *exps_b, double *C, const DevBlock *blocks, const DevSplitPair *spairs,
                                const SplitItem *items, const int32_t *cta_begin, int32_t n_ctas, int64_t longest,
                                const GemmReduce *reduces, int64_t n_reduces, double *partial, int *tickets,
                                const int32_t *relabel, cudaStream_t stream)
@@ -1019,7 +1039,7 @@ namespace ttg
       // one CTA per list the schedule dealt, as many workers as its longest list needs
       const int workers = static_cast<int>(std::clamp<int64_t>(longest, 1, kSplitWorkers));
       return launch_dependent(gemm_split_kernel<S>, n_ctas, workers * kWorkerThreads, bytes, stream, sa, sb, exps_a, exps_b,
-                              stride_a, stride_b, C, blocks, spairs, items, cta_begin, reduces, n_reduces, partial, tickets,
+                              C, blocks, spairs, items, cta_begin, reduces, n_reduces, partial, tickets,
                               relabel);
     }
   } // namespace
@@ -1113,8 +1133,10 @@ namespace ttg
       const SplitSchedule s = schedule_split(p, op, true);
       dst.n_items = static_cast<int64_t>(s.items.size());
       dst.n_reduces = static_cast<int64_t>(s.reduces.size());
-      dst.n_lines_a = s.lines_a;
-      dst.n_lines_b = static_cast<int64_t>(s.lines.size()) - s.lines_a;
+      dst.n_groups_a = s.groups_a;
+      dst.n_groups_b = static_cast<int64_t>(s.groups.size()) - s.groups_a;
+      dst.longest_line = s.longest_line;
+      dst.partial_bytes = split_partial_bytes(s, schedule_tc(p, op));
       dst.slice_a = s.slice_a;
       dst.slice_b = s.slice_b;
       dst.exps_a = s.exps_a;
@@ -1129,24 +1151,29 @@ namespace ttg
       staging.add(s.items, &dst.items);
       staging.add(s.reduces, reinterpret_cast<void **>(&dst.reduces));
       staging.add(s.pairs, &dst.pairs);
-      staging.add(s.lines, &dst.lines);
+      staging.add(s.groups, &dst.groups);
+      DeviceTables::TcTables &tc = t.tc[op_index];
+      const TcSchedule ts = schedule_tc(p, op, &s.pairs);
+      staging.add(ts.items, &tc.items);
+      staging.add(ts.reduces, reinterpret_cast<void **>(&tc.reduces));
+      tc.n_ctas = ts.ctas;
+      tc.longest = ts.longest;
+      tc.n = ts.n;
       const cudaError_t e = staging.commit(&dst.base);
       if (e != cudaSuccess) return e;
       dst.ready = true;
       return cudaSuccess;
     }
 
-    cudaError_t launch_lines(const DeviceTables::SplitTables &sched, const double *A, const double *B, uint16_t *sa,
-                             uint16_t *sb, int16_t *exps_a, int16_t *exps_b, int64_t begin, int64_t end, int slices,
-                             cudaStream_t stream)
+    cudaError_t launch_groups(const DeviceTables::SplitTables &sched, const double *A, const double *B, uint16_t *sa,
+                              uint16_t *sb, int16_t *exps_a, int16_t *exps_b, int64_t begin, int64_t end, int slices,
+                              cudaStream_t stream)
     {
       if (begin >= end) return cudaSuccess;
-      const auto *lines = reinterpret_cast<const SplitLine *>(sched.lines);
-      // a warp per line, two warps per CTA so that the lines spread over every SM
-      return launch_dependent(split_lines_kernel,
-                              static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((end - begin + 1) / 2, device_sms() * 32))),
-                              64, 0, stream, A, B, sa, sb, exps_a, exps_b, sched.slice_a, sched.slice_b, lines,
-                              sched.n_lines_a, begin, end, slices);
+      // threads for a whole line of 8 x 8 entries a thread, four warps at least
+      const int threads = sched.longest_line > 128 ? 256 : 128;
+      return launch_dependent(split_groups_kernel, static_cast<unsigned>(end - begin), threads, 0, stream, A, B, sa, sb, exps_a,
+                              exps_b, static_cast<const SplitGroup *>(sched.groups), sched.n_groups_a, begin, slices);
     }
   } // namespace
 
@@ -1165,9 +1192,9 @@ namespace ttg
       auto *slices = reinterpret_cast<uint16_t *>(base + c.offset);
       auto *exps = reinterpret_cast<int16_t *>(base + c.exps_offset);
       const auto *value = static_cast<const double *>(arena);
-      e = c.side == 0 ? launch_lines(sched, value, nullptr, slices, nullptr, exps, nullptr, 0, sched.n_lines_a, kMaxSlices, stream)
-                      : launch_lines(sched, nullptr, value, nullptr, slices, nullptr, exps, sched.n_lines_a,
-                                     sched.n_lines_a + sched.n_lines_b, kMaxSlices, stream);
+      e = c.side == 0 ? launch_groups(sched, value, nullptr, slices, nullptr, exps, nullptr, 0, sched.n_groups_a, kMaxSlices, stream)
+                      : launch_groups(sched, nullptr, value, nullptr, slices, nullptr, exps, sched.n_groups_a,
+                                      sched.n_groups_a + sched.n_groups_b, kMaxSlices, stream);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1183,22 +1210,16 @@ namespace ttg
     if (sched.n_items == 0) return cudaSuccess;
     char *base = static_cast<char *>(scratch);
     auto *sa = reinterpret_cast<uint16_t *>(base);
-    base += up256(2 * kMaxSlices * sched.slice_a);
+    base += up256(2 * sched.slice_a);
     auto *sb = reinterpret_cast<uint16_t *>(base);
-    base += up256(2 * kMaxSlices * sched.slice_b);
+    base += up256(2 * sched.slice_b);
     auto *exps_a = reinterpret_cast<int16_t *>(base);
     auto *exps_b = exps_a + sched.exps_a;
     base += up256(2 * sched.exps);
     auto *partial = reinterpret_cast<double *>(base);
-    base += up256(sched.slots * kSplitTileM * kSplitTileN * 8);
-    int *tickets = ticket_region;
-    if (sched.n_reduces > kTicketInts)
-    {
-      tickets = reinterpret_cast<int *>(base);
-      if ((e = cudaMemsetAsync(tickets, 0, static_cast<size_t>(sched.n_reduces) * 4, stream)) != cudaSuccess) return e;
-    }
+    base += sched.partial_bytes;
     // a side whose operand's prepared arena the caller holds was cut when the arena was prepared
-    int64_t begin = 0, end = sched.n_lines_a + sched.n_lines_b;
+    int64_t begin = 0, end = sched.n_groups_a + sched.n_groups_b;
     if (p.gemm_plans && prepared)
     {
       const int32_t ca = p.gemm_plans->cache_a[op_index], cb = p.gemm_plans->cache_b[op_index];
@@ -1208,7 +1229,7 @@ namespace ttg
         char *arena = static_cast<char *>(const_cast<void *>(prepared[c.operand]));
         sa = reinterpret_cast<uint16_t *>(arena + c.offset);
         exps_a = reinterpret_cast<int16_t *>(arena + c.exps_offset);
-        begin = sched.n_lines_a;
+        begin = sched.n_groups_a;
       }
       if (cb >= 0 && prepared[p.gemm_plans->caches[static_cast<size_t>(cb)].operand])
       {
@@ -1216,19 +1237,24 @@ namespace ttg
         char *arena = static_cast<char *>(const_cast<void *>(prepared[c.operand]));
         sb = reinterpret_cast<uint16_t *>(arena + c.offset);
         exps_b = reinterpret_cast<int16_t *>(arena + c.exps_offset);
-        end = sched.n_lines_a;
+        end = sched.n_groups_a;
       }
     }
-    if ((e = launch_lines(sched, A, B, sa, sb, exps_a, exps_b, begin, end, slices, stream)) != cudaSuccess) return e;
-    // large blocks: whole 128 x 64 tiles on the tensor cores (tcgen05), no partial tiles
+    if ((e = launch_groups(sched, A, B, sa, sb, exps_a, exps_b, begin, end, slices, stream)) != cudaSuccess) return e;
     static const bool tc_enabled = []
     {
       const char *v = std::getenv("TENTORCH_GB300_TCGEN05");
       return !(v && v[0] == '0');
     }();
-    if (tc_enabled && tensor_cores && !relabel && split_tc_suits(p, op, slices))
-      return launch_split_tc(p, op, t, op_index, slices, sa, sb, exps_a, exps_b, sched.slice_a, sched.slice_b, sched.pairs,
-                             C, ticket_region + kTicketInts - 1, stream);
+    if (tc_enabled && tensor_cores)
+      return launch_split_tc(t, op_index, slices, sa, sb, exps_a, exps_b, sched.pairs, C, partial, ticket_region, relabel,
+                             stream);
+    int *tickets = ticket_region;
+    if (sched.n_reduces > kTicketInts)
+    {
+      tickets = reinterpret_cast<int *>(base);
+      if ((e = cudaMemsetAsync(tickets, 0, static_cast<size_t>(sched.n_reduces) * 4, stream)) != cudaSuccess) return e;
+    }
     const auto *blocks = reinterpret_cast<const DevBlock *>(t.blocks);
     const auto *spairs = reinterpret_cast<const DevSplitPair *>(sched.pairs);
     const auto *items = reinterpret_cast<const SplitItem *>(sched.items);
@@ -1236,7 +1262,7 @@ namespace ttg
     {
 #define TTG_SPLIT(S)                                                                                                    \
   case S:                                                                                                               \
-    e = launch_split_s<S>(sa, sb, exps_a, exps_b, sched.slice_a, sched.slice_b, C, blocks, spairs, items,              \
+    e = launch_split_s<S>(sa, sb, exps_a, exps_b, C, blocks, spairs, items,                                             \
                           sched.cta_begin, sched.n_ctas, sched.longest, sched.reduces, sched.n_reduces, partial, tickets,  \
                           relabel, stream);                                                                             \
     break;

@@ -51,29 +51,38 @@ namespace ttg
   {
     int32_t block, m0, n0, pair, k0, k1, slot, reduce;
   };
-  // Where a pair's slices and exponents sit in scratch: A slices rows of `kp` (K padded to 32),
-  // B slices transposed, one row of `kp` per column.
+  // Where a pair's slices and exponents sit in scratch.  The rows of A and the columns of B ("lines")
+  // are cut into kMaxSlices slices and kept in the order the tensor cores read them: lines in tiles of
+  // kSliceTileA (A) or kSliceTileB (B), K in steps of 32; per tile and step the slices one after
+  // another, each as groups of 8 lines x 32 of K (512 bytes: four runs of 8 lines x 16 bytes, the
+  // core matrices of tcgen05's K-major layout without swizzle).  A tile over one step is then one
+  // contiguous piece a slice, which a bulk copy brings into shared memory as the products read it;
+  // the last tile of a block keeps only the groups it has (slice_place below).
   struct SplitPair
   {
-    int64_t sa, sb;
-    int32_t kp, ea, eb, pad;
+    int64_t sa, sb;  // elements: the first tile of the A lines, of the B lines
+    int32_t ksteps, ea, eb, pad;
   };
-  struct SplitLine
+  // Up to eight lines to slice together.
+  struct SplitGroup
   {
-    int64_t src, dst;
-    int32_t len, src_stride, padded, exp;
+    int64_t src, dst;                   // the first line's first entry; its place in the first step's first slice
+    int32_t len, line_step, entry_step; // entries a line, source elements between lines and between entries
+    int32_t lines, exp;                 // lines in the group, the first one's exponent
+    int32_t slice_stride, step_stride, pad;  // elements between slices, between steps of K
   };
   struct SplitSchedule
   {
     std::vector<SplitItem> items;
     std::vector<GemmReduce> reduces;
-    std::vector<SplitPair> pairs;  // one per GemmPair of the program (only this op's are filled)
-    std::vector<SplitLine> lines;  // rows of A then columns of B
-    int64_t lines_a = 0;
-    int64_t slice_a = 0, slice_b = 0;  // elements of one slice of all A (B) rows
+    std::vector<SplitPair> pairs;    // one per GemmPair of the program (only this op's are filled)
+    std::vector<SplitGroup> groups;  // rows of A then columns of B
+    int64_t groups_a = 0;
+    int64_t slice_a = 0, slice_b = 0;  // elements of all slices of A (B)
     int64_t exps_a = 0, exps_b = 0;    // int16 exponents of the rows of A, of the columns of B
     int64_t exps = 0;                  // both
     int64_t slots = 0;
+    int64_t longest_line = 0;          // the longest K
     std::vector<int32_t> cta_begin;    // CTA b runs items [cta_begin[b], cta_begin[b + 1])
   };
   // The split-precision schedule of a GEMM op; with full = false only its sizes (slices, exponents,
@@ -88,7 +97,50 @@ namespace ttg
   // threads per CTA taking items round robin.
   constexpr int kF64Workers = 4, kSplitWorkers = 2, kWorkerThreads = 128;
   constexpr int kMaxSlices = 8;
-  constexpr int kExactChunk = 256;  // K over which fp32 sums of slice products stay exact
+  // K over which the sums of slice products stay integers of at most 2^24, which fp32 adds exactly:
+  // level l sums 2^12 (l + 3) a K at most (2^14 for l = 0), so 512 holds through level 5.  Levels 6
+  // and 7 weigh 2^-14 and less of level 4, whose rounding theirs stays below.
+  constexpr int kExactChunk = 512;
+  constexpr int kSplitChunk = 256;  // the K after which the mma.sync kernel folds its level sums
+  constexpr int kSliceTileA = 128, kSliceTileB = 64;  // lines of a tile of slices
+  constexpr int kSliceGroup = 8 * 32;                 // elements of eight lines over 32 of K
+
+  // The element of the first slice of line `line` (a multiple of 8) at a step of K, for `lines` lines
+  // starting at `base` in tiles of `tile`; the elements between slices there in `slice_stride`.
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  inline int64_t slice_place(int64_t base, int32_t lines, int32_t ksteps, int32_t tile, int32_t line, int32_t step,
+                             int32_t &slice_stride)
+  {
+    const int32_t t = line / tile, full = tile / 8, left = (lines - t * tile + 7) / 8;
+    const int32_t groups = left < full ? left : full;
+    slice_stride = groups * kSliceGroup;
+    return base + (static_cast<int64_t>(t) * ksteps * full + static_cast<int64_t>(step) * groups) * kMaxSlices * kSliceGroup +
+           static_cast<int64_t>((line - t * tile) / 8) * kSliceGroup;
+  }
+
+  // The work of split products on the tensor cores (split_tc.cu): an item is a 128 x n output tile
+  // over steps [s0, s1) of 32 of K (its block's pairs one after another, each in whole steps).  It
+  // carries its block and first pair, so that a CTA has all it needs of most tiles after one read.
+  struct TcItem
+  {
+    int64_t c, sa, sb;                 // the block's place in C, the first pair's slices (SplitPair)
+    int32_t m, n, m0, n0;              // the block, the tile's corner; m 0 ends a CTA's list
+    int32_t s0, s1, slot, reduce;
+    int32_t pair_begin, pair_count;
+    int32_t k, ksteps, ea, eb;         // the first pair
+  };
+  struct TcSchedule
+  {
+    std::vector<TcItem> items;  // `longest` places a CTA, its list and then items of m 0
+    std::vector<GemmReduce> reduces;
+    int32_t ctas = 0, longest = 0;
+    int32_t n = 64;     // columns of a tile
+    int64_t slots = 0;  // partial tiles of 128 x n doubles
+  };
+  // With `pairs` (the op's, from schedule_split) the whole schedule, else its sizes.
+  TcSchedule schedule_tc(const Program &p, const Op &op, const std::vector<SplitPair> *pairs = nullptr);
 
   // The FP64 schedule of a GEMM op; with full = false only its sizes (items, partial slots,
   // reductions), for sizing the scratch: the items are dealt on the op's first FP64 launch.

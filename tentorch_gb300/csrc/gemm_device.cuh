@@ -28,7 +28,7 @@ namespace ttg
     struct DevSplitPair
     {
       int64_t sa, sb;
-      int32_t kp, ea, eb, pad;
+      int32_t ksteps, ea, eb, pad;
     };
 
     __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c)
@@ -100,29 +100,17 @@ namespace ttg
       return (64 - __clzll(static_cast<long long>(bits))) - 1074;  // subnormal: bits * 2^-1074
     }
 
-    // __double2ll_rn(ldexp(x, k)) for |x| < 2^(63 - k) on the bits of x: the significand shifted by
-    // the exponent, rounded to nearest with ties to even.
+    // __double2ll_rn(ldexp(x, k)) for |x| < 2^(56 - k) on the bits of x: the significand shifted by the
+    // exponent, rounded to nearest with ties to even (no branch: the eight entries of a thread overlap).
     __device__ __forceinline__ long long scaled_integer(double x, int k)
     {
       const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(x));
       const int field = static_cast<int>((bits >> 52) & 0x7ff);
-      unsigned long long mant = bits & 0xfffffffffffffull;
-      if (field != 0) mant |= 1ull << 52;
-      const int shift = (field != 0 ? field : 1) - 1075 + k;  // x 2^k = mant 2^shift
-      unsigned long long q;
-      if (mant == 0)
-        q = 0;
-      else if (shift >= 0)
-        q = mant << shift;
-      else if (shift < -62)
-        q = 0;
-      else
-      {
-        const int down = -shift;
-        q = mant >> down;
-        const unsigned long long rem = mant & ((1ull << down) - 1), half = 1ull << (down - 1);
-        if (rem > half || (rem == half && (q & 1ull))) ++q;
-      }
+      const unsigned long long mant = ((bits & 0xfffffffffffffull) | (field != 0 ? 1ull << 52 : 0ull)) << 3;
+      // x 2^k = mant 2^-down; a value below 2^56 shifts down
+      const int down = min(max(1078 - k - (field != 0 ? field : 1), 0), 62);
+      const unsigned long long half = (1ull << down) >> 1;
+      const unsigned long long q = (mant + (down ? half - 1ull + ((mant >> down) & 1ull) : 0ull)) >> down;
       const long long v = static_cast<long long>(q);
       return (bits >> 63) ? -v : v;
     }
@@ -134,6 +122,34 @@ namespace ttg
       return ldexp(1.0, k);
     }
 
+    // x 2^e, rounded only where the result leaves the normal range.
+    __device__ __forceinline__ double scaled(double x, int e)
+    {
+      const long long bits = __double_as_longlong(x);
+      const int field = static_cast<int>((bits >> 52) & 0x7ff);
+      if (field != 0 && field + e > 0 && field + e < 2047) return __longlong_as_double(bits + (static_cast<long long>(e) << 52));
+      return ldexp(x, e);
+    }
+    // The level sums of a pair as one double, without the row's and the column's scale (taken last, so
+    // that the parts of a K that several workers share are added before it can round them):
+    // head 2^-35 + tail 2^-42, summed exactly in 128 bits and rounded once, with integers (five FP64
+    // instructions an entry took longer than the products of a small tile).
+    __device__ __forceinline__ double level_sum(long long head, float tail)
+    {
+      const __int128 v = (static_cast<__int128>(head) << 28) + __float2ll_rn(tail * 2097152.0f);
+      if (v == 0) return 0.0;
+      const unsigned __int128 u = v < 0 ? -static_cast<unsigned __int128>(v) : static_cast<unsigned __int128>(v);
+      const unsigned long long hi = static_cast<unsigned long long>(u >> 64), lo = static_cast<unsigned long long>(u);
+      const int lz = hi ? __clzll(static_cast<long long>(hi)) : 64 + __clzll(static_cast<long long>(lo));
+      const unsigned __int128 top = u << lz;  // the leading one at bit 127
+      const unsigned long long m = static_cast<unsigned long long>(top >> 64), rest = m & 0x7ffull;
+      const bool sticky = static_cast<unsigned long long>(top) != 0;
+      unsigned long long q = m >> 11;
+      q += (rest > 0x400ull || (rest == 0x400ull && (sticky || (q & 1ull)))) ? 1ull : 0ull;
+      // v 2^-63: exponent 127 - lz - 63, one lower for q's leading one
+      const unsigned long long bits = (static_cast<unsigned long long>(1023 + 64 - lz - 1) << 52) + q;
+      return __longlong_as_double(static_cast<long long>(v < 0 ? bits | 0x8000000000000000ull : bits));
+    }
 
     __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
     {

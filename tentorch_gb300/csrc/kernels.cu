@@ -199,8 +199,6 @@ namespace ttg
     if (base) cudaFree(base);
     if (chain.base) cudaFree(chain.base);
     if (chain.relabel_base) cudaFree(chain.relabel_base);
-    for (TcTables &g : tc)
-      if (g.base) cudaFree(g.base);
     for (GemmTables &g : gemm)
       if (g.base) cudaFree(g.base);
     for (SplitTables &g : split)

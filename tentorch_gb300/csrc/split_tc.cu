@@ -1,26 +1,33 @@
-// Split-precision block products on the 5th-generation tensor cores (tcgen05) for GEMM ops whose
-// blocks are large enough to fill 128 x 64 output tiles (the SU(2) and Fibonacci recouplings, large
-// bonds).  The numerical scheme is the one of gemm.cu (Ozaki's error-free splitting: every row of A
-// and column of B cut into S exact 7-bit bf16 slices, cut once by the slicing pass); what changes is
-// where the slice products run:
+// Split-precision block products on the 5th-generation tensor cores (tcgen05).  The numerical scheme
+// is the one of gemm.h (Ozaki's error-free splitting: every row of A and column of B cut into S exact
+// 7-bit bf16 slices by the slicing pass); this is where the slice products run.
 //
-//   - a CTA (16 warps, one per SM) owns a 128 x 64 output tile and runs every pair of its block over
-//     the whole K, so no tile is split into partial sums;
-//   - K advances 32 at a time through a ring of three shared-memory stages, each holding the S
-//     slices of A (128 x 32) and of B (64 x 32) in the K-major core-matrix layout (8 rows x 16 bytes
-//     per core matrix, no swizzle), filled with 16-byte cp.async;
-//   - one thread issues tcgen05.mma kind::f16 (bf16 x bf16 -> fp32, M = 128, N = 64, K = 16) for
-//     every slice pair (t, u) with t + u < S, into the accumulator of level t + u in tensor memory
-//     (S accumulators of 64 columns: at most 6 x 64 = 384 of the SM's 512 columns); tcgen05.commit
-//     on the stage's mbarrier tells when the stage may be refilled;
-//   - every 256 of K (the level sums are integers below 2^24 that far, so fp32 holds them exactly)
-//     the warps read the levels back with tcgen05.ld (warp w reads lanes 32 (w % 4) .. + 31, the rows
-//     of its quarter, columns 16 (w / 4) .. + 15) and fold them exactly: the four leading levels as
-//     an int64 sum_l lev_l 2^(7 (3 - l)), the rest through one fp32 sum; at the end of a pair one FP64
-//     step per entry applies the row and column scales and adds into the tile's FP64 value.
-// Every wait on an mbarrier gives up after two seconds and raises an error flag; the outcome of every
-// wait is made the same for the whole CTA before anything depends on it, and the CTA frees its
-// tensor memory on every path out.
+//   - A CTA (one per SM) owns 128 x N output tiles, N = 64 or 32, over a range of K.  Warps have
+//     roles: one thread copies, one issues the products, eight warps read the sums back.
+//   - The slicing pass leaves every slice of a tile over 32 of K as one contiguous piece in the
+//     core-matrix layout the products read (8 rows x 16 bytes, K-major, no swizzle; SplitPair), so a
+//     stage is 2 S bulk copies (cp.async.bulk) that signal the stage's mbarrier, in a ring of as
+//     many stages as fit in shared memory.
+//   - The sums of level l = t + u sit in tensor memory at columns l N .. l N + N - 1, and the slices of
+//     B follow one another in a stage, so that slice t of A times ALL the slices u < S - t of B is one
+//     product of N (S - t) columns landing in levels t .. S - 1: eight tcgen05.mma of up to 256 columns
+//     a 16 of K (S = 6) instead of 21 of 64, each reading A from shared memory once.  With 64 columns
+//     a product is bound by shared memory (6 KB in 32 clocks), with 256 by the tensor cores.
+//   - Every 512 of K (gemm.h kExactChunk) the level sums, exact integers, are read back and folded:
+//     the four leading levels as an int64 sum_l lev_l 2^(7 (3 - l)), the rest through one fp32 sum.
+//   - FP64 runs at 2 multiply-adds a clock and SM here, 64 times slower than integers: an FP64
+//     combination per entry would take longer than the products of a tile of K below 1000.  A tile's
+//     value is therefore kept as a fixed-point int64 (head 2^7 + tail with up to 8 more bits) and
+//     becomes a double by shifting, with one rounding; the partial tiles of a K that several CTAs
+//     share add as integers, exactly, in any order.  Blocks of several pairs (their scales differ),
+//     S above 6 and K beyond 2^16 combine in FP64.
+// Measured on the SU(2) recoupling of bond 8 x 9 spins (85.9 GFLOP, S = 6: 1.80 PFLOP of slice products)
+// 1.16 ms, 1.55 PFLOP/s, 0.78 of the measured bf16 peak; as 21 products of 64 columns staged by cp.async
+// from slices a row apart it took 5.99 ms.  The matvec of bond 1001 (both products and their
+// slicing) takes 178 us, 425 on mma.sync.
+// The roles pass stages, level sums and free tensor memory through mbarriers.  Every wait gives up
+// after two seconds or once another has, and raises an error flag; on every path out the copies and
+// products in flight are waited for (again with a limit) and the tensor memory is freed.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -38,43 +45,46 @@ namespace ttg
 {
   namespace
   {
-    constexpr int kTcM = 128, kTcN = 64, kTcK = 32;  // output tile, K per stage
-    constexpr int kTcStages = 3;
-    constexpr int kTcThreads = 512;
-    constexpr int kTcCols = kTcN / (kTcThreads / 128);  // columns of a tile each thread folds and stores
-    constexpr int kTcMaxSlices = 6;
-    constexpr int kTcChunkSteps = kExactChunk / kTcK;  // stages between drains of the level sums
-    // core-matrix layout of one operand slice in a stage: 16 bytes per (row, 8 of K); the 4 groups of
-    // 8 of K of a row group follow one another (LBO), row groups after them (SBO)
-    constexpr int kTcLbo = 128, kTcSbo = (kTcK / 8) * 128;
-    constexpr int kTcSliceA = kTcM * kTcK * 2, kTcSliceB = kTcN * kTcK * 2;  // bytes
+    constexpr int kTcM = kSliceTileA, kTcK = 32;  // rows of a tile, K per stage
+    constexpr int kTcChunkSteps = kExactChunk / kTcK;  // stages between readings of the level sums
+    // core-matrix layout of one slice in a stage: 16 bytes per (row, 8 of K); the 4 groups of 8 of K
+    // of a row group follow one another (LBO), row groups after them (SBO)
+    constexpr int kTcLbo = 128, kTcSbo = kSliceGroup * 2;
+    constexpr int kTcSmem = 216 * 1024;
+    constexpr int kTcFixedSlices = 6;  // the most slices whose sums the fixed-point values hold
+    constexpr int32_t kTcFixedK = 1 << 16;
     constexpr unsigned long long kTcWaitNs = 2000000000ull;
 
-    template <int S>
-    __host__ __device__ constexpr int tc_stage_bytes() { return S * (kTcSliceA + kTcSliceB); }
-    template <int S>
-    __host__ __device__ constexpr int tc_smem_bytes() { return kTcStages * tc_stage_bytes<S>(); }
-    // at least 120 KiB, so that a second CTA never shares the SM (each holds all 512 columns of its
-    // tensor memory)
-    template <int S>
-    constexpr int tc_launch_bytes() { return tc_smem_bytes<S>() > 120 * 1024 ? tc_smem_bytes<S>() : 120 * 1024; }
-
-    struct TcItem
+    // 32 columns: sixteen warps read the sums back, eight columns a thread, so that the latency of a small
+    // tile's end is short.  64 columns: eight, 32 columns a thread, in two warpgroups of 216 registers;
+    // launched with 168 a thread (3 x 128 x 168 of the SM's 65536), the third warpgroup (the copying
+    // and the issuing warp) keeps 56: 2 x 216 + 56 = 488 of the 504 they came with.
+    template <int S, int N>
+    struct TcShape
     {
-      int32_t block, m0, n0, pad;
+      static constexpr int slice_a = kTcM * kTcK * 2, slice_b = N * kTcK * 2;  // bytes
+      static constexpr int stage = S * (slice_a + slice_b);
+      static constexpr int stages = kTcSmem / stage < 6 ? kTcSmem / stage : 6;
+      // more than half of the SM's, so that a second CTA never shares it (each holds all 512 columns of
+      // its tensor memory)
+      static constexpr int bytes = stages * stage > 120 * 1024 ? stages * stage : 120 * 1024;
+      static constexpr int warps = N == 32 ? 16 : 8;      // that read the sums back
+      static constexpr int cols = N / (warps / 4);        // columns of a tile a thread reads back
+      static constexpr int threads = (warps + 4) * 32;
     };
 
     struct TcArgs
     {
-      const uint16_t *sa, *sb;  // slices of A rows and of B columns (gemm.cu's scratch layout)
+      const uint16_t *sa, *sb;  // slices of A rows and of B columns (SplitPair's layout)
       const int16_t *exps_a, *exps_b;
-      int64_t stride_a, stride_b;  // elements between two slices of all A rows (B columns)
       double *c;
-      const DevBlock *blocks;
-      const DevPair *pairs;
+      const int32_t *relabel;   // per entry of C its place after the leg move that follows, or null
       const DevSplitPair *spairs;
       const TcItem *items;
-      const int32_t *cta_begin;
+      const GemmReduce *reduces;
+      int32_t longest;
+      double *partial;
+      int *tickets;
       int *error;
     };
 
@@ -90,14 +100,40 @@ namespace ttg
 
     // kind::f16 instruction descriptor: D fp32, A and B bf16, both K-major, N >> 3 at bit 17, M >> 4
     // at bit 24
-    constexpr uint32_t kTcInstr = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kTcN >> 3) << 17) |
-                                  (static_cast<uint32_t>(kTcM >> 4) << 24);
+    __host__ __device__ constexpr uint32_t tc_instr(int n)
+    {
+      return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(kTcM >> 4) << 24);
+    }
 
-    __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate)
+    __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t instr, uint32_t accumulate)
     {
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                   "l"(a), "l"(b), "r"(kTcInstr), "r"(accumulate));
+                   "l"(a), "l"(b), "r"(instr), "r"(accumulate)
+                   : "memory");
+    }
+    __device__ __forceinline__ void tc_commit(uint64_t *bar)
+    {
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+    }
+    __device__ __forceinline__ void bar_init(uint64_t *bar, int count)
+    {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+    }
+    __device__ __forceinline__ void bar_arrive(uint64_t *bar)
+    {
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+    }
+    __device__ __forceinline__ void bar_expect(uint64_t *bar, uint32_t bytes)
+    {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+    }
+    // bytes (a multiple of 16) of global memory into shared memory, counted on `bar` as they land
+    __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar)
+    {
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                   "r"(bytes), "r"(smem_addr(bar))
+                   : "memory");
     }
 
     __device__ __forceinline__ unsigned long long tc_now()
@@ -107,11 +143,12 @@ namespace ttg
       return t;
     }
 
-    // Wait for the phase of `bar` with parity `parity`; false when two seconds passed first.
-    __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity)
+    // Wait for the phase of `bar` with parity `parity`; false when two seconds passed first, or when
+    // another wait of the CTA has given up (`failed`, null to wait regardless).
+    __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *failed)
     {
       const uint32_t at = smem_addr(bar);
-      const unsigned long long start = tc_now();
+      unsigned long long start = 0;
       while (true)
       {
         uint32_t done;
@@ -120,223 +157,469 @@ namespace ttg
                      : "r"(at), "r"(parity)
                      : "memory");
         if (done) return true;
-        if (tc_now() - start > kTcWaitNs) return false;
+        const unsigned long long now = tc_now();
+        if (start == 0) start = now;
+        if ((failed && *failed) || now - start > kTcWaitNs)
+        {
+          if (failed) *failed = 1;
+          return false;
+        }
       }
     }
 
-    // 16 columns of one lane of tensor memory
-    __device__ __forceinline__ void tc_load16(uint32_t addr, uint32_t (&r)[16])
+    // 8 columns of one lane of tensor memory
+    __device__ __forceinline__ void tc_load8(uint32_t addr, uint32_t *r)
     {
-      asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                     "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                    : "r"(addr));
     }
 
-    template <int S>
-    __global__ void __launch_bounds__(kTcThreads, 1) gemm_split_tc_kernel(TcArgs a)
+    // The bits a fixed-point value of a pair keeps below the unit of level 4: 8, fewer from K = 4096 on
+    // (a value is at most 2^(42 + bits) K).
+    __device__ __forceinline__ int fixed_bits(int k) { return k <= 4096 ? 8 : max(0, 8 - (32 - __clz((k - 1) >> 12))); }
+
+    // v 2^e as a double, rounded once (to nearest, ties to even), when it is in the normal range;
+    // `outside` collects whether it was not (fixed_slow then gives it).
+    __device__ __forceinline__ double fixed_to_double(long long v, int e, bool &outside)
     {
-      dependent_entry();
+      const unsigned long long sign = static_cast<unsigned long long>(v) & 0x8000000000000000ull;
+      const unsigned long long a = static_cast<unsigned long long>(sign ? -v : v);
+      const int lz = min(__clzll(static_cast<long long>(a)), 63), field = 1086 - lz + e;
+      const unsigned long long m = a << lz, rest = m & 0x7ffull;
+      unsigned long long q = m >> 11;
+      q += (rest > 0x400ull || (rest == 0x400ull && (q & 1ull))) ? 1ull : 0ull;
+      outside |= v != 0 && (field <= 0 || field >= 2046);
+      // q has its leading one at bit 52: added to the exponent field one lower, a carry moves it up
+      const unsigned long long bits = ((static_cast<unsigned long long>(field - 1) << 52) + q) | sign;
+      return __longlong_as_double(static_cast<long long>(v == 0 ? 0ull : bits));
+    }
+    __device__ __noinline__ double fixed_slow(long long v, int e) { return ldexp(static_cast<double>(v), e); }
+
+    // The 8 x 8 transpose within each group of eight lanes: lane 8 g + i holds entries 0 .. 7 of row i
+    // of its group and takes entry i of rows 0 .. 7, so that a store of eight lanes is 64 contiguous
+    // bytes instead of eight places a row apart.
+    __device__ __forceinline__ void transpose8(long long *v, int lane)
+    {
+#pragma unroll
+      for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+          if (j & m) continue;
+          const bool high = lane & m;
+          const long long got = __shfl_xor_sync(0xffffffffu, high ? v[j] : v[j | m], m);
+          if (high) v[j] = got;
+          else v[j | m] = got;
+        }
+    }
+
+    // The steps of an item, pair by pair: calls f(pair, lo, hi) for the range of the pair's steps that
+    // lies in the item; f returns false to stop.
+    struct TcPair
+    {
+      int64_t sa, sb;
+      int32_t ksteps, ea, eb;
+    };
+    template <typename F>
+    __device__ __forceinline__ bool tc_segments(const TcArgs &a, const TcItem &it, F f)
+    {
+      if (it.pair_count == 0) return true;
+      int lo = it.s0, hi = min(it.s1, it.ksteps), base = it.ksteps;
+      if (lo < hi && !f(TcPair{it.sa, it.sb, it.ksteps, it.ea, it.eb}, lo, hi)) return false;
+      for (int p = 1; p < it.pair_count; ++p)
+      {
+        const DevSplitPair sp = a.spairs[it.pair_begin + p];
+        lo = max(it.s0 - base, 0);
+        hi = min(it.s1 - base, sp.ksteps);
+        base += sp.ksteps;
+        if (lo < hi && !f(TcPair{sp.sa, sp.sb, sp.ksteps, sp.ea, sp.eb}, lo, hi)) return false;
+      }
+      return true;
+    }
+
+    template <int S, int N>
+    __global__ void __launch_bounds__(TcShape<S, N>::threads, 1) gemm_split_tc_kernel(const __grid_constant__ TcArgs a)
+    {
+      using Shape = TcShape<S, N>;
+      constexpr int kStages = Shape::stages, kCols = Shape::cols, kWarps = Shape::warps;
       extern __shared__ __align__(1024) unsigned char smem[];
-      __shared__ __align__(8) uint64_t stage_done[kTcStages];
+      // a stage holds its copies' bytes; a stage's products are done; the level sums are complete, and
+      // their tensor memory free again; every product issued is done
+      __shared__ __align__(8) uint64_t full[kStages], empty[kStages], sums_full, sums_free, drained;
       __shared__ uint32_t tmem_base;
-      __shared__ int col_exp[kTcN];
-      __shared__ int failed;
+      __shared__ int failed_flag, last_flag;
+      volatile int *failed = &failed_flag;
       const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-      // tensor-memory lanes 32 quarter .. + 31 (the quarter a warp may access), columns kTcCols part ..
-      const int quarter = warp & 3, part = warp >> 2;
+      asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
       if (warp == 0)
       {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
       }
-      if (tid == 0)
+      if (tid == 32)
       {
-        for (int s = 0; s < kTcStages; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&stage_done[s])));
+        for (int s = 0; s < kStages; ++s)
+        {
+          bar_init(&full[s], 1);
+          bar_init(&empty[s], 1);
+        }
+        bar_init(&sums_full, 1);
+        bar_init(&sums_free, kWarps);
+        bar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        failed = 0;
+        failed_flag = 0;
       }
+      // this CTA's list; the first item is read, as all above is done, while the kernel before still runs
+      const TcItem *list = a.items + static_cast<int64_t>(blockIdx.x) * a.longest;
+      TcItem it = list[0];
       __syncthreads();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem = tmem_base;
-      // per stage: whether a commit is outstanding, and the parity of the phase it completes (the
-      // same for every thread: control flow is uniform)
-      bool pending[kTcStages] = {};
-      uint32_t parity[kTcStages] = {};
-      const auto settle = [&](int s) -> bool
-      {
-        if (!pending[s]) return true;
-        pending[s] = false;
-        const bool ok = tc_wait(&stage_done[s], parity[s]);
-        parity[s] ^= 1u;
-        return ok;
+      const auto next = [&](int &at) {
+        if (++at < a.longest) it = list[at];
+        else it.m = 0;
       };
-      const int64_t list_begin = a.cta_begin[blockIdx.x], list_end = a.cta_begin[blockIdx.x + 1];
-      for (int64_t idx = list_begin; idx < list_end && !failed; ++idx)
+      // the results of the kernel before are read, and memory that it may still read written, from here on
+      asm volatile("griddepcontrol.wait;\n" ::: "memory");
+
+      if (warp >= kWarps)
       {
-        const TcItem it = a.items[idx];
-        const DevBlock blk = a.blocks[it.block];
-        const int row = it.m0 + 32 * quarter + lane;
-        const int col0 = kTcCols * part;
-        double value[kTcCols];
-#pragma unroll
-        for (int j = 0; j < kTcCols; ++j) value[j] = 0.0;
-        for (int32_t pi = 0; pi < blk.pair_count && !failed; ++pi)
+        if constexpr (N == 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == kWarps && lane == 0)
         {
-          const DevPair pr = a.pairs[blk.pair_begin + pi];
-          const DevSplitPair sp = a.spairs[blk.pair_begin + pi];
-          if (pr.k <= 0) continue;
-          const int steps = (pr.k + kTcK - 1) / kTcK;
-          const uint16_t *ga = a.sa + sp.sa + static_cast<int64_t>(it.m0) * sp.kp;
-          const uint16_t *gb = a.sb + sp.sb + static_cast<int64_t>(it.n0) * sp.kp;
-          const int rows = min(kTcM, blk.m - it.m0), cols = min(kTcN, blk.n - it.n0);
-          // the stage of step `step`: S slices of A then of B, zeros outside the block
-          const auto load = [&](int step)
+          // the slices were written through the generic proxy
+          asm volatile("fence.proxy.async;" ::: "memory");
+          int stage = 0;
+          uint32_t phase = 0;
+          int64_t issued = 0;
+          bool ok = true;
+          for (int at = 0; it.m > 0 && ok; next(at))
           {
-            unsigned char *base = smem + (step % kTcStages) * tc_stage_bytes<S>();
-            const int k = step * kTcK;
-            for (int c = tid; c < S * kTcM * 4; c += kTcThreads)
-            {
-              const int t = c / (kTcM * 4), r = (c >> 2) % kTcM, q = c & 3;
-              const bool in = r < rows;
-              const uint32_t dst = smem_addr(base + t * kTcSliceA + (r >> 3) * kTcSbo + q * kTcLbo + (r & 7) * 16);
-              const uint16_t *src = ga + t * a.stride_a + static_cast<int64_t>(in ? r : 0) * sp.kp + k + q * 8;
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 16 : 0));
-            }
-            for (int c = tid; c < S * kTcN * 4; c += kTcThreads)
-            {
-              const int u = c / (kTcN * 4), r = (c >> 2) % kTcN, q = c & 3;
-              const bool in = r < cols;
-              const uint32_t dst =
-                smem_addr(base + S * kTcSliceA + u * kTcSliceB + (r >> 3) * kTcSbo + q * kTcLbo + (r & 7) * 16);
-              const uint16_t *src = gb + u * a.stride_b + static_cast<int64_t>(in ? r : 0) * sp.kp + k + q * 8;
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 16 : 0));
-            }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-          };
-          if (tid < kTcN) col_exp[tid] = tid < cols ? a.exps_b[sp.eb + it.n0 + tid] : 0;
-          const int row_exp = row < blk.m ? a.exps_a[sp.ea + row] : 0;
-          long long head[kTcCols];
-          float tail[kTcCols];
-#pragma unroll
-          for (int j = 0; j < kTcCols; ++j)
-          {
-            head[j] = 0;
-            tail[j] = 0.0f;
-          }
-          // the ring: steps 0 and 1 in flight before the first products
-          bool ok = settle(0);
-          ok = settle(1) && ok;
-          ok = __syncthreads_and(ok);
-          if (ok)
-          {
-            load(0);
-            if (steps > 1) load(1);
-          }
-          for (int step = 0; step < steps && ok; ++step)
-          {
-            const int s = step % kTcStages;
-            bool good = true;
-            if (step + 2 < steps)
-            {
-              good = settle((step + 2) % kTcStages);  // the products of step - 1 read it
-              load(step + 2);
-              asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-            }
-            else if (step + 1 < steps)
-              asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-            else
-              asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            // the stage's bytes, written through the generic proxy, become visible to the tensor cores
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (!__syncthreads_and(good))
-            {
-              ok = false;
-              break;
-            }
-            const bool chunk_first = step % kTcChunkSteps == 0;
-            if (tid == 0)
-            {
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              const uint32_t a_base = smem_addr(smem + s * tc_stage_bytes<S>());
-              const uint32_t b_base = a_base + S * kTcSliceA;
-#pragma unroll 1
-              for (int kk = 0; kk < kTcK; kk += 16)
-#pragma unroll 1
-                for (int t = 0; t < S; ++t)
-#pragma unroll 1
-                  for (int u = 0; u + t < S; ++u)
-                  {
-                    // level t + u is first reached at t = 0: that product starts the chunk's sum
-                    const uint32_t accumulate = (chunk_first && kk == 0 && t == 0) ? 0u : 1u;
-                    tc_mma(tmem + static_cast<uint32_t>((t + u) * kTcN), tc_desc(a_base + t * kTcSliceA + (kk / 8) * kTcLbo),
-                           tc_desc(b_base + u * kTcSliceB + (kk / 8) * kTcLbo), accumulate);
-                  }
-              asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_addr(&stage_done[s])));
-            }
-            pending[s] = true;
-            if ((step + 1) % kTcChunkSteps == 0 || step + 1 == steps)
-            {
-              // the chunk's level sums: wait for its products, read them back, fold them exactly
-              good = settle(s);
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              uint32_t lev[kTcCols];
-              const uint32_t lane_addr = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(col0);
-#pragma unroll
-              for (int l = 0; l < S; ++l)
+            const int groups_a = min(kTcM / 8, (it.m - it.m0 + 7) / 8), groups_b = min(N / 8, (it.n - it.n0 + 7) / 8);
+            const uint32_t bytes_a = groups_a * kSliceGroup * 2, bytes_b = groups_b * kSliceGroup * 2;
+            ok = tc_segments(a, it, [&](const TcPair &sp, int lo, int hi) {
+              for (int step = lo; step < hi; ++step)
               {
-                tc_load16(lane_addr + static_cast<uint32_t>(l * kTcN), lev);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (!tc_wait(&empty[stage], phase ^ 1u, failed)) return false;
+                int32_t stride_a, stride_b;
+                const uint16_t *ga = a.sa + slice_place(sp.sa, it.m, sp.ksteps, kSliceTileA, it.m0, step, stride_a);
+                const uint16_t *gb = a.sb + slice_place(sp.sb, it.n, sp.ksteps, kSliceTileB, it.n0, step, stride_b);
+                const uint32_t to = smem_addr(smem) + stage * Shape::stage;
+                bar_expect(&full[stage], S * (bytes_a + bytes_b));
 #pragma unroll
-                for (int j = 0; j < kTcCols; ++j)
+                for (int t = 0; t < S; ++t)
                 {
-                  const float x = __uint_as_float(lev[j]);
-                  if (l < 4)
-                    head[j] += static_cast<long long>(__float2int_rn(x)) << (7 * (3 - l));
-                  else
-                    tail[j] = fmaf(x, ldexpf(1.0f, -7 * (l - 4)), tail[j]);
+                  bulk_copy(to + t * Shape::slice_a, ga + t * stride_a, bytes_a, &full[stage]);
+                  bulk_copy(to + S * Shape::slice_a + t * Shape::slice_b, gb + t * stride_b, bytes_b, &full[stage]);
+                }
+                ++issued;
+                if (++stage == kStages)
+                {
+                  stage = 0;
+                  phase ^= 1u;
                 }
               }
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              if (!__syncthreads_and(good))
+              return true;
+            });
+          }
+          // no copy may still write this CTA's shared memory when it leaves
+          if (!ok)
+            for (int64_t i = max(static_cast<int64_t>(0), issued - kStages); i < issued; ++i)
+              tc_wait(&full[i % kStages], static_cast<uint32_t>(i / kStages) & 1u, nullptr);
+        }
+        else if (warp == kWarps + 1 && lane == 0)
+        {
+          int stage = 0;
+          uint32_t phase = 0, sums = 0;
+          bool ok = true;
+          for (int at = 0; it.m > 0 && ok; next(at))
+            ok = tc_segments(a, it, [&](const TcPair &, int lo, int hi) {
+              for (int step = lo; step < hi; ++step)
               {
-                ok = false;
-                break;
+                const bool chunk_first = (step - lo) % kTcChunkSteps == 0;
+                if (chunk_first && !tc_wait(&sums_free, sums ^ 1u, failed)) return false;
+                if (!tc_wait(&full[stage], phase, failed)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a_base = smem_addr(smem) + stage * Shape::stage, b_base = a_base + S * Shape::slice_a;
+#pragma unroll
+                for (int kk = 0; kk < kTcK / 16; ++kk)
+#pragma unroll
+                  for (int t = 0; t < S; ++t)
+#pragma unroll
+                    for (int c = 0; c < N * (S - t); c += 256)
+                    {
+                      constexpr int most = 256;
+                      const int n = N * (S - t) - c < most ? N * (S - t) - c : most;
+                      // slice t = 0 reaches every level: its first product starts the chunk's sums
+                      const uint32_t accumulate = (chunk_first && kk == 0 && t == 0) ? 0u : 1u;
+                      tc_mma(tmem + static_cast<uint32_t>(t * N + c), tc_desc(a_base + t * Shape::slice_a + kk * 2 * kTcLbo),
+                             tc_desc(b_base + (c / 8) * kTcSbo + kk * 2 * kTcLbo), tc_instr(n), accumulate);
+                    }
+                tc_commit(&empty[stage]);
+                if (step + 1 == hi || (step + 1 - lo) % kTcChunkSteps == 0)
+                {
+                  tc_commit(&sums_full);
+                  sums ^= 1u;
+                }
+                if (++stage == kStages)
+                {
+                  stage = 0;
+                  phase ^= 1u;
+                }
+              }
+              return true;
+            });
+          // no product may still run when the tensor memory is freed
+          if (!ok)
+          {
+            tc_commit(&drained);
+            tc_wait(&drained, 0, nullptr);
+          }
+        }
+      }
+      else
+      {
+        if constexpr (N == 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        // tensor-memory lanes 32 quarter .. + 31 (the quarter a warp may access), columns kCols part ..
+        const int quarter = warp & 3, part = warp >> 2, col0 = kCols * part;
+        const uint32_t lane_addr = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(col0);
+        const auto epilogue_sync = [] { asm volatile("bar.sync 1, %0;\n" ::"n"(kWarps * 32) : "memory"); };
+        uint32_t sums = 0;
+        bool ok = true;
+        for (int at_item = 0; it.m > 0 && ok; next(at_item))
+        {
+          const int row = it.m0 + 32 * quarter + lane;
+          // where the thread stores: rows top .. top + 7 of one column of each run of eight
+          const int top = it.m0 + 32 * quarter + (lane & 24), side = it.n0 + col0 + (lane & 7);
+          const auto place_of = [&](int c, int j) -> int64_t {
+            return top + j < it.m && side + c < it.n ? it.c + static_cast<int64_t>(top + j) * it.n + side + c : -1;
+          };
+          // the exponents of the row and of the columns (unconditional reads, so that all are in flight
+          // together); a tile's of 32 columns, and the places its entries go to, before the sums are there
+          const auto exponents = [&](int32_t ea, int32_t eb, int &re, int (&ce)[kCols]) {
+            re = a.exps_a[ea + min(row, it.m - 1)];
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) ce[j] = a.exps_b[eb + min(it.n0 + col0 + j, it.n - 1)];
+          };
+          // the tile's values: with one pair its level sums, fixed-point integers or doubles, whose scales are
+          // taken last; with several, scaled doubles
+          const bool single = it.pair_count == 1, fixed = S <= kTcFixedSlices && single && it.k <= kTcFixedK;
+          const int bits = fixed_bits(it.k);
+          int row_exp = 0, col_exp[kCols];
+          int32_t place[8];
+          if constexpr (N == 32)
+          {
+            if (single) exponents(it.ea, it.eb, row_exp, col_exp);
+            if (a.relabel)
+            {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+              {
+                const int64_t at = place_of(0, j);
+                place[j] = at >= 0 ? a.relabel[at] : -1;
               }
             }
           }
-          if (!ok)
-          {
-            if (tid == 0) atomicExch(a.error, 1);
-            failed = 1;
-          }
-          __syncthreads();
-          // one FP64 step per entry: head 2^-35 + tail 2^-42 times the row and column scales
+          long long value[kCols];
 #pragma unroll
-          for (int j = 0; j < kTcCols; ++j)
-          {
-            const int ex = row_exp + col_exp[col0 + j];
-            value[j] += fma(static_cast<double>(head[j]), pow2(ex - 35), static_cast<double>(tail[j]) * pow2(ex - 42));
-          }
-          __syncthreads();  // col_exp is rewritten by the next pair
-        }
-        if (row < blk.m)
-        {
-          double *out = a.c + blk.c + static_cast<int64_t>(row) * blk.n + it.n0 + col0;
+          for (int j = 0; j < kCols; ++j) value[j] = 0;  // also 0.0
+          bool some = false;
+          ok = tc_segments(a, it, [&](const TcPair &sp, int lo, int hi) {
+            long long head[kCols];
+            float tail[kCols];
 #pragma unroll
-          for (int j = 0; j < kTcCols; ++j)
-            if (it.n0 + col0 + j < blk.n) out[j] = value[j];
+            for (int j = 0; j < kCols; ++j)
+            {
+              head[j] = 0;
+              tail[j] = 0.0f;
+            }
+            for (int step = lo; step < hi; step += kTcChunkSteps)
+            {
+              if (!tc_wait(&sums_full, sums, failed)) return false;
+              sums ^= 1u;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+              for (int c = 0; c < kCols; c += 8)
+#pragma unroll
+                for (int l0 = 0; l0 < S; l0 += 3)
+                {
+                  // three levels of eight columns in flight at a time
+                  constexpr int kAhead = 3;
+                  uint32_t lev[kAhead][8];
+#pragma unroll
+                  for (int l = 0; l < kAhead && l0 + l < S; ++l) tc_load8(lane_addr + static_cast<uint32_t>((l0 + l) * N + c), lev[l]);
+                  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                  for (int l = 0; l < kAhead && l0 + l < S; ++l)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                    {
+                      const float x = __uint_as_float(lev[l][j]);
+                      if (l0 + l < 4)
+                        head[c + j] += static_cast<long long>(__float2int_rn(x)) * (1ll << (7 * (3 - l0 - l)));
+                      else
+                        tail[c + j] = fmaf(x, 1.0f / static_cast<float>(1 << (7 * (l0 + l - 4))), tail[c + j]);
+                    }
+                }
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) bar_arrive(&sums_free);
+            }
+            if (fixed)
+            {
+              // the tail in two 32-bit conversions (below 7.1 2^12 K <= 2^31), the fraction exact
+#pragma unroll
+              for (int j = 0; j < kCols; ++j)
+              {
+                const float whole = rintf(tail[j]);
+                const int low = __float2int_rn((tail[j] - whole) * static_cast<float>(1 << bits));
+                value[j] = (head[j] << (7 + bits)) + static_cast<long long>(__float2int_rn(whole)) * (1ll << bits) + low;
+              }
+            }
+            else
+            {
+              // one FP64 step per entry, and the scales of a pair among several
+              int re = 0, ce[kCols] = {};
+              if (!single) exponents(sp.ea, sp.eb, re, ce);
+#pragma unroll
+              for (int j = 0; j < kCols; ++j)
+              {
+                double x = level_sum(head[j], tail[j]);
+                if (!single) x = scaled(x, re + ce[j]);
+                if (some) x += __longlong_as_double(value[j]);
+                value[j] = __double_as_longlong(x);
+              }
+            }
+            some = true;
+            return true;
+          });
+          if (!ok) break;
+          if (it.slot >= 0)
+          {
+            // a partial tile, columns of 128 rows so that a warp writes 256 contiguous bytes; the CTA
+            // that holds the tile's last ticket sums them in slot order
+            long long *out = reinterpret_cast<long long *>(a.partial) + static_cast<int64_t>(it.slot) * kTcM * N + col0 * kTcM +
+                             32 * quarter + lane;
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) __stcg(out + j * kTcM, value[j]);
+            const GemmReduce r = a.reduces[it.reduce];
+            __threadfence();
+            epilogue_sync();
+            if (tid == 0)
+            {
+              last_flag = atomicAdd(a.tickets + it.reduce, 1) == r.nslots - 1;
+              // every other part of the tile has its ticket: left zero for the next launch
+              if (last_flag) a.tickets[it.reduce] = 0;
+            }
+            epilogue_sync();
+            const bool last = last_flag;
+            epilogue_sync();
+            if (!last) continue;
+            __threadfence();
+            const long long *from = reinterpret_cast<const long long *>(a.partial) + static_cast<int64_t>(r.slot0) * kTcM * N +
+                                    col0 * kTcM + 32 * quarter + lane;
+#pragma unroll
+            for (int c = 0; c < kCols; c += 8)
+            {
+              // three parts' reads in flight at a time
+              constexpr int kAhead = 3;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) value[c + j] = 0;
+              for (int s0 = 0; s0 < r.nslots; s0 += kAhead)
+              {
+                long long x[kAhead][8];
+#pragma unroll
+                for (int s = 0; s < kAhead; ++s)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j)
+                    x[s][j] = s0 + s < r.nslots ? __ldcg(from + static_cast<int64_t>(s0 + s) * kTcM * N + (c + j) * kTcM) : 0;
+#pragma unroll
+                for (int s = 0; s < kAhead; ++s)
+#pragma unroll
+                  for (int j = 0; j < 8; ++j)
+                    value[c + j] = fixed ? value[c + j] + x[s][j]
+                                         : __double_as_longlong(__longlong_as_double(value[c + j]) + __longlong_as_double(x[s][j]));
+              }
+            }
+          }
+          if constexpr (N != 32)
+            if (single) exponents(it.ea, it.eb, row_exp, col_exp);
+          if (single && !fixed)
+          {
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+              value[j] = __double_as_longlong(scaled(__longlong_as_double(value[j]), row_exp + col_exp[j]));
+          }
+          if (fixed)
+          {
+            row_exp -= 42 + bits;
+            bool outside = false;
+            long long number[kCols];
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+              number[j] = __double_as_longlong(fixed_to_double(value[j], row_exp + col_exp[j], outside));
+            if (outside)
+            {
+#pragma unroll 1
+              for (int j = 0; j < kCols; ++j)
+              {
+                long long v = 0;
+                int ex = 0;
+#pragma unroll
+                for (int i = 0; i < kCols; ++i)
+                  if (i == j)
+                  {
+                    v = value[i];
+                    ex = row_exp + col_exp[i];
+                  }
+                const long long slow = __double_as_longlong(fixed_slow(v, ex));
+#pragma unroll
+                for (int i = 0; i < kCols; ++i)
+                  if (i == j) number[i] = slow;
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) value[j] = number[j];
+          }
+#pragma unroll
+          for (int c = 0; c < kCols; c += 8)
+          {
+            transpose8(value + c, lane);
+            if (a.relabel)
+            {
+              // straight to its place after the leg move that follows
+              if constexpr (N != 32)
+              {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                {
+                  const int64_t at = place_of(c, j);
+                  place[j] = at >= 0 ? a.relabel[at] : -1;
+                }
+              }
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (place[j] >= 0) a.c[place[j]] = __longlong_as_double(value[c + j]);
+            }
+            else
+            {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+              {
+                const int64_t at = place_of(c, j);
+                if (at >= 0) a.c[at] = __longlong_as_double(value[c + j]);
+              }
+            }
+          }
+          // the alignment pad after an odd-sized block reads as zero in arena-wide sums
+          const int64_t entries = static_cast<int64_t>(it.m) * it.n;
+          if (!a.relabel && tid == 0 && it.m0 + kTcM >= it.m && it.n0 + N >= it.n && (entries & 1)) a.c[it.c + entries] = 0.0;
         }
-        const int64_t entries = static_cast<int64_t>(blk.m) * blk.n;
-        if (tid == 0 && it.m0 + kTcM >= blk.m && it.n0 + kTcN >= blk.n && (entries & 1)) a.c[blk.c + entries] = 0.0;
       }
-      // no copy or product may still write shared or tensor memory when the CTA leaves
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-      for (int s = 0; s < kTcStages; ++s)
-        if (!settle(s) && lane == 0) atomicExch(a.error, 1);
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();
+      if (tid == 0 && failed_flag) atomicExch(a.error, 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
     }
   } // namespace
@@ -345,9 +628,110 @@ namespace ttg
   // host
   // ------------------------------------------------------------------------------------------
 
-  bool split_tc_suits(const Program &p, const Op &op, int32_t slices)
+  // Tiles of 64 columns, of 32 when 64 would leave SMs without a tile (half the time to the end of a
+  // small product); a tile whose K is more than an
+  // SM's share of the work is cut along K into equal parts of at least sixteen steps, so that the parts
+  // fill the SMs once.  A part costs its pipeline's fill, a partial tile of 32 or 64 KB and the ticket
+  // (6 us of a 12 us product): the matvec of bond 400 takes 63.5, 49.6, 47.6 and 49.2 us with at
+  // least 4, 6, 8 and 16 steps a part, that of bond 512 69.5, 69.2, 69.2 and 64.0, of bond 200 29.4,
+  // 30.6, 30.7 and 28.1.
+  TcSchedule schedule_tc(const Program &p, const Op &op, const std::vector<SplitPair> *pairs)
   {
-    if (slices < 1 || slices > kTcMaxSlices) return false;
+    TcSchedule s;
+    const auto steps_of = [&p](const GemmBlock &blk) {
+      int64_t steps = 0;
+      for (int32_t q = 0; q < blk.pair_count; ++q)
+        steps += (p.gemm_pairs[static_cast<size_t>(blk.pair_begin + q)].k + kTcK - 1) / kTcK;
+      return steps;
+    };
+    int64_t tiles[2] = {}, total[2] = {};
+    for (int64_t b = op.begin; b < op.begin + op.count; ++b)
+    {
+      const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
+      const int64_t steps = steps_of(blk), high = (blk.m + kTcM - 1) / kTcM;
+      for (int w = 0; w < 2; ++w)
+      {
+        const int64_t n = high * ((blk.n + (32 << w) - 1) / (32 << w));
+        tiles[w] += n;
+        total[w] += n * steps;
+      }
+    }
+    const int w = tiles[1] <= p.ctas ? 0 : 1;
+    s.n = 32 << w;
+    int64_t share = std::max<int64_t>(16, (total[w] + p.ctas - 1) / p.ctas);
+    // a ticket per cut tile, and the error flag after them
+    if (tiles[w] >= kTicketInts - 1) share = INT32_MAX;
+    struct Sized
+    {
+      TcItem item;
+      int64_t work;
+    };
+    std::vector<Sized> all;
+    for (int64_t b = op.begin; b < op.begin + op.count; ++b)
+    {
+      const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
+      const int64_t steps = steps_of(blk), parts = std::max<int64_t>(1, (steps + share - 1) / share);
+      const int64_t per = (steps + parts - 1) / parts;
+      TcItem it{blk.c, 0, 0, blk.m, blk.n, 0, 0, 0, static_cast<int32_t>(steps), -1, -1, blk.pair_begin, blk.pair_count, 0, 0, 0, 0};
+      if (pairs && blk.pair_count > 0)
+      {
+        const SplitPair &sp = (*pairs)[static_cast<size_t>(blk.pair_begin)];
+        it.sa = sp.sa;
+        it.sb = sp.sb;
+        it.k = p.gemm_pairs[static_cast<size_t>(blk.pair_begin)].k;
+        it.ksteps = sp.ksteps;
+        it.ea = sp.ea;
+        it.eb = sp.eb;
+      }
+      for (it.m0 = 0; it.m0 < blk.m; it.m0 += kTcM)
+        for (it.n0 = 0; it.n0 < blk.n; it.n0 += s.n)
+        {
+          if (parts == 1)
+          {
+            if (pairs) all.push_back({it, steps + 4});
+            continue;
+          }
+          const int32_t slot0 = static_cast<int32_t>(s.slots);
+          TcItem cut = it;
+          cut.reduce = static_cast<int32_t>(s.reduces.size());
+          for (int64_t s0 = 0; s0 < steps; s0 += per)
+          {
+            cut.s0 = static_cast<int32_t>(s0);
+            cut.s1 = static_cast<int32_t>(std::min(steps, s0 + per));
+            cut.slot = static_cast<int32_t>(s.slots++);
+            if (pairs) all.push_back({cut, per + 5});
+          }
+          s.reduces.push_back({static_cast<int32_t>(b), it.m0, it.n0, slot0, static_cast<int32_t>(s.slots) - slot0, 0});
+        }
+    }
+    if (!pairs) return s;
+    // the largest first, each to the least loaded SM
+    std::stable_sort(all.begin(), all.end(), [](const Sized &x, const Sized &y) { return x.work > y.work; });
+    s.ctas = static_cast<int32_t>(std::min<size_t>(static_cast<size_t>(p.ctas), all.size()));
+    std::vector<std::vector<int32_t>> lists(static_cast<size_t>(s.ctas));
+    std::vector<std::pair<int64_t, int>> heap;
+    for (int c = 0; c < s.ctas; ++c) heap.push_back({0, c});
+    const auto later = [](const std::pair<int64_t, int> &x, const std::pair<int64_t, int> &y) { return x > y; };
+    std::make_heap(heap.begin(), heap.end(), later);
+    for (size_t i = 0; i < all.size(); ++i)
+    {
+      std::pop_heap(heap.begin(), heap.end(), later);
+      auto &least = heap.back();
+      lists[static_cast<size_t>(least.second)].push_back(static_cast<int32_t>(i));
+      least.first += all[i].work;
+      std::push_heap(heap.begin(), heap.end(), later);
+    }
+    for (const auto &list : lists) s.longest = std::max(s.longest, static_cast<int32_t>(list.size()));
+    s.items.assign(static_cast<size_t>(s.ctas) * static_cast<size_t>(s.longest), TcItem{});
+    for (size_t c = 0; c < lists.size(); ++c)
+      for (size_t i = 0; i < lists[c].size(); ++i)
+        s.items[c * static_cast<size_t>(s.longest) + i] = all[static_cast<size_t>(lists[c][i])].item;
+    return s;
+  }
+
+  bool split_tc_large(const Program &p, const Op &op, int32_t slices)
+  {
+    if (slices < 1) return false;
     // enough whole tiles to give every SM several, and most of the work in them
     double work = 0, tiled = 0;
     int64_t tiles = 0;
@@ -358,88 +742,38 @@ namespace ttg
       for (int32_t q = 0; q < blk.pair_count; ++q) k += p.gemm_pairs[static_cast<size_t>(blk.pair_begin + q)].k;
       const double w = static_cast<double>(blk.m) * blk.n * k;
       work += w;
-      tiles += static_cast<int64_t>((blk.m + kTcM - 1) / kTcM) * ((blk.n + kTcN - 1) / kTcN);
-      if (blk.m >= kTcM / 2 && blk.n >= kTcN / 2) tiled += w;
+      tiles += static_cast<int64_t>((blk.m + kTcM - 1) / kTcM) * ((blk.n + 63) / 64);
+      if (blk.m >= kTcM / 2 && blk.n >= 32) tiled += w;
     }
     return tiles >= 4 * static_cast<int64_t>(p.ctas) && tiled >= 0.9 * work;
   }
 
-  cudaError_t launch_split_tc(const Program &p, const Op &op, DeviceTables &t, size_t op_index, int32_t slices,
+  cudaError_t launch_split_tc(const DeviceTables &t, size_t op_index, int32_t slices,
                               const uint16_t *sa, const uint16_t *sb, const int16_t *exps_a, const int16_t *exps_b,
-                              int64_t stride_a, int64_t stride_b, const void *spairs, double *C, int *error,
+                              const void *spairs, double *C, double *partial, int *tickets, const int32_t *relabel,
                               cudaStream_t stream)
   {
-    DeviceTables::TcTables &tc = t.tc[op_index];
-    {
-      std::lock_guard<std::mutex> lock(t.mutex);
-      if (!tc.ready)
-      {
-        // tiles largest first (K of the block), each to the least loaded SM
-        struct Sized
-        {
-          TcItem item;
-          double work;
-        };
-        std::vector<Sized> all;
-        for (int64_t b = op.begin; b < op.begin + op.count; ++b)
-        {
-          const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
-          int64_t k = 0;
-          for (int32_t q = 0; q < blk.pair_count; ++q) k += p.gemm_pairs[static_cast<size_t>(blk.pair_begin + q)].k;
-          for (int32_t m0 = 0; m0 < blk.m; m0 += kTcM)
-            for (int32_t n0 = 0; n0 < blk.n; n0 += kTcN)
-              all.push_back({{static_cast<int32_t>(b), m0, n0, 0}, static_cast<double>(kTcK) * (1 + (k + kTcK - 1) / kTcK)});
-        }
-        std::stable_sort(all.begin(), all.end(), [](const Sized &x, const Sized &y) { return x.work > y.work; });
-        const int ctas = static_cast<int>(std::min<size_t>(static_cast<size_t>(p.ctas), std::max<size_t>(all.size(), 1)));
-        std::vector<std::vector<TcItem>> lists(static_cast<size_t>(ctas));
-        std::vector<std::pair<double, int>> heap;
-        for (int c = 0; c < ctas; ++c) heap.push_back({0.0, c});
-        const auto later = [](const std::pair<double, int> &x, const std::pair<double, int> &y)
-        { return x.first > y.first || (x.first == y.first && x.second > y.second); };
-        std::make_heap(heap.begin(), heap.end(), later);
-        for (const Sized &s : all)
-        {
-          std::pop_heap(heap.begin(), heap.end(), later);
-          auto &least = heap.back();
-          lists[static_cast<size_t>(least.second)].push_back(s.item);
-          least.first += s.work;
-          std::push_heap(heap.begin(), heap.end(), later);
-        }
-        std::vector<TcItem> items;
-        std::vector<int32_t> begin{0};
-        for (const auto &list : lists)
-        {
-          items.insert(items.end(), list.begin(), list.end());
-          begin.push_back(static_cast<int32_t>(items.size()));
-        }
-        TableStaging staging;
-        staging.add(items, &tc.items);
-        staging.add(begin, reinterpret_cast<void **>(&tc.cta_begin));
-        const cudaError_t e = staging.commit(&tc.base);
-        if (e != cudaSuccess) return e;
-        tc.n_ctas = ctas;
-        tc.ready = true;
-      }
-    }
-    TcArgs args{sa, sb, exps_a, exps_b, stride_a, stride_b, C, reinterpret_cast<const DevBlock *>(t.blocks),
-                reinterpret_cast<const DevPair *>(t.pairs), static_cast<const DevSplitPair *>(spairs),
-                static_cast<const TcItem *>(tc.items), tc.cta_begin, error};
+    const DeviceTables::TcTables &tc = t.tc[op_index];
+    const TcArgs args{sa, sb, exps_a, exps_b, C, relabel,
+                      static_cast<const DevSplitPair *>(spairs), static_cast<const TcItem *>(tc.items), tc.reduces, tc.longest,
+                      partial, tickets, tickets + kTicketInts - 1};
     cudaError_t e = cudaSuccess;
-    switch (slices)
+    switch (slices * 128 + tc.n)
     {
-#define TTG_TC(S)                                                                                                          \
-  case S:                                                                                                                  \
+#define TTG_TC(S, N)                                                                                                       \
+  case S * 128 + N:                                                                                                        \
   {                                                                                                                        \
     static std::once_flag once;                                                                                            \
     std::call_once(once, [&] {                                                                                             \
-      e = cudaFuncSetAttribute(gemm_split_tc_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_launch_bytes<S>()); \
+      e = cudaFuncSetAttribute(gemm_split_tc_kernel<S, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<S, N>::bytes); \
     });                                                                                                                    \
     if (e != cudaSuccess) return e;                                                                                        \
-    e = launch_dependent(gemm_split_tc_kernel<S>, tc.n_ctas, kTcThreads, tc_launch_bytes<S>(), stream, args);             \
+    e = launch_dependent(gemm_split_tc_kernel<S, N>, tc.n_ctas, TcShape<S, N>::threads, TcShape<S, N>::bytes, stream, args);          \
     break;                                                                                                                 \
   }
-      TTG_TC(1) TTG_TC(2) TTG_TC(3) TTG_TC(4) TTG_TC(5) TTG_TC(6)
+#define TTG_TC2(S) TTG_TC(S, 32) TTG_TC(S, 64)
+      TTG_TC2(1) TTG_TC2(2) TTG_TC2(3) TTG_TC2(4) TTG_TC2(5) TTG_TC2(6) TTG_TC2(7) TTG_TC2(8)
+#undef TTG_TC2
 #undef TTG_TC
     default: return cudaErrorInvalidValue;
     }

@@ -1,0 +1,60 @@
+'''Split-precision block products at the sizes where their kernels can go wrong: one block of m x k times
+k x n around the tiles (128 rows, 32 and 64 columns), the groups of eight lines, the steps of 32 and the
+exact chunks of 512 of K, with K shared by several CTAs; rows and columns scaled far apart, a zero row,
+and results below the normal range.
+
+The bound, per entry, with e the exponents above the row's and the column's largest entries and
+u = 2^(e_row + e_col): each operand's S digits leave at most 2^(-7S-1) (1 + 2^-6) of its scale, the
+products of digits past level S - 1 sum to at most (S - 1) 2^(-7S-2) (1 + 2^-6) a K, and the levels from 4
+on (below 2^-25 K u together) are added in fp32: below 2^-48 K u.  The result is rounded to FP64 once.'''
+import numpy as np
+import pytest
+import torch
+
+import tentorch_gb300 as tg
+from tentorch_gb300 import linalg as la
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(1, 1, 1), (7, 9, 31), (8, 32, 32), (129, 65, 33), (128, 64, 512), (130, 33, 545), (40, 31, 1100)]
+
+
+def _tensor(matrix):
+    m, n = matrix.shape
+    cat = tg.no_symmetry
+    legs = [tg.Leg(cat, [(0,)], [x]) for x in (m, n)]
+    out = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = torch.float64, device = 'cuda')
+    out.block((0,), (0,)).copy_(torch.from_numpy(matrix))
+    return out
+
+
+def _exponents(largest):
+    return np.where(largest > 0, np.frexp(largest)[1], 0)
+
+
+@pytest.mark.parametrize('slices', [1, 3, 6, 8])
+@pytest.mark.parametrize('size', SIZES)
+def test_one_block_within_its_bound(size, slices):
+    m, n, k = size
+    rng = np.random.default_rng(m * 1000 + k)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    a *= 2.0 ** rng.integers(-40, 40, m)[:, None]
+    b *= 2.0 ** rng.integers(-40, 40, n)[None, :]
+    if m > 2:
+        a[1] = 0.0
+        a[2] *= 2.0 ** -990  # its products with the smaller columns lie below the normal range
+    want = a.astype(np.longdouble) @ b.astype(np.longdouble)
+    scale = np.ldexp(np.longdouble(1), _exponents(np.abs(a).max(1))[:, None] + _exponents(np.abs(b).max(0))[None, :])
+    bound = k * scale * (2.0 ** (-7 * slices) * (1.02 + 0.26 * (slices - 1)) + 2.0 ** -48) + 2.0 ** -52 * np.abs(want) + 2.0 ** -1074
+    ta, tb = _tensor(a), _tensor(b)
+    with tg.precision(slices):
+        plan = la.contract_plan(ta._space, tb._space, [1], [0])
+        try:
+            for forms in (0, la.FORM_NO_TENSOR_CORES):
+                la.store_forms(plan, forms)
+                for _ in range(2):
+                    got = tg.contract(ta, tb, [1], [0]).block((0,), (0,)).cpu().numpy()
+                    worst = np.abs(got.astype(np.longdouble) - want) / bound
+                    assert worst.max() <= 1, (forms, float(worst.max()))
+        finally:
+            la.clear_tuning()
