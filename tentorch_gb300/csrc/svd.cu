@@ -10,31 +10,36 @@
 // truncating DMRG needs for the kept vectors however small their values.
 //
 // FP64 on this GPU runs at about 1/64 of the FP32 rate (about two FP64 multiply-adds per clock
-// per SM), so the sweeps are mixed precision and the FP64 part is spread over several SMs:
-//   0. (blocks of 32 columns or more) the columns sorted by norm and factored A P = Q R; steps 1-4
-//      then work on the graded X = R^T, and U = Q J at the end (Drmac & Veselic 2008).
-//   1. FP32 sweeps on a scaled copy of the block until its columns are orthogonal to ~1e-5; they
-//      give a rotation V32 close to the right singular vectors.
-//   2. V = V32 in FP64, made orthonormal to FP64 precision by two Newton-Schulz steps
-//      V <- V + V (I - V^T V) / 2 (quadratic: 1e-6 -> 1e-12 -> round-off).
-//   3. W = A V in FP64 (columns already orthogonal to ~1e-6).
-//   4. FP64 sweeps on W with V accumulated: from a start that close, Jacobi's quadratic
-//      convergence needs two or three sweeps; a sweep whose cosines were all below sqrt(tol) is
-//      the last (the cosines it leaves are below ~tol).
+// per SM), so the rotations run in FP32 and FP64 only refines what they leave:
+//   0. the columns sorted by norm and factored A P = Q R; the rest works on the graded X = R^T, and
+//      U = Q J at the end (Drmac & Veselic 2008).
+//   1. FP32 sweeps on a scaled copy until its columns are orthogonal to ~1e-5; they give a rotation
+//      close to the right singular vectors, small columns included (their cosines are formed without
+//      squares that underflow).  Blocks of four columns at a time (blocked_sweeps), or column by column
+//      for columns beyond 320.
+//   2. V refined in FP64 by matrix products: from the Gram matrices of W = X V and of V, all pairs' angles
+//      at once and V's orthonormality, quadratically (1e-5 -> 1e-9 -> round-off), three or four times.
+//   3. where the refinement does not settle (singular values closer than FP32 separates): V made
+//      orthonormal by two Newton-Schulz steps, W = X V, and FP64 sweeps on W with V accumulated; a
+//      sweep whose cosines were all below sqrt(tol) is the last (the cosines it leaves are below ~tol).
 // In the FP64 sweeps only the dot product of the pair is taken (the squared column norms are
 // carried along with the exact update of a rotation and recomputed at each sweep's start), and the
 // angle is found in FP32 and then made exactly orthogonal in FP64 (c^2 + s^2 = 1 by a second-order
 // correction): an angle good to 1e-7 still shrinks the pair's cosine by that factor each rotation.
 //
-// A thread-block cluster of up to 8 CTAs (1024 threads each) per block.  Rank 0 runs step 1 alone;
-// steps 2-4 run on the whole cluster, step 4 with the rows of W and V dealt to the ranks and the
-// dot products of each round summed over the cluster through distributed shared memory.  Each
-// sweep runs the pairs in the round-robin (circle) order, k - 1 rounds of disjoint pairs, a group
-// of lanes per pair.  Working sets sit in shared memory when they fit (227 KB per CTA), else in
-// the global workspace (L2 resident).  At most kMaxSweeps sweeps per phase; a block whose FP64
-// phase did not converge reports -1 in `info` (the host raises).  All loops are bounded and every
-// CTA of a cluster passes the same sequence of cluster barriers: the number of sweeps is decided
-// by rank 0's flag, read by all.
+// One launch, one block of 148 x 148 / 92 x 92 / 31 x 31 with singular values over twelve decades: 2782 / 1378 /
+// 466 us; with FP32 sweeps column by column that skipped the small columns and 3 to 6 FP64 sweeps 7557 /
+// 3783 / 2152 us.  Factors orthonormal to 1e-15 (3e-15 before; clusters of values 1e-9 apart 1e-11, 1e-7
+// before).  At 148 columns now: QR 0.56 ms, FP32 sweeps 1.16 (eight), refinement 0.73, U = Q J 0.27.
+//
+// A thread-block cluster of up to 16 CTAs per block, which shares every step: QR by columns, FP32 sweeps
+// by pairs of column blocks in distributed shared memory, the products by tiles, the FP64 sweeps with
+// the rows of W and V dealt to the ranks and the dot products of each round summed over the cluster.
+// Each sweep runs the pairs in the round-robin (circle) order.  Working sets sit in shared memory
+// when they fit (227 KB per CTA), else in the global workspace (L2 resident).  At most kMaxSweeps
+// sweeps per phase; a block whose FP64 phase did not converge reports -1 in `info` (the host raises).
+// All loops are bounded and every CTA of a cluster passes the same sequence of cluster barriers: what
+// ends a loop is the same on every rank.
 //
 // A second kernel writes the kept part of each block's factors into the two output arenas, with
 // the singular values absorbed as the caller asks, so that a whole truncating split is two
@@ -98,7 +103,7 @@ namespace ttg
       l.w_slices = 3 * k * k;
       l.v_slices = l.w_slices + (len + kMaxCluster) * k;
       l.w32_slices = l.v_slices + (k + kMaxCluster) * k;
-      l.v32_slices = l.w32_slices + ((len + kMaxCluster) * k + 1) / 2;
+      l.v32_slices = l.w32_slices + ((len + kMaxCluster) * k + 1) / 2;  // (together k^2 doubles and more)
       l.f = l.v32_slices + ((k + kMaxCluster) * k + 1) / 2;
       l.tau = l.f + len * k;
       l.order = l.tau + k;
@@ -107,8 +112,9 @@ namespace ttg
       l.total = (l.total + 31) / 32 * 32;
       return l;
     }
-    // Blocks of at least this many columns (swept over a cluster) are preconditioned by QR.
-    constexpr int64_t kQrMinCols = 32;
+    // Blocks of at least this many columns are preconditioned by QR (below 32 columns, on one CTA, it
+    // costs little, and the refinement needs the graded columns it leaves).
+    constexpr int64_t kQrMinCols = 2;
 
     // The circle method's pair t of a round (players even, round < players - 1, t < players / 2):
     // player players - 1 stays, the others turn; p < q.  In 32-bit arithmetic with one conditional
@@ -145,12 +151,27 @@ namespace ttg
     // orthogonal: w_p' = c w_p - s w_q, w_q' = s w_p + c w_q with t = s / c the smaller root of
     // t^2 + 2 zeta t - 1 = 0, zeta = (beta - alpha) / (2 gamma).  Found in FP32 on values scaled
     // by a power of two; false when gamma is negligible at that scale.
-    __device__ __forceinline__ bool angle_of(float a, float b, float g, float &c, float &s)
+    // (`diff` is b - a: in FP64 taken before the rounding to FP32, so that close norms keep their
+    // difference.)
+    __device__ __forceinline__ bool angle_of(float diff, float g, float &c, float &s)
     {
       if (g == 0.0f) return false;
-      const float zeta = (b - a) / (2.0f * g);
+      const float zeta = diff / (2.0f * g);
       const float t = fabsf(zeta) > 1e15f ? 0.5f / zeta : copysignf(1.0f, zeta) / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
       c = rsqrtf(1.0f + t * t);
+      s = c * t;
+      return true;
+    }
+
+    // The same with the hardware's approximate reciprocal and reciprocal root (a few units in the last
+    // place, like the rotations' own rounding; V is made orthonormal afterwards).
+    __device__ __forceinline__ bool angle_fast(float diff, float g, float &c, float &s)
+    {
+      if (g == 0.0f) return false;
+      const float zeta = __fdividef(diff, 2.0f * g), one = fmaf(zeta, zeta, 1.0f);
+      const float t = fabsf(zeta) > 1e15f ? __fdividef(0.5f, zeta)
+                                          : copysignf(__fdividef(1.0f, fabsf(zeta) + one * rsqrtf(one)), zeta);
+      c = rsqrtf(fmaf(t, t, 1.0f));
       s = c * t;
       return true;
     }
@@ -159,14 +180,25 @@ namespace ttg
     // the angle; FP64 ones are brought to that scale by a power of two first
     __device__ __forceinline__ bool angle(float alpha, float beta, float gamma, float &c, float &s)
     {
-      return angle_of(alpha, beta, gamma, c, s);
+      return angle_of(beta - alpha, gamma, c, s);
     }
     __device__ __forceinline__ bool angle(double alpha, double beta, double gamma, float &c, float &s)
     {
       int ex;
       frexp(fmax(alpha, beta), &ex);
-      return angle_of(static_cast<float>(ldexp(alpha, -ex)), static_cast<float>(ldexp(beta, -ex)),
-                      static_cast<float>(ldexp(gamma, -ex)), c, s);
+      return angle_of(static_cast<float>(ldexp(beta - alpha, -ex)), static_cast<float>(ldexp(gamma, -ex)), c, s);
+    }
+
+    // Whether the pair's cosine is above `limit`.  In FP32 the squares of the smaller columns' products
+    // would underflow (columns 1e-10 of the largest and below were never rotated so, and were left to
+    // the FP64 sweeps), so the cosine itself is formed.
+    __device__ __forceinline__ bool above(float gamma, float alpha, float beta, float limit)
+    {
+      return fabsf(gamma) * rsqrtf(alpha) * rsqrtf(beta) > limit;
+    }
+    __device__ __forceinline__ bool above(double gamma, double alpha, double beta, double limit)
+    {
+      return gamma * gamma > limit * limit * alpha * beta;
     }
 
     template <typename T, int G>
@@ -298,11 +330,11 @@ namespace ttg
       const int group = lane / G, gl = lane % G;
       constexpr int per_warp = 32 / G;
       const int64_t players = k + (k & 1), pairs = players / 2;
-      const T tol2 = static_cast<T>(tol * tol);
+      const T least = static_cast<T>(tol);
       // a sweep whose rotations all had cosines below sqrt(tol) ends the phase: Jacobi converges
       // quadratically there, so the cosines it leaves are below ~tol and a further sweep (which
       // would find nothing above tol to rotate) is not run
-      const T settled2 = static_cast<T>(tol);
+      const T settled = static_cast<T>(sqrt(tol));
       // FP64 over a cluster: after the barrier a group of lanes per pair finds the rotation (the
       // scalar part) and lists it, then the whole CTA rotates the listed pairs' entries, so that
       // the FP64 instructions of the rotations spread over every warp instead of the few that hold
@@ -354,7 +386,7 @@ namespace ttg
             {
               if (!pair) continue;
               const T alpha = norms[p], beta = norms[q];
-              if (gamma * gamma <= tol2 * alpha * beta) continue;
+              if (!above(gamma, alpha, beta, least)) continue;
               float cf, sf;
               if (!angle(alpha, beta, gamma, cf, sf)) continue;
               T c, sn;
@@ -366,7 +398,7 @@ namespace ttg
                 const T cc = c * c, ss = sn * sn, cs2 = 2 * c * sn * gamma;
                 norms[p] = cc * alpha - cs2 + ss * beta;
                 norms[q] = ss * alpha + cs2 + cc * beta;
-                if (gamma * gamma > settled2 * alpha * beta) flags[sweep & 1] = 1;
+                if (above(gamma, alpha, beta, settled)) flags[sweep & 1] = 1;
               }
             }
           }
@@ -390,7 +422,7 @@ namespace ttg
                 gamma = group_sum<T, G>(gamma);
                 if (!pair || gl != 0) continue;
                 const T alpha = norms[p], beta = norms[q];
-                if (gamma * gamma <= tol2 * alpha * beta) continue;
+                if (!above(gamma, alpha, beta, least)) continue;
                 float cf, sf;
                 if (!angle(alpha, beta, gamma, cf, sf)) continue;
                 T c, sn;
@@ -398,7 +430,7 @@ namespace ttg
                 const T cc = c * c, ss = sn * sn, cs2 = 2 * c * sn * gamma;
                 norms[p] = cc * alpha - cs2 + ss * beta;
                 norms[q] = ss * alpha + cs2 + cc * beta;
-                if (gamma * gamma > settled2 * alpha * beta) flags[sweep & 1] = 1;
+                if (above(gamma, alpha, beta, settled)) flags[sweep & 1] = 1;
                 const int at = atomicAdd(flags + 4, 1);
                 list[at] = static_cast<int>(t);
                 lc[at] = c;
@@ -436,7 +468,7 @@ namespace ttg
                 gamma = group_sum<T, G>(gamma);
                 if (!pair) continue;
                 const T alpha = norms[p], beta = norms[q];
-                if (gamma * gamma <= tol2 * alpha * beta) continue;
+                if (!above(gamma, alpha, beta, least)) continue;
                 float cf, sf;
                 if (!angle(alpha, beta, gamma, cf, sf)) continue;
                 T c, sn;
@@ -448,7 +480,7 @@ namespace ttg
                   const T cc = c * c, ss = sn * sn, cs2 = 2 * c * sn * gamma;
                   norms[p] = cc * alpha - cs2 + ss * beta;
                   norms[q] = ss * alpha + cs2 + cc * beta;
-                  if (gamma * gamma > settled2 * alpha * beta) flags[sweep & 1] = 1;
+                  if (above(gamma, alpha, beta, settled)) flags[sweep & 1] = 1;
                 }
               }
             }
@@ -476,6 +508,254 @@ namespace ttg
       if (most <= 8 * kNper) return sweeps<T, 8>(cluster, alone, w, rows, v, vrows, k, tol, norms, exchange, partial, flags, list);
       if (most <= 16 * kNper) return sweeps<T, 16>(cluster, alone, w, rows, v, vrows, k, tol, norms, exchange, partial, flags, list);
       return sweeps<T, 32>(cluster, alone, w, rows, v, vrows, k, tol, norms, exchange, partial, flags, list);
+    }
+
+    // FP32 sweeps in blocks of four columns.  W (k columns of at most 32 NR rows) and V (k x k) lie in the
+    // cluster's shared memory, block b with rank b % ranks, columns 32 NR apart and zero-padded, k padded
+    // to whole pairs of blocks with zero columns.  A warp takes a pair of blocks into registers (a lane
+    // holds NR rows of each of the eight columns), rotates the sixteen pairs across the blocks four
+    // disjoint ones at a time (the first round also the pairs within each block), and puts the columns
+    // back; the rotations are accumulated as an 8 x 8 matrix (lane i its row i) and applied to the
+    // block's columns of V as one product.  A sweep is one cluster barrier per round of block pairs, a
+    // quarter as many rounds as columns, and the pairs of a round are dealt to all ranks.  The four dot
+    // products of a step are reduced together, each lane group of eight ending with one of them and
+    // finding its angle.  Returns the sweeps, -1 beyond kMaxSweeps.
+    template <int NR>
+    __device__ int blocked_sweeps(const cg::cluster_group &cluster, float *w, float *v, int k, float tol, float *jbuf, int *flags)
+    {
+      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+      const int ranks = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+      const int blocks = (k + 7) / 8 * 2;
+      const float settled = sqrtf(tol);
+      float *jm = jbuf + warp * 64;
+      const auto sync = [&] {
+        if (ranks == 1) __syncthreads();
+        else cluster.sync();
+      };
+      const auto at_home = [&](float *base, int b) -> float * {
+        float *here = base + static_cast<int64_t>(b / ranks) * 4 * 32 * NR;
+        return ranks == 1 ? here : cluster.map_shared_rank(here, static_cast<unsigned>(b % ranks));
+      };
+      for (int sweep = 0; sweep < kMaxSweeps; ++sweep)
+      {
+        if (threadIdx.x == 0) flags[sweep & 1] = 0;
+        sync();
+        for (int round = 0; round + 1 < blocks; ++round)
+        {
+          for (int bp = rank + warp * ranks; bp < blocks / 2; bp += warps * ranks)
+          {
+            int64_t bl, br;
+            circle_pair(round, bp, blocks, bl, br);
+            float *left = at_home(w, static_cast<int>(bl)), *right = at_home(w, static_cast<int>(br));
+            float x[8][NR + 1];
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+            {
+              const float *from = (c < 4 ? left + c * 32 * NR : right + (c - 4) * 32 * NR) + lane;
+#pragma unroll
+              for (int r = 0; r < NR; ++r) x[c][r] = from[r * 32];
+              x[c][NR] = lane == c ? 1.0f : 0.0f;
+            }
+            // the columns of V on their way meanwhile, where registers allow
+            constexpr bool kAhead = NR <= 3;
+            float *vl = at_home(v, static_cast<int>(bl)) + lane, *vr = at_home(v, static_cast<int>(br)) + lane;
+            float held[kAhead ? NR : 1][8];
+            if constexpr (kAhead)
+            {
+#pragma unroll
+              for (int r = 0; r < NR; ++r)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) held[r][i] = (i < 4 ? vl + i * 32 * NR : vr + (i - 4) * 32 * NR)[r * 32];
+            }
+            // squared norms: eight sums reduced together (lane bits 4..2 end with column 4 b4 + 2 b3 + b2)
+            float n2[8];
+            {
+              float p[8];
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+              {
+                p[c] = 0.0f;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) p[c] = fmaf(x[c][r], x[c][r], p[c]);
+              }
+#pragma unroll
+              for (int half = 4, bit = 16; half > 0; half >>= 1, bit >>= 1)
+#pragma unroll
+                for (int c = 0; c < half; ++c)
+                {
+                  const bool high = lane & bit;
+                  const float give = high ? p[c] : p[c + half], keep = high ? p[c + half] : p[c];
+                  p[c] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+              p[0] += __shfl_xor_sync(0xffffffffu, p[0], 2);
+              p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
+#pragma unroll
+              for (int c = 0; c < 8; ++c) n2[c] = __shfl_sync(0xffffffffu, p[0], c * 4);
+            }
+            bool any = false, large = false;
+            // four disjoint pairs (pc[i], qc[i])
+            const auto rotate4 = [&](const int (&pc)[4], const int (&qc)[4]) {
+              float g[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+              {
+                g[i] = 0.0f;
+#pragma unroll
+                for (int r = 0; r < NR; ++r) g[i] = fmaf(x[pc[i]][r], x[qc[i]][r], g[i]);
+              }
+#pragma unroll
+              for (int half = 2, bit = 16; half > 0; half >>= 1, bit >>= 1)
+#pragma unroll
+                for (int i = 0; i < half; ++i)
+                {
+                  const bool high = lane & bit;
+                  const float give = high ? g[i] : g[i + half], keep = high ? g[i + half] : g[i];
+                  g[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+#pragma unroll
+              for (int off = 4; off > 0; off >>= 1) g[0] += __shfl_xor_sync(0xffffffffu, g[0], off);
+              // lanes 8 i .. 8 i + 7 hold pair i's product
+              const int mine = lane >> 3;
+              float alpha = n2[pc[0]], beta = n2[qc[0]];
+#pragma unroll
+              for (int i = 1; i < 4; ++i)
+              {
+                alpha = mine == i ? n2[pc[i]] : alpha;
+                beta = mine == i ? n2[qc[i]] : beta;
+              }
+              const float cosine = fabsf(g[0]) * rsqrtf(alpha) * rsqrtf(beta);
+              float c = 1.0f, sn = 0.0f;
+              const bool turn = cosine > tol && angle_fast(beta - alpha, g[0], c, sn);
+              if (!turn)
+              {
+                c = 1.0f;
+                sn = 0.0f;
+              }
+              const float cc = c * c, ss = sn * sn, cs2 = 2.0f * c * sn * g[0];
+              const float na = turn ? cc * alpha - cs2 + ss * beta : alpha, nb = turn ? ss * alpha + cs2 + cc * beta : beta;
+              if (!__any_sync(0xffffffffu, turn)) return;
+              any = true;
+              large = large || cosine > settled;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+              {
+                const float ci = __shfl_sync(0xffffffffu, c, 8 * i), si = __shfl_sync(0xffffffffu, sn, 8 * i);
+                n2[pc[i]] = __shfl_sync(0xffffffffu, na, 8 * i);
+                n2[qc[i]] = __shfl_sync(0xffffffffu, nb, 8 * i);
+#pragma unroll
+                for (int r = 0; r <= NR; ++r)
+                {
+                  const float p = x[pc[i]][r], q = x[qc[i]][r];
+                  x[pc[i]][r] = fmaf(ci, p, -si * q);
+                  x[qc[i]][r] = fmaf(si, p, ci * q);
+                }
+              }
+            };
+            if (round == 0)
+            {
+              rotate4({0, 2, 4, 6}, {1, 3, 5, 7});
+              rotate4({0, 1, 4, 5}, {2, 3, 6, 7});
+              rotate4({0, 1, 4, 5}, {3, 2, 7, 6});
+            }
+            rotate4({0, 1, 2, 3}, {4, 5, 6, 7});
+            rotate4({0, 1, 2, 3}, {5, 6, 7, 4});
+            rotate4({0, 1, 2, 3}, {6, 7, 4, 5});
+            rotate4({0, 1, 2, 3}, {7, 4, 5, 6});
+            if (__any_sync(0xffffffffu, large) && lane == 0) flags[sweep & 1] = 1;
+            if (!any) continue;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+            {
+              float *to = (c < 4 ? left + c * 32 * NR : right + (c - 4) * 32 * NR) + lane;
+#pragma unroll
+              for (int r = 0; r < NR; ++r) to[r * 32] = x[c][r];
+              if (lane < 8) jm[lane * 8 + c] = x[c][NR];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+            {
+              float out[8] = {};
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+              {
+                float in;
+                if constexpr (kAhead) in = held[r][i];
+                else in = (i < 4 ? vl + i * 32 * NR : vr + (i - 4) * 32 * NR)[r * 32];
+                const float4 lo = *reinterpret_cast<const float4 *>(jm + i * 8), hi = *reinterpret_cast<const float4 *>(jm + i * 8 + 4);
+                out[0] = fmaf(in, lo.x, out[0]);
+                out[1] = fmaf(in, lo.y, out[1]);
+                out[2] = fmaf(in, lo.z, out[2]);
+                out[3] = fmaf(in, lo.w, out[3]);
+                out[4] = fmaf(in, hi.x, out[4]);
+                out[5] = fmaf(in, hi.y, out[5]);
+                out[6] = fmaf(in, hi.z, out[6]);
+                out[7] = fmaf(in, hi.w, out[7]);
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) (i < 4 ? vl + i * 32 * NR : vr + (i - 4) * 32 * NR)[r * 32] = out[i];
+            }
+            __syncwarp();
+          }
+          sync();
+        }
+        int more = threadIdx.x < ranks ? *cluster.map_shared_rank(flags + (sweep & 1), threadIdx.x) : 0;
+        if (!__syncthreads_or(more)) return sweep + 1;
+      }
+      return -1;
+    }
+    constexpr int kBlockedRows = 320;  // the longest columns of blocked_sweeps
+
+    __device__ int blocked_sweeps(const cg::cluster_group &cluster, float *w, float *v, int k, int nr, float tol, float *jbuf, int *flags)
+    {
+      switch (nr)
+      {
+      case 1: return blocked_sweeps<1>(cluster, w, v, k, tol, jbuf, flags);
+      case 2: return blocked_sweeps<2>(cluster, w, v, k, tol, jbuf, flags);
+      case 3: return blocked_sweeps<3>(cluster, w, v, k, tol, jbuf, flags);
+      case 4: return blocked_sweeps<4>(cluster, w, v, k, tol, jbuf, flags);
+      case 5: return blocked_sweeps<5>(cluster, w, v, k, tol, jbuf, flags);
+      case 6: return blocked_sweeps<6>(cluster, w, v, k, tol, jbuf, flags);
+      case 8: return blocked_sweeps<8>(cluster, w, v, k, tol, jbuf, flags);
+      default: return blocked_sweeps<10>(cluster, w, v, k, tol, jbuf, flags);
+      }
+    }
+
+    // out(i, j) = sum_x a(x, i) b(x, j) over a 16 x 16 tile, x < depth, staged 32 of x at a time (the next
+    // stage's reads in flight during this one's products), each thread half the depth of one entry.
+    // Small tiles deal evenly over a cluster; FP64 issue is the bound.  The loaders are called with x
+    // fastest across the threads when `x_fast`, else i (or j) fastest.
+    constexpr int kSmallTile = 16, kSmallDepth = 32, kSmallPitch = kSmallTile + 1;
+    constexpr int64_t kSmallBytes = 2 * kSmallDepth * kSmallPitch * 8;
+    template <typename Acc, typename FA, typename FB, typename Out>
+    __device__ void small_product(int64_t depth, FA fa, bool a_x_fast, FB fb, bool b_x_fast, void *stage, Out out)
+    {
+      Acc *sa = static_cast<Acc *>(stage), *sb = sa + kSmallDepth * kSmallPitch;
+      const int t = threadIdx.x, i = t & 15, j = (t >> 4) & 15, half = t >> 8;
+      const int xa = a_x_fast ? t & 31 : t >> 4, ia = a_x_fast ? t >> 5 : t & 15;
+      const int xb = b_x_fast ? t & 31 : t >> 4, jb = b_x_fast ? t >> 5 : t & 15;
+      Acc acc = 0;
+      Acc na = xa < depth ? static_cast<Acc>(fa(xa, ia)) : Acc(0), nb = xb < depth ? static_cast<Acc>(fb(xb, jb)) : Acc(0);
+      for (int64_t x0 = 0; x0 < depth; x0 += kSmallDepth)
+      {
+        sa[xa * kSmallPitch + ia] = na;
+        sb[xb * kSmallPitch + jb] = nb;
+        __syncthreads();
+        const int64_t x1 = x0 + kSmallDepth;
+        if (x1 < depth)
+        {
+          na = x1 + xa < depth ? static_cast<Acc>(fa(x1 + xa, ia)) : Acc(0);
+          nb = x1 + xb < depth ? static_cast<Acc>(fb(x1 + xb, jb)) : Acc(0);
+        }
+#pragma unroll
+        for (int x = 0; x < kSmallDepth / 2; ++x)
+          acc = fma(sa[(half * 16 + x) * kSmallPitch + i], sb[(half * 16 + x) * kSmallPitch + j], acc);
+        __syncthreads();
+      }
+      if (half == 1) sa[j * kSmallPitch + i] = acc;
+      __syncthreads();
+      if (half == 0) out(i, j, acc + sa[j * kSmallPitch + i]);
+      __syncthreads();
     }
 
     // out(i, j) = sum_x a(x, i) b(x, j) + c(i, j) over a kTile x kTile tile, x < depth, staged
@@ -514,10 +794,8 @@ namespace ttg
     }
 
     // A thread-block cluster of up to 16 CTAs per block (grid = blocks x cluster size, the largest
-    // blocks first).  The FP32 sweeps run on rank 0 alone when its working set fits in shared
-    // memory (a cluster barrier per round would cost more than it saves), else over the cluster;
-    // the cluster shares the Newton-Schulz steps and W = A V as 32 x 32 tiles; the FP64 sweeps run
-    // over the cluster for blocks of 32 columns or more, on rank 0 alone for smaller ones.
+    // blocks first).  The FP64 sweeps, when they run, run over the cluster for blocks of 32 columns or
+    // more, on rank 0 alone for smaller ones.
     __global__ void __launch_bounds__(kSvdThreads, 1)
       jacobi_svd_kernel(const SvdEntry *__restrict__ table, const double *__restrict__ a, double *__restrict__ u,
                         double *__restrict__ s, double *__restrict__ vh, double *__restrict__ workspace,
@@ -529,6 +807,7 @@ namespace ttg
       __shared__ int rank_of[kMaxCols];
       __shared__ int flags[5];  // [0], [1]: a sweep rotated above sqrt(tol), by sweep parity; [4]: the rotations listed in a round
       __shared__ double big;
+      __shared__ double taus[2];
       const cg::cluster_group cluster = cg::this_cluster();
       const unsigned ranks = cluster.num_blocks(), rank = cluster.block_rank();
       const int64_t block = blockIdx.x / ranks;
@@ -549,15 +828,15 @@ namespace ttg
       const auto entry_a = [&](int64_t row, int64_t col) -> double
       { return wide ? src[col * n + row] : src[row * n + col]; };  // row < len, col < k
 
-      // 0. Preconditioning (blocks swept over a cluster): the columns sorted by norm, largest
+      // 0. Preconditioning: the columns sorted by norm, largest
       // first, and factored A P = Q R by Householder reflections; the sweeps then run on X = R^T
       // (k x k), whose graded columns the FP32 sweeps orthogonalise in about a third of the
       // sweeps the block itself takes (Drmac & Veselic, "New fast and accurate Jacobi SVD
       // algorithm", SIAM J. Matrix Anal. Appl. 29 (2008), with the pivoting of their QR replaced by
       // the one sort).  The factors of X give those of A: A P = (Q J) S (U_x)^T with X J = U_x S.
-      // Rank r owns the factored columns [q0, q1) (and so the rows [q0, q1) of X, which are its
-      // rows of the sweeps).
-      const bool precond = ranks > 1 && k >= kQrMinCols;
+      // The columns are dealt to the ranks in turn while they are factored; at the end rank r transforms
+      // columns [q0, q1) of the left factor.
+      const bool precond = k >= kQrMinCols;
       double *qf = ws + lay.f, *qtau = ws + lay.tau, *qb = ws + lay.b;
       int64_t *qorder = reinterpret_cast<int64_t *>(ws + lay.order);
       const int64_t cpr = (k + ranks - 1) / ranks;
@@ -588,79 +867,125 @@ namespace ttg
         __syncthreads();
         // this rank's columns in shared memory while they are factored when they fit (else in the
         // global factored matrix); each reflector goes to the global one as it is made
-        const bool qr_smem = (cpr + 1) * len * 8 <= kDynamicBytes;
+        const bool qr_smem = (cpr + 2) * len * 8 <= kDynamicBytes;
         double *own = reinterpret_cast<double *>(dynamic);
-        double *vst = qr_smem ? own + cpr * len : own;  // the reflector of the step, staged
-        const auto colp = [&](int64_t c) -> double * { return qr_smem ? own + (c - q0) * len : qf + c * len; };
-        for (int64_t c = q0; c < q1; ++c)
+        double *vst = qr_smem ? own + cpr * len : own;  // the reflectors of two steps in turn (when they fit)
+        const bool push = qr_smem || 2 * len * 8 <= kDynamicBytes;
+        const auto colp = [&](int64_t c) -> double * { return qr_smem ? own + (c / ranks) * len : qf + c * len; };
+        for (int64_t c = rank; c < k; c += ranks)
         {
           const int64_t from = rank_of[c];
           double *to = colp(c);
           for (int64_t i = threadIdx.x; i < len; i += blockDim.x) to[i] = entry_a(i, from);
           if (threadIdx.x == 0) qorder[c] = from;
         }
-        __syncthreads();
-        // step j: the owner of column j makes its reflector (as LAPACK's dlarfg: H = I - tau v v^T,
-        // v_0 = 1, R_jj = beta) and publishes it, the cluster waits for it, and every rank applies
-        // it to its own columns right of j, a warp per column, with v staged in shared memory
+        cluster.sync();
+        // Step j: the owner of column j has made its reflector (as LAPACK's dlarfg: H = I - tau v v^T, v_0 = 1,
+        // R_jj = beta) and pushed it into every rank's shared memory; a warp per column right of j
+        // applies it.  The warp that holds column j + 1 does that column first and makes its reflector
+        // at once, so a step is one cluster barrier and one warp's chain of a dot product, the update,
+        // the norm and the scalars (the columns are dealt in turn, so that every rank has columns to the end).
+        const auto reflect = [&](int64_t j, double xn) {
+          // by one warp, xn the squared norm of column j below its diagonal
+          double *col = colp(j);
+          const double alpha = col[j];
+          double beta = alpha, tau = 0.0, scale = 0.0;
+          if (xn > 0.0)
+          {
+            const double norm2 = fma(alpha, alpha, xn), inv = rsqrt(norm2), norm = norm2 * inv;
+            const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
+            beta = -copysign(norm, alpha);
+            tau = fabs(d) * inv;                             // (beta - alpha) / beta
+            scale = 1.0 / d;
+          }
+          __syncwarp();
+          double *slot = vst + (j & 1) * len;
+          for (int64_t i = j + 1 + lane; i < len; i += 32)
+          {
+            const double x = col[i] * scale;
+            col[i] = x;
+            qf[j * len + i] = x;
+            if (push)
+              for (unsigned r = 0; r < ranks; ++r) cluster.map_shared_rank(slot, r)[i] = x;
+          }
+          if (lane == 0)
+          {
+            col[j] = beta;
+            qf[j * len + j] = beta;
+            qtau[j] = tau;
+            for (unsigned r = 0; r < ranks; ++r) cluster.map_shared_rank(taus, r)[j & 1] = tau;
+          }
+        };
+        if (rank == 0 && warp == 0)
+        {
+          const double *col = colp(0);
+          double xn = 0.0;
+          for (int64_t i = 1 + lane; i < len; i += 32) xn = fma(col[i], col[i], xn);
+          reflect(0, warp_sum(xn));
+        }
         for (int64_t j = 0; j < k; ++j)
         {
-          if (j >= q0 && j < q1)
+          cluster.sync();
+          const double *v = vst + (j & 1) * len;
+          if (!push)
           {
-            double *col = colp(j);
-            double part = 0.0;
-            for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x) part = fma(col[i], col[i], part);
-            part = warp_sum(part);
-            if (lane == 0) norms_raw[warp] = part;
-            __syncthreads();
-            if (threadIdx.x == 0)
+            v = qf + j * len;  // too long for shared memory: read through L2
+          }
+          const double tau = taus[j & 1];
+          // FP64 issue is what a step is made of (a warp instruction in 64 clocks a quarter of the SM): column
+          // j + 1 has warp 0 and its quarter to itself, the others go four to a warp, eight lanes a column
+          // (three shuffled additions for the four dot products instead of five each), on the other quarters.
+          const auto vi = [&](int64_t i) { return push ? v[i] : __ldcg(v + i); };
+          const int64_t first = (j + 1 + ranks - 1 - rank) / ranks;  // the first local column c with c ranks + rank > j
+          const bool next = (j + 1) % ranks == rank;                 // it is column j + 1
+          if (warp == 0)
+          {
+            if (next && j + 1 < k)
             {
-              double xn = 0.0;
-              for (int w = 0; w < warps; ++w) xn += norms_raw[w];
-              const double alpha = col[j];
-              double beta = alpha, tau = 0.0, scale = 0.0;
-              if (xn > 0.0)
+              double *fc = colp(j + 1), xn = 0.0;
+              if (tau != 0.0)
               {
-                const double norm = sqrt(fma(alpha, alpha, xn));
-                const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
-                beta = -copysign(norm, alpha);
-                tau = -d / beta;                                 // (beta - alpha) / beta
-                scale = 1.0 / d;
+                double dot = 0.0;
+                for (int64_t i = j + 1 + lane; i < len; i += 32) dot = fma(vi(i), fc[i], dot);
+                dot = warp_sum(dot);
+                const double wt = tau * (fc[j] + dot);
+                for (int64_t i = j + 1 + lane; i < len; i += 32)
+                {
+                  const double x = fma(-wt, vi(i), fc[i]);
+                  fc[i] = x;
+                  if (i > j + 1) xn = fma(x, x, xn);
+                }
+                __syncwarp();
+                if (lane == 0) fc[j] -= wt;
               }
-              col[j] = beta;
-              qf[j * len + j] = beta;
-              qtau[j] = tau;
-              big = scale;
-            }
-            __syncthreads();
-            const double scale = big;
-            for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x)
-            {
-              const double x = col[i] * scale;
-              col[i] = x;
-              qf[j * len + i] = x;
+              else
+                for (int64_t i = j + 2 + lane; i < len; i += 32) xn = fma(fc[i], fc[i], xn);
+              __syncwarp();
+              reflect(j + 1, warp_sum(xn));
             }
           }
-          cluster.sync();
-          for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x) vst[i] = __ldcg(qf + j * len + i);
-          __syncthreads();
-          const double tau = __ldcg(qtau + j);
-          if (tau != 0.0)
-            for (int64_t c = max(q0, j + 1) + warp; c < q1; c += warps)
+          else if ((warp & 3) != 0 && tau != 0.0)
+          {
+            const int slot = (warp >> 2) * 3 + (warp & 3) - 1, lanes = lane & 7;
+            for (int64_t l0 = first + (next ? 1 : 0) + slot * 4; l0 * ranks + rank < k; l0 += (warps >> 2) * 12)
             {
-              double *fc = colp(c);
-              double dot = 0.0;
-              for (int64_t i = j + 1 + lane; i < len; i += 32) dot = fma(vst[i], fc[i], dot);
-              dot = warp_sum(dot);
-              const double w = tau * (fc[j] + dot);
-              for (int64_t i = j + 1 + lane; i < len; i += 32) fc[i] = fma(-w, vst[i], fc[i]);
-              if (lane == 0) fc[j] -= w;
+              const int64_t c = (l0 + (lane >> 3)) * ranks + rank;
+              const bool live = c < k;
+              double *fc = colp(live ? c : l0 * ranks + rank), dot = 0.0;
+              for (int64_t i = j + 1 + lanes; i < len; i += 8) dot = fma(vi(i), fc[i], dot);
+              dot = group_sum<double, 8>(dot);
+              const double head = fc[j], wt = tau * (head + dot);
+              __syncwarp();
+              if (!live) continue;
+              for (int64_t i = j + 1 + lanes; i < len; i += 8) fc[i] = fma(-wt, vi(i), fc[i]);
+              if (lanes == 0) fc[j] = head - wt;
             }
-          __syncthreads();
+          }
         }
+        __syncthreads();
         // R's part of this rank's columns to the global factored matrix
         if (qr_smem)
-          for (int64_t c = q0; c < q1; ++c)
+          for (int64_t c = rank; c < k; c += ranks)
             for (int64_t i = threadIdx.x; i <= c && i < len; i += blockDim.x) qf[c * len + i] = colp(c)[i];
         cluster.sync();
       }
@@ -670,7 +995,39 @@ namespace ttg
       { return precond ? (col <= row ? __ldcg(qf + row * len + col) : 0.0) : entry_a(row, col); };  // row < xl
 
       // 1. FP32 sweeps on the block scaled to |entries| <= 1, from V = I; V goes out in FP64.
-      // Rank 0 alone when W and V fit in its shared memory, else rows dealt over the cluster.
+      // In blocks of columns over the cluster when W and V fit in its shared memory (columns of up to
+      // 320), else column by column with the rows dealt over the cluster.
+      const int rows32 = static_cast<int>((max(xl, k) + 31) / 32), nr = rows32 <= 6 ? rows32 : rows32 <= 8 ? 8 : 10;
+      const int64_t column_blocks = (k + 7) / 8 * 2, mine = (column_blocks + ranks - 1) / ranks, ld32 = 32 * nr;
+      const bool blocked = max(xl, k) <= kBlockedRows && (2 * mine * 4 * ld32 + 64 * (kSvdThreads / 32)) * 4 <= kDynamicBytes;
+      if (blocked)
+      {
+        float *w32 = reinterpret_cast<float *>(dynamic), *v32 = w32 + mine * 4 * ld32, *jbuf = v32 + mine * 4 * ld32;
+        if (threadIdx.x == 0) big = 0.0;
+        __syncthreads();
+        double local = 0.0;
+        for (int64_t i = threadIdx.x; i < xl * k; i += blockDim.x) local = fmax(local, fabs(entry(i % xl, i / xl)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) local = fmax(local, __shfl_xor_sync(0xffffffffu, local, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned long long *>(&big), __double_as_longlong(local));
+        __syncthreads();
+        const double scale = big > 0.0 ? 1.0 / big : 1.0;
+        // place i of this rank's columns: column 4 (rank + ranks b) + c of block b here
+        const auto column_of = [&](int64_t i) { return ((i / ld32 / 4) * ranks + rank) * 4 + i / ld32 % 4; };
+        for (int64_t i = threadIdx.x; i < mine * 4 * ld32; i += blockDim.x)
+        {
+          const int64_t row = i % ld32, col = column_of(i);
+          w32[i] = row < xl && col < k ? static_cast<float>(entry(row, col) * scale) : 0.0f;
+          v32[i] = row == col && col < k ? 1.0f : 0.0f;
+        }
+        blocked_sweeps(cluster, w32, v32, static_cast<int>(k), nr, 1e-5f, jbuf, flags);
+        for (int64_t i = threadIdx.x; i < mine * 4 * ld32; i += blockDim.x)
+        {
+          const int64_t row = i % ld32, col = column_of(i);
+          if (row < k && col < k) v_cur[col * k + row] = static_cast<double>(v32[i]);
+        }
+      }
+      else
       {
         const bool alone = ranks == 1 || (k < 32 && (xl * k + k * k) * 4 <= kDynamicBytes);
         const int64_t rows = alone ? xl : (xl + ranks - 1) / ranks, vrows = alone ? k : (k + ranks - 1) / ranks;
@@ -733,13 +1090,139 @@ namespace ttg
       }
       cluster.sync();
 
-      // 2. V orthonormal to FP64 precision by two Newton-Schulz steps V <- V + V (I - V^T V) / 2:
+      // 2. V refined in FP64 with matrix products: W = X V, its Gram matrix G = W^T W and H = V^T V say how
+      // far every pair of columns is from orthogonal; V <- V + V E with E_rc = t_rc - h_rc / 2, t the tangent
+      // of the pair's Jacobi angle (from G with V's own non-orthogonality taken out) and the rest the
+      // Newton-Schulz step, takes cosines of 1e-5 to 1e-9 and then to round-off (all pairs at once, the
+      // idea of T. Ogita and K. Aishima, "Iterative refinement for symmetric eigenvalue decomposition",
+      // Japan J. Indust. Appl. Math. 35 (2018), on the one-sided form, whose graded columns keep their
+      // relative accuracy).  E has to be good only to FP32, so V E is an FP32 product.  Done when no
+      // cosine is above tol and V is orthonormal to it (or, from the fourth time on, both stand at the
+      // round-off of W = X V, within four times that).  Pairs whose angle is not small (close singular values
+      // that FP32 left mixed) are left out; when there are some after the first time, or it does not
+      // settle, the FP64 sweeps below take over.  Against the 3 to 6 FP64 sweeps of 0.7 ms each that it
+      // replaces, a step is about 0.1 ms at 148 columns.
+      const double tol = 2.220446049250313e-16 * sqrt(static_cast<double>(xl));
+      double *wg = qb, *hm = ws + lay.w_slices;
+      float *em = reinterpret_cast<float *>(ws + lay.v_slices);
+      void *small_stage = dynamic + kDynamicBytes - kSmallBytes;
+      double *v_start = ws + lay.w32_slices;  // V as FP32 left it, for the sweeps should they run (k x k)
+      bool refined = false;
+      int refinements = 0;
+      for (int64_t i = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x; i < k * k; i += static_cast<int64_t>(ranks) * blockDim.x)
+        v_start[i] = __ldcg(v_cur + i);
+      for (int it = 0; it < 7 && !refined; ++it)
+      {
+        const double *vc = v_cur;
+        const int64_t nrow = (xl + kSmallTile - 1) / kSmallTile, ncol = (k + kSmallTile - 1) / kSmallTile;
+        for (int64_t tile = rank; tile < nrow * ncol; tile += ranks)
+        {
+          // the deepest tiles of the triangular X first
+          const int64_t tr = nrow - 1 - tile / ncol, tc = tile % ncol;
+          small_product<double>(
+            precond ? min(k, (tr + 1) * kSmallTile) : k,
+            [&](int64_t x, int i) { const int64_t row = tr * kSmallTile + i; return row < xl ? entry(row, x) : 0.0; }, precond || !wide,
+            [&](int64_t x, int j) { return tc * kSmallTile + j < k ? __ldcg(vc + (tc * kSmallTile + j) * k + x) : 0.0; }, true, small_stage,
+            [&](int i, int j, double sum) {
+              const int64_t row = tr * kSmallTile + i, c = tc * kSmallTile + j;
+              if (row < xl && c < k) wg[c * xl + row] = sum;
+            });
+        }
+        cluster.sync();
+        int64_t turn = 0;
+        for (int which = 0; which < 2; ++which)
+          for (int64_t tr = 0; tr < ncol; ++tr)
+            for (int64_t tc = tr; tc < ncol; ++tc, ++turn)
+            {
+              if (turn % ranks != rank) continue;
+              const double *m = which == 0 ? wg : vc;
+              double *to = which == 0 ? g : hm;
+              const int64_t ld = which == 0 ? xl : k;
+              small_product<double>(
+                ld, [&](int64_t x, int i) { return tr * kSmallTile + i < k ? __ldcg(m + (tr * kSmallTile + i) * ld + x) : 0.0; }, true,
+                [&](int64_t x, int j) { return tc * kSmallTile + j < k ? __ldcg(m + (tc * kSmallTile + j) * ld + x) : 0.0; }, true, small_stage,
+                [&](int i, int j, double sum) {
+                  const int64_t r = tr * kSmallTile + i, c = tc * kSmallTile + j;
+                  if (r < k && c < k && r <= c) to[c * k + r] = sum;
+                });
+            }
+        cluster.sync();
+        for (int64_t j = threadIdx.x; j < k; j += blockDim.x) norms_raw[j] = __ldcg(g + j * k + j);
+        __syncthreads();
+        int status = 0;  // 1: a cosine above tol, 2: V off by more, 4: an angle that is not small, 8: either above four times tol
+        for (int64_t i = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x; i < k * k; i += static_cast<int64_t>(ranks) * blockDim.x)
+        {
+          const int64_t c = i / k, r = i - c * k;
+          if (r > c) continue;
+          const double h = __ldcg(hm + i);
+          if (r == c)
+          {
+            const double off = 1.0 - h;
+            em[i] = static_cast<float>(0.5 * off);
+            if (!(fabs(off) <= tol + 1e-15)) status |= fabs(off) <= 4.0 * tol ? 2 : 10;
+            continue;
+          }
+          const double gamma = __ldcg(g + i), lr = norms_raw[r], lc = norms_raw[c];
+          if (!(fabs(h) <= tol + 1e-15)) status |= fabs(h) <= 4.0 * tol ? 2 : 10;
+          const double limit = tol * tol * lr * lc, square = gamma * gamma;
+          if (!(square <= limit)) status |= square <= 16.0 * limit ? 1 : 9;
+          const double st = fma(-0.5 * h, lr + lc, gamma);
+          float cf, sf;
+          double tangent = 0.0;
+          if (angle(lr, lc, st, cf, sf))
+          {
+            const float tf = sf / cf;
+            if (fabsf(tf) > 0.1f) status |= 4;
+            else tangent = tf;
+          }
+          em[c * k + r] = static_cast<float>(fma(-0.5, h, tangent));
+          em[r * k + c] = static_cast<float>(fma(-0.5, h, -tangent));
+        }
+        status = (__syncthreads_or(status & 1) ? 1 : 0) | (__syncthreads_or(status & 2) ? 2 : 0) | (__syncthreads_or(status & 4) ? 4 : 0) |
+                 (__syncthreads_or(status & 8) ? 8 : 0);
+        if (threadIdx.x == 0) flags[2] = status;
+        cluster.sync();
+        status = 0;
+        for (unsigned r = 0; r < ranks; ++r) status |= cluster.map_shared_rank(flags, r)[2];
+        refinements = it + 1;
+        if (!(status & 3) || (it >= 3 && !(status & 8)))
+        {
+          refined = true;
+          break;
+        }
+        if ((it >= 1 && (status & 4)) || it == 6) break;
+        for (int64_t tile = rank; tile < ncol * ncol; tile += ranks)
+        {
+          const int64_t tr = tile / ncol, tc = tile % ncol;
+          small_product<float>(
+            k, [&](int64_t x, int i) { return tr * kSmallTile + i < k ? static_cast<float>(__ldcg(vc + x * k + tr * kSmallTile + i)) : 0.0f; }, false,
+            [&](int64_t x, int j) { return tc * kSmallTile + j < k ? __ldcg(em + (tc * kSmallTile + j) * k + x) : 0.0f; }, true, small_stage,
+            [&](int i, int j, float sum) {
+              const int64_t row = tr * kSmallTile + i, c = tc * kSmallTile + j;
+              if (row < k && c < k) v_next[c * k + row] = __ldcg(vc + c * k + row) + static_cast<double>(sum);
+            });
+        }
+        cluster.sync();
+        double *t = v_cur;
+        v_cur = v_next;
+        v_next = t;
+      }
+      // no rank writes over what another still reads of the statuses
+      cluster.sync();
+      if (!refined)
+      {
+        for (int64_t i = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x; i < k * k; i += static_cast<int64_t>(ranks) * blockDim.x)
+          v_cur[i] = __ldcg(v_start + i);
+        cluster.sync();
+      }
+
+      // 3. (when the refinement did not settle) V orthonormal to FP64 precision by two Newton-Schulz steps V <- V + V (I - V^T V) / 2:
       // G = V^T V in FP64 (the tiles on and above the diagonal), the correction V E, E = I - G of
       // size ~1e-6 and then ~1e-12, in FP32 accumulation (its rounding, ~1e-7 of E, is below FP64
       // precision of V after the second step).  Tiles are dealt to the ranks; V and G pass between
       // the CTAs through the workspace, read past L1 (__ldcg) so that no CTA sees an earlier value.
       const int64_t nt = (k + kTile - 1) / kTile;
-      for (int step = 0; step < 2; ++step)
+      for (int step = 0; step < (refined ? 0 : 2); ++step)
       {
         for (int64_t tile = rank; tile < nt * nt; tile += ranks)
         {
@@ -784,8 +1267,8 @@ namespace ttg
         v_next = t;
       }
 
-      // 3. this rank's rows of W = A V (FP64) and of V.  FP64 sweeps over the cluster for 32
-      // columns or more, on rank 0 alone below that.
+      // this rank's rows of W = A V (FP64) and of V.  FP64 sweeps over the cluster for 32 columns or
+      // more, on rank 0 alone below that.
       const bool alone = ranks == 1 || k < 32;
       const int64_t rows = alone ? (rank == 0 ? xl : 0) : (xl + ranks - 1) / ranks;
       const int64_t vrows = alone ? (rank == 0 ? k : 0) : (k + ranks - 1) / ranks;
@@ -797,10 +1280,16 @@ namespace ttg
       double *v = slices_in_smem ? w + rows * k : ws + lay.v_slices + static_cast<int64_t>(rank) * vrows * k;
       {
         const double *vc = v_cur;
-        const int64_t nr = (rows + kTile - 1) / kTile;
-        for (int64_t tile = 0; tile < nr * nt; ++tile)
+        if (refined)
+          for (int64_t i = threadIdx.x; i < rows * k; i += blockDim.x)
+          {
+            const int64_t row = r0 + i % rows;
+            w[i] = row < r1 ? __ldcg(wg + (i / rows) * xl + row) : 0.0;
+          }
+        const int64_t row_tiles = refined ? 0 : (rows + kTile - 1) / kTile;
+        for (int64_t tile = 0; tile < row_tiles * nt; ++tile)
         {
-          const int64_t tr = tile % nr, tc = tile / nr;
+          const int64_t tr = tile % row_tiles, tc = tile / row_tiles;
           tile_product<double>(
             k, [&](int64_t x, int i) { const int64_t row = r0 + tr * kTile + i; return row < r1 ? entry(row, x) : 0.0; }, precond || !wide,
             [&](int64_t x, int j) { return tc * kTile + j < k ? __ldcg(vc + (tc * kTile + j) * k + x) : 0.0; }, true,
@@ -819,9 +1308,8 @@ namespace ttg
       }
 
       // 4. FP64 sweeps
-      const double tol = 2.220446049250313e-16 * sqrt(static_cast<double>(xl));
-      int sweeps_taken = 0;
-      if (!alone || rank == 0)
+      int sweeps_taken = refinements;
+      if (!refined && (!alone || rank == 0))
         sweeps_taken = sweeps<double>(cluster, alone, w, rows, v, vrows, k, tol, norms_raw,
                                       reinterpret_cast<double *>(dynamic + kDynamicBytes - swap64), partial_raw, flags, rank_of);
 
@@ -926,21 +1414,28 @@ namespace ttg
             }
             if (threadIdx.x < top - low + 1) stau[threadIdx.x] = __ldcg(qtau + top - threadIdx.x);
             __syncthreads();
-            for (int64_t c = q0 + warp; c < q1; c += warps)
+            // eight lanes a column, four columns a warp (as in the factorisation)
+            for (int64_t c0 = q0 + warp * 4; c0 < q1; c0 += warps * 4)
             {
-              double *bc = bcols + (c - q0) * len;
+              const int64_t c = c0 + (lane >> 3);
+              const bool live = c < q1;
+              const int lanes = lane & 7;
+              double *bc = bcols + ((live ? c : c0) - q0) * len;
               for (int64_t t = top; t >= low; --t)
               {
                 const double tau = stau[top - t];
                 if (tau == 0.0) continue;
                 const double *vt = stage + (top - t) * len;
                 double dot = 0.0;
-                for (int64_t i = t + 1 + lane; i < len; i += 32) dot = fma(vt[i], bc[i], dot);
-                dot = warp_sum(dot);
-                const double wt = tau * (bc[t] + dot);
-                for (int64_t i = t + 1 + lane; i < len; i += 32) bc[i] = fma(-wt, vt[i], bc[i]);
+                for (int64_t i = t + 1 + lanes; i < len; i += 8) dot = fma(vt[i], bc[i], dot);
+                dot = group_sum<double, 8>(dot);
+                const double head = bc[t], wt = tau * (head + dot);
                 __syncwarp();
-                if (lane == 0) bc[t] -= wt;
+                if (live)
+                {
+                  for (int64_t i = t + 1 + lanes; i < len; i += 8) bc[i] = fma(-wt, vt[i], bc[i]);
+                  if (lanes == 0) bc[t] = head - wt;
+                }
                 __syncwarp();
               }
             }
@@ -1003,7 +1498,7 @@ namespace ttg
       int32_t rows, cols, k, kept, first_ld, column, row, absorb;
     };
 
-    // one CTA per kept block: first[:, column:column+kept] = U[:, :kept] (times s or sqrt(s)),
+    // eight CTAs per kept block: first[:, column:column+kept] = U[:, :kept] (times s or sqrt(s)),
     // second[row:row+kept, :] = Vh[:kept, :] (times s or sqrt(s)), values[...] = s[:kept]
     __global__ void keep_kernel(const KeepEntry *__restrict__ table, const double *__restrict__ u,
                                 const double *__restrict__ s, const double *__restrict__ vh,
@@ -1011,23 +1506,24 @@ namespace ttg
     {
       const KeepEntry e = table[blockIdx.x];
       const double *sv = s + e.s_off;
-      for (int64_t i = threadIdx.x; i < static_cast<int64_t>(e.rows) * e.kept; i += blockDim.x)
+      const int32_t at = static_cast<int32_t>(blockIdx.y * blockDim.x + threadIdx.x), step = static_cast<int32_t>(gridDim.y * blockDim.x);
+      for (int32_t i = at; i < e.rows * e.kept; i += step)
       {
-        const int64_t r = i / e.kept, j = i % e.kept;
-        double x = u[e.u_off + r * e.k + j];
+        const int32_t r = i / e.kept, j = i - r * e.kept;
+        double x = u[e.u_off + static_cast<int64_t>(r) * e.k + j];
         if (e.absorb == 1) x *= sv[j];
         else if (e.absorb == 3) x *= sqrt(sv[j]);
-        first[e.first_off + r * e.first_ld + e.column + j] = x;
+        first[e.first_off + static_cast<int64_t>(r) * e.first_ld + e.column + j] = x;
       }
-      for (int64_t i = threadIdx.x; i < static_cast<int64_t>(e.kept) * e.cols; i += blockDim.x)
+      for (int32_t i = at; i < e.kept * e.cols; i += step)
       {
-        const int64_t j = i / e.cols, c = i % e.cols;
-        double x = vh[e.vh_off + j * e.cols + c];
+        const int32_t j = i / e.cols, c = i - j * e.cols;
+        double x = vh[e.vh_off + static_cast<int64_t>(j) * e.cols + c];
         if (e.absorb == 2) x *= sv[j];
         else if (e.absorb == 3) x *= sqrt(sv[j]);
         second[e.second_off + (e.row + j) * static_cast<int64_t>(e.cols) + c] = x;
       }
-      for (int64_t j = threadIdx.x; j < e.kept; j += blockDim.x) values[e.values_off + j] = sv[j];
+      for (int32_t j = at; j < e.kept; j += step) values[e.values_off + j] = sv[j];
     }
   } // namespace
 
@@ -1066,10 +1562,10 @@ namespace ttg
       }
     });
     if (configured != cudaSuccess) return configured;
-    // the cluster the largest block wants (16 CTAs from 128 columns, 8 from 32, below that the
-    // sweeps run on one CTA), or the largest the GPU can hold; blocks come largest first, so a
-    // second wave of clusters only holds small blocks
-    const int want = largest >= 128 ? 16 : largest >= 32 ? 8 : 1;
+    // the cluster the largest block wants (16 CTAs from 128 columns, 8 from 16, one CTA below that), or
+    // the largest the GPU can hold; blocks come largest first, so a second wave of clusters only
+    // holds small blocks
+    const int want = largest >= 128 ? 16 : largest >= 16 ? 8 : 1;
     int size = 1;
     for (int c = want; c > 1; c /= 2)
       if (cluster_for[c] >= 1)
@@ -1103,7 +1599,7 @@ namespace ttg
                        double *first, double *second, double *values, cudaStream_t stream)
   {
     if (count <= 0) return cudaSuccess;
-    keep_kernel<<<count, 256, 0, stream>>>(static_cast<const KeepEntry *>(table), u, s, vh, first, second, values);
+    keep_kernel<<<dim3(static_cast<unsigned>(count), 8), 256, 0, stream>>>(static_cast<const KeepEntry *>(table), u, s, vh, first, second, values);
     return cudaGetLastError();
   }
 
@@ -1119,7 +1615,7 @@ namespace ttg
   {
     // Every singular value of a split (block after block, each block's in descending order) sorted
     // by (value descending, position ascending) — the order of the host's stable sort — by a bitonic
-    // sort in shared memory; then one thread walks the sorted values: the cut (values above `tol`,
+    // sort in shared memory; then, the threads sharing the sorted values: the cut (values above `tol`,
     // at most `max_bond`), the values each block keeps, and the +-q pairing of the bond (a domain
     // sector keeps at most as many as its dual, the first ones in the sorted order; a sector whose
     // dual keeps nothing drops out), as tentorch/linalg/graded/svd.cpp:68-118 ranks them on the host.
@@ -1135,7 +1631,8 @@ namespace ttg
       int32_t *block_of = pos + n;                                                  // [n_values]
       int32_t *kept = block_of + n_values;                                          // [n_blocks]
       int32_t *mult = kept + n_blocks;                                              // [n_sectors] x 3
-      int32_t *paired = mult + n_sectors, *used = paired + n_sectors;
+      int32_t *paired = mult + n_sectors;
+      __shared__ int32_t cut, any, differs;
       // keys: the complement of |value|'s bits (ascending keys = descending values); padding last
       for (int i = threadIdx.x; i < n; i += blockDim.x)
       {
@@ -1150,14 +1647,18 @@ namespace ttg
           pos[i] = 0x7fffffff;
         }
       }
-      if (threadIdx.x == 0)
+      for (int32_t b = threadIdx.x; b < n_blocks; b += blockDim.x)
       {
         int32_t at = 0;
-        for (int32_t b = 0; b < n_blocks; ++b)
-        {
-          for (int32_t j = 0; j < block_k[b]; ++j) block_of[at + j] = b;
-          at += block_k[b];
-        }
+        for (int32_t i = 0; i < b; ++i) at += block_k[i];
+        for (int32_t j = 0; j < block_k[b]; ++j) block_of[at + j] = b;
+        kept[b] = 0;
+      }
+      for (int32_t s = threadIdx.x; s < n_sectors; s += blockDim.x) mult[s] = 0;
+      if (threadIdx.x == 0)
+      {
+        cut = n_values;
+        any = differs = 0;
       }
       __syncthreads();
       for (int size = 2; size <= n; size <<= 1)
@@ -1183,40 +1684,50 @@ namespace ttg
           }
           __syncthreads();
         }
-      if (threadIdx.x != 0) return;
-      int32_t cut = 0;
-      while (cut < n_values && values[pos[cut]] > tol) ++cut;
-      if (max_bond >= 0 && cut > max_bond) cut = static_cast<int32_t>(max_bond);
-      for (int32_t b = 0; b < n_blocks; ++b) kept[b] = 0;
-      for (int32_t s = 0; s < n_sectors; ++s) mult[s] = used[s] = 0;
-      for (int32_t r = 0; r < cut; ++r) ++kept[block_of[pos[r]]];
-      for (int32_t b = 0; b < n_blocks; ++b) mult[block_sector[b]] += kept[b];
-      bool any = false, differs = false;
-      for (int32_t s = 0; s < n_sectors; ++s)
+      // the cut: the first of the sorted values that is not above tol
+      for (int32_t r = threadIdx.x; r < n_values; r += blockDim.x)
+        if (!(values[pos[r]] > tol)) atomicMin(&cut, r);
+      __syncthreads();
+      const int32_t last = max_bond >= 0 && cut > max_bond ? static_cast<int32_t>(max_bond) : cut;
+      for (int32_t r = threadIdx.x; r < last; r += blockDim.x) atomicAdd(kept + block_of[pos[r]], 1);
+      __syncthreads();
+      for (int32_t b = threadIdx.x; b < n_blocks; b += blockDim.x) atomicAdd(mult + block_sector[b], kept[b]);
+      __syncthreads();
+      for (int32_t s = threadIdx.x; s < n_sectors; s += blockDim.x)
       {
         paired[s] = -1;
         if (mult[s] == 0) continue;
         if (mult[dual[s]] > 0)
         {
           paired[s] = min(mult[s], mult[dual[s]]);
-          any = true;
-          if (paired[s] != mult[s]) differs = true;
+          any = 1;
+          if (paired[s] != mult[s]) differs = 1;
         }
         else
-          differs = true;
+          differs = 1;
       }
+      __syncthreads();
       if (any && differs)
       {
-        for (int32_t b = 0; b < n_blocks; ++b) kept[b] = 0;
-        for (int32_t r = 0; r < cut; ++r)
+        for (int32_t b = threadIdx.x; b < n_blocks; b += blockDim.x) kept[b] = 0;
+        __syncthreads();
+        // a warp per sector walks the sorted values 32 at a time and keeps the sector's first ones
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+        for (int32_t s = warp; s < n_sectors; s += warps)
         {
-          const int32_t b = block_of[pos[r]], s = block_sector[b];
-          if (paired[s] < 0 || used[s] >= paired[s]) continue;
-          ++used[s];
-          ++kept[b];
+          int32_t used = 0;
+          for (int32_t r0 = 0; r0 < last && used < paired[s]; r0 += 32)
+          {
+            const int32_t r = r0 + lane, b = r < last ? block_of[pos[r]] : -1;
+            const bool in = b >= 0 && block_sector[b] == s;
+            const unsigned mask = __ballot_sync(0xffffffffu, in);
+            if (in && used + __popc(mask & ((1u << lane) - 1u)) < paired[s]) atomicAdd(kept + b, 1);
+            used += __popc(mask);
+          }
         }
+        __syncthreads();
       }
-      for (int32_t b = 0; b < n_blocks; ++b) kept_out[b] = kept[b];
+      for (int32_t b = threadIdx.x; b < n_blocks; b += blockDim.x) kept_out[b] = kept[b];
     }
   } // namespace
 

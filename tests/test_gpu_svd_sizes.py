@@ -1,0 +1,60 @@
+'''The engine's batched SVD where its phases change: one column, the smallest preconditioned blocks, the
+padding of the column blocks (8), the cluster's thresholds (16, 128 columns), the longest columns of the
+blocked FP32 sweeps (320), tall and wide; spectra over twelve decades, without structure, and rank
+deficient, several blocks in one launch.
+
+Bounds, with n the longer side and eps = 2^-52: Jacobi's method and the products around it are backward
+stable with errors of a few eps sqrt(n) a column; 8 n eps, relative to the largest singular value, for
+the values and the product of the factors, and for the orthonormality of the vectors of nonzero values.'''
+import numpy as np
+import pytest
+import torch
+
+import tentorch_gb300 as tg
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -52
+
+
+def _graded(rng, m, n):
+    k = min(m, n)
+    u, v = (np.linalg.qr(rng.standard_normal((x, k)))[0] for x in (m, n))
+    return (u * 10.0 ** (-12 * np.arange(k) / k)) @ v.T
+
+
+def _deficient(rng, m, n):
+    r = max(1, min(m, n) // 3)
+    return rng.standard_normal((m, r)) @ rng.standard_normal((r, n))
+
+
+SPECTRA = {'graded': _graded, 'unstructured': lambda rng, m, n: rng.standard_normal((m, n)), 'deficient': _deficient}
+
+
+@pytest.mark.parametrize('spectrum', SPECTRA)
+@pytest.mark.parametrize('sizes', [[(1, 1), (1, 5), (2, 2), (9, 2)], [(15, 15), (16, 40), (7, 7)], [(17, 16), (31, 33), (8, 9)],
+                                   [(127, 70), (97, 96)], [(128, 128), (33, 200), (16, 16)], [(321, 40), (161, 161)], [(330, 325)]])
+def test_factors_within_their_bounds(sizes, spectrum):
+    rng = np.random.default_rng(len(sizes) * 1000 + sizes[0][0])
+    blocks = [SPECTRA[spectrum](rng, m, n) for m, n in sizes]
+    cat = tg.su2  # its sectors are their own duals: the split keeps each block's values
+    legs = [tg.Leg(cat, [(i,) for i in range(len(sizes))], [s[side] for s in sizes]) for side in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = torch.float64, device = 'cuda')
+    for i, b in enumerate(blocks):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    first, values, second = tg.svd(t, None, 1e-13)
+    bond = first.domain[0]
+    at = 0
+    kept = dict(zip(bond.sectors, bond.multiplicities))
+    for i, b in enumerate(blocks):
+        n = max(b.shape)
+        count = kept.get((i,), 0)
+        u, v = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+        s = values[at:at + count].cpu().numpy()
+        at += count
+        want = np.linalg.svd(b, compute_uv = False)
+        scale, tol = want[0], 8 * n * EPS
+        assert np.abs(s - want[:count]).max() <= tol * scale
+        assert want[count:].max(initial = 0.0) <= 1e-13 + tol * scale
+        for q in (u.T @ u, v @ v.T):
+            assert np.abs(q - np.eye(count)).max() <= tol
+        assert np.abs((u * s) @ v - b).max() <= tol * scale + 1e-13 * n
