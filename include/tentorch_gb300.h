@@ -226,17 +226,28 @@ int32_t tt_lanczos_async(const tt_plan *plan, int32_t dtype, int32_t precision, 
 
 /* ---- truncating splittings (tentorch/linalg/graded/svd.cpp:41-177) -------------------------- */
 
-/* Thin SVDs of `count` float64 blocks in one launch (one-sided Jacobi, mixed precision: FP32 sweeps,
- * then FP64 re-orthonormalisation and FP64 sweeps to full accuracy; blocks of 32 columns or more
- * sorted by column norm and QR-factored first, the sweeps then working on R^T; a thread-block
- * cluster per block; replaces the per-block at::linalg_svd of svd.cpp:57-62).  `table` is a DEVICE array of 7
+/* Thin QR factorisations of `count` blocks in one launch (Householder reflections with LAPACK's signs, a
+ * thread-block cluster per block; replaces the per-block at::linalg_qr of svd.cpp:203-257).
+ * tt_qr_plan: from the blocks' lengths and columns (host pairs) the offset in elements of each block's
+ * part of the workspace, the elements in all and the cluster size for the launch (0: some block does
+ * not fit a cluster's shared memory, factor it elsewhere).  tt_qr_blocks: `table` is a DEVICE array of 8
+ * int64 per block: the offsets in elements of the matrix (in `a`), Q, R and the workspace part, then
+ * len, columns and the element strides matrix row, matrix column, Q row, Q column, R row, R column as
+ * eight int32.  With k = min(len, columns), Q (len x k) and R (k x columns, zeros below its diagonal)
+ * go to their places in `q` and `r`.  Asynchronous on `stream`. */
+int32_t tt_qr_plan(int32_t dtype, int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int32_t *ranks);
+int32_t tt_qr_blocks(int32_t dtype, int32_t count, int32_t ranks, const int64_t *table, const void *a, void *q, void *r,
+                     void *workspace, void *stream);
+/* Thin SVDs of `count` float64 blocks in one launch (one-sided Jacobi, mixed precision: the columns
+ * sorted by norm and QR-factored, FP32 sweeps on R^T, then FP64 refinement by matrix products, or FP64
+ * sweeps where that does not settle; a thread-block cluster per block; replaces the per-block at::linalg_svd of svd.cpp:57-62).  `table` is a DEVICE array of 7
  * int64 per block: a_off, rows, cols, u_off, s_off, vh_off, ws_off (offsets in doubles), best
  * ordered largest block first; `largest` is the largest min(rows, cols) among them (it sets the
  * cluster size).  Block i is rows x cols row-major at a + a_off; with k = min(rows, cols) <= 1024
  * it writes U (rows x k, row-major) at u + u_off, the k singular values in descending order at
  * s + s_off and Vh (k x cols, row-major) at vh + vh_off.  ws_off places the block's working set in
- * `workspace` (from tt_svd_workspace).  info[i] (device int32) receives the FP64 sweeps block i
- * took, -1 when they did not converge (then its factors are not to be used).  Asynchronous on
+ * `workspace` (from tt_svd_workspace).  info[i] (device int32) receives the FP64 refinements or sweeps block
+ * i took, -1 when they did not converge (then its factors are not to be used).  Asynchronous on
  * `stream`. */
 int32_t tt_svd_blocks(int32_t count, int64_t largest, const int64_t *table, const double *a, double *u, double *s,
                       double *vh, double *workspace, int32_t *info, void *stream);

@@ -885,6 +885,35 @@ extern "C"
     return TT_OK;
   }
 
+  int32_t tt_qr_plan(int32_t dtype, int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int32_t *ranks)
+  {
+    if (count < 0) return fail(TT_EINVAL, "a negative block count");
+    if (dtype != TT_DTYPE_FLOAT64 && dtype != TT_DTYPE_COMPLEX128) return fail(TT_EINVAL, "unknown dtype");
+    return guarded([&] {
+      *total = 0;
+      for (int32_t i = 0; i < count; ++i)
+      {
+        if (shapes[2 * i] < 1 || shapes[2 * i + 1] < 1 || shapes[2 * i] > INT32_MAX || shapes[2 * i + 1] > INT32_MAX)
+          throw ttg::InvalidArgument("a block of the batched QR needs rows and columns");
+        offsets[i] = *total;
+        *total += ttg::qr_workspace(shapes[2 * i], shapes[2 * i + 1]);
+      }
+      *ranks = ttg::qr_cluster(count, shapes, dtype == TT_DTYPE_COMPLEX128);
+    });
+  }
+
+  int32_t tt_qr_blocks(int32_t dtype, int32_t count, int32_t ranks, const int64_t *table, const void *a, void *q, void *r,
+                       void *workspace, void *stream)
+  {
+    if (count < 0) return fail(TT_EINVAL, "a negative block count");
+    if (dtype != TT_DTYPE_FLOAT64 && dtype != TT_DTYPE_COMPLEX128) return fail(TT_EINVAL, "unknown dtype");
+    if (ranks < 1 || ranks > 16 || (ranks & (ranks - 1))) return fail(TT_EINVAL, "the batched QR takes the cluster size tt_qr_plan gave");
+    const cudaError_t e =
+      ttg::qr_blocks(count, ranks, table, a, q, r, workspace, dtype == TT_DTYPE_COMPLEX128, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(TT_ECUDA, std::string("CUDA: ") + cudaGetErrorString(e));
+    return TT_OK;
+  }
+
   int32_t tt_dots(int32_t dtype, int32_t count, const void *const *as, const void *b, int64_t n, double *scratch,
                   double *out, void *stream)
   {

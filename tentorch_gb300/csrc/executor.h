@@ -220,6 +220,14 @@ namespace ttg
   cudaError_t svd_keep(int32_t count, const void *table, const double *u, const double *s, const double *vh,
                        double *first, double *second, double *values, cudaStream_t stream);
 
+  // Thin QR of float64 or complex128 blocks in one launch (qr.cu): the cluster size for blocks of these
+  // lengths and columns (0: some block does not fit the shared memory of the largest cluster), the
+  // workspace elements of one block, and the launch (`table` a device array of 64 bytes per block).
+  int32_t qr_cluster(int32_t count, const int64_t *shapes, bool complex);
+  int64_t qr_workspace(int64_t len, int64_t columns);
+  cudaError_t qr_blocks(int32_t count, int32_t ranks, const void *table, const void *a, void *q, void *r, void *workspace, bool complex,
+                        cudaStream_t stream);
+
   // The Lanczos loop of a window (lanczos.cu): `base` carries the plan's operands (the vector
   // operand's pointer is replaced by each basis vector), prepared arenas and workspace; scratch holds
   // lanczos_scratch_doubles() doubles; the normalised Ritz vector goes to `result`, the lowest Ritz

@@ -133,6 +133,7 @@ def clear_plans() -> None:
     _pools.clear()
     _batch_pools.clear()
     _superseded.clear()
+    _qr_plans.clear()
     check(lib.tt_plan_cache_clear())
 
 
@@ -807,9 +808,78 @@ def _split_blocks(tensor: Tensor, pieces):
     return first, second
 
 
+# (space, rows or columns first, dtype, device) -> the batched QR of a tensor of that space: its two
+# output spaces, the device table, workspace elements and cluster size; None where a block does not fit
+_qr_plans = {}
+
+
+def _qr_plan(arranged: Tensor, transposed: bool):
+    space, device = arranged._space, arranged.device
+    key = (space.id, transposed, arranged.dtype, device.index)
+    if key in _qr_plans:
+        return _qr_plans[key]
+    cat = space.cat
+    present = [(i, k) for i, k in enumerate(space.keys) if space.shapes[i][0] * space.shapes[i][1] > 0]
+    multiplicities, offsets = {}, []
+    for i, k in present:
+        offsets.append(multiplicities.get(k.domain, 0))
+        multiplicities[k.domain] = offsets[-1] + min(space.shapes[i])
+    bond = Leg.from_blocks(cat, sorted((multiplicities or {cat.trivial(): 1}).items()))[0]
+    first = Space.of(cat, space.codomain, [bond], space.qtotal)
+    second = Space.of(cat, [bond], space.domain, cat.trivial())
+    # the matrix factored is the block, or its transpose
+    shapes, count = ints64(x for i, _ in present for x in (reversed(space.shapes[i]) if transposed else space.shapes[i]))
+    places, total, ranks = (i64 * max(len(present), 1))(), i64(), i32()
+    check(lib.tt_qr_plan(_DTYPE[arranged.dtype], len(present), shapes, places, ctypes.byref(total), ctypes.byref(ranks)))
+    plan = None
+    if ranks.value and max([s for i, _ in present for s in space.shapes[i]] + list(multiplicities.values()), default = 0) < 2 ** 31:
+        table = []
+        for at, ((i, k), offset) in enumerate(zip(present, offsets)):
+            rows, cols = space.shapes[i]
+            fi, si = first.index[BlockKey(k.codomain, k.domain, k.copy)], second.index[BlockKey(k.domain, k.domain, 0)]
+            ld = first.shapes[fi][1]
+            head, tail = first.offsets[fi] + offset, second.offsets[si] + offset * cols
+            if transposed:  # Q^T goes to the second factor, R^T to the first
+                entry, strides = (space.offsets[i], tail, head), (cols, rows, 1, cols, 1, cols, 1, ld)
+            else:
+                entry, strides = (space.offsets[i], head, tail), (rows, cols, cols, 1, ld, 1, cols, 1)
+            table += [*entry, places[at], *(strides[s] | strides[s + 1] << 32 for s in range(0, 8, 2))]
+        plan = (len(present), first, second, _uploaded(table, torch.int64, device), total.value, ranks.value)
+    if len(_qr_plans) >= _PLAN_BUDGET and not _captured:
+        _qr_plans.clear()
+    _qr_plans[key] = plan
+    return plan
+
+
+def _qr_blocks(arranged: Tensor, transposed: bool):
+    '''Every block factored in one launch straight into the two output arenas, or None when the tensor is not on
+    a CUDA device or a block does not fit (then the blocks are factored one by one).'''
+    if arranged.device.type != 'cuda' or _precision == PER_BLOCK:
+        return None
+    plan = _qr_plan(arranged, transposed)
+    if plan is None:
+        return None
+    count, first, second, table, total, ranks = plan
+    data = arranged._data
+    stream = torch.cuda.current_stream(data.device).cuda_stream
+    if torch.cuda.is_current_stream_capturing():
+        _note_capture()
+    # zeros: what no block covers (and the pads after odd blocks) is part of the factors
+    out = [torch.zeros(s.size, dtype = data.dtype, device = data.device) for s in (first, second)]
+    if count:
+        ws = torch.empty(total, dtype = data.dtype, device = data.device)
+        q, r = (out[1], out[0]) if transposed else (out[0], out[1])
+        check(lib.tt_qr_blocks(_DTYPE[data.dtype], count, ranks, table.data_ptr(), data.data_ptr(), q.data_ptr(), r.data_ptr(),
+                               ws.data_ptr(), stream))
+    return Tensor._wrap(first, out[0]), Tensor._wrap(second, out[1])
+
+
 def qr(tensor: Tensor, left = None):
     '''tentorch/linalg/graded/svd.cpp:233-244'''
     arranged = tensor.place(left) if left is not None else tensor
+    factors = _qr_blocks(arranged, False)
+    if factors is not None:
+        return factors
     pieces = []
     for i, key in enumerate(arranged.keys()):
         matrix = arranged._view(i)
@@ -823,6 +893,9 @@ def qr(tensor: Tensor, left = None):
 def rq(tensor: Tensor, left = None):
     '''tentorch/linalg/graded/svd.cpp:246-257'''
     arranged = tensor.place(left) if left is not None else tensor
+    factors = _qr_blocks(arranged, True)
+    if factors is not None:
+        return factors
     pieces = []
     for i, key in enumerate(arranged.keys()):
         matrix = arranged._view(i)

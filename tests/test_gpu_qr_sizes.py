@@ -1,0 +1,47 @@
+'''The batched QR and RQ where its kernel changes: one row or column, tall and wide blocks, the cluster's
+thresholds (16 and 96 columns), odd sizes (blocks followed by a pad), several blocks in one launch, and
+columns that are already zero below the diagonal, in float64 and complex128, scaled far from one.
+
+Against LAPACK (numpy) with its signs: Householder QR is columnwise backward stable, so Q R reproduces the
+block, Q^H Q the identity, to 8 max(m, n) eps, and R lies within 8 max(m, n) eps times the condition of the
+leading columns (below 100 n for these random blocks) of LAPACK's.'''
+import numpy as np
+import pytest
+import torch
+
+import tentorch_gb300 as tg
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -52
+
+
+@pytest.mark.parametrize('scale', [0, -600, 500])
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('side', ['qr', 'rq'])
+@pytest.mark.parametrize('sizes', [[(1, 1), (1, 7), (7, 1), (2, 2)], [(15, 15), (9, 20), (20, 9)], [(16, 16), (17, 40), (33, 17)],
+                                   [(95, 96), (130, 97), (60, 200)]])
+def test_factors_match_lapack(sizes, side, dtype, scale):
+    rng = np.random.default_rng(len(sizes) * 1000 + sizes[0][0])
+    blocks = []
+    for m, n in sizes:
+        b = rng.standard_normal((m, n)) + (1j * rng.standard_normal((m, n)) if dtype.is_complex else 0)
+        if m > 3 and n > 3:
+            b[1:, 0] = 0  # nothing to reflect
+        blocks.append(b * 2.0 ** scale)
+    cat = tg.su2
+    legs = [tg.Leg(cat, [(i,) for i in range(len(sizes))], [s[at] for s in sizes]) for at in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = dtype, device = 'cuda')
+    for i, b in enumerate(blocks):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    first, second = getattr(tg, side)(t)
+    for i, b in enumerate(blocks):
+        one, two = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+        q, r, want = (one, two, b) if side == 'qr' else (two.T, one.T, b.T)
+        wq, wr = np.linalg.qr(want)
+        n = max(b.shape)
+        tol = 8 * n * EPS
+        norm = np.abs(want / 2.0 ** scale).sum(0).max()
+        assert np.abs(q.conj().T @ q - np.eye(q.shape[1])).max() <= tol
+        assert np.abs((q @ (r / 2.0 ** scale)) - want / 2.0 ** scale).max() <= tol * norm
+        assert np.abs((r - wr) / 2.0 ** scale).max() <= tol * 100 * n * norm
+        assert np.abs(np.tril(r, -1)).max(initial = 0) == 0
