@@ -1169,7 +1169,8 @@ namespace ttg
           const double st = fma(-0.5 * h, lr + lc, gamma);
           float cf, sf;
           double tangent = 0.0;
-          if (angle(lr, lc, st, cf, sf))
+          // (a pair at round-off is left: with equal values its angle is noise)
+          if (square > 0.25 * limit && angle(lr, lc, st, cf, sf))
           {
             const float tf = sf / cf;
             if (fabsf(tf) > 0.1f) status |= 4;
