@@ -84,7 +84,7 @@ namespace ttg
       GemmReduce *reduces = nullptr;
       int32_t n_ctas = 0, longest = 0, n = 0;
     };
-    std::vector<GemmTables> gemm;
+    std::vector<GemmTables> gemm, gemm_complex;
     std::vector<SplitTables> split;
     std::vector<TcTables> tc;
     // the program's product chain (chain.cu): the relabelling table of its move (built on its first

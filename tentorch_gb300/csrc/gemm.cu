@@ -46,7 +46,7 @@ namespace ttg
     int64_t up256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
   } // namespace
 
-  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full)
+  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full, bool lanes)
   {
     GemmSchedule s;
     // The workers of one SM share its FP64 pipe, so what has to balance is the work per SM: items
@@ -55,8 +55,11 @@ namespace ttg
     // Cost of an item: the 16 x 8 DMMA fragments it computes (fragments wholly outside the block are
     // skipped) times its K range, plus per staged K step (its copies and barriers) and per item
     // (claim, write or partial tile) a quarter of a full tile over 16 of K.
-    const auto cost = [bm, bn](double rows, double cols, double k)
+    // On FMA lanes (complex128): its live entries' multiply-adds, and per staged step of 16 and per item
+    // the time of 1024 (a quarter of a 16 x 16 tile over 16).
+    const auto cost = [bm, bn, lanes](double rows, double cols, double k)
     {
+      if (lanes) return std::ceil(rows * cols / 32.0) * 32.0 * k + 1024.0 * (std::ceil(k / 16.0) + 1.0);
       const double frag = std::ceil(rows / 16.0) * 16.0 * std::ceil(cols / 8.0) * 8.0;
       return frag * k + 0.25 * bm * bn * 16.0 * (std::ceil(k / kDmmaStepK) + 1.0);
     };
@@ -317,10 +320,10 @@ namespace ttg
       return up256(2 * s.slice_a) + up256(2 * s.slice_b) + up256(2 * s.exps) + split_partial_bytes(s, tc) +
              up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
     }
-    // bytes of FP64 scratch: partial tiles (two doubles an entry for complex), tickets
-    int64_t f64_bytes(const GemmSchedule &s)
+    // bytes of FP64 scratch: partial tiles (`entry` bytes an entry), tickets
+    int64_t f64_bytes(const GemmSchedule &s, int tile, int entry)
     {
-      return up256(s.slots * kF64TileM * kF64TileN * 16) + up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
+      return up256(s.slots * tile * tile * entry) + up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
     }
   } // namespace
 
@@ -360,7 +363,9 @@ namespace ttg
       plans->f64[i] = schedule_gemm(p, op, kF64TileM, kF64TileN, false);
       // the split schedule itself is built on the first split launch (most plans never run one);
       // here only its scratch
-      need = std::max(need, (f64_bytes(plans->f64[i]) + 7) / 8);
+      need = std::max(need, (f64_bytes(plans->f64[i], kF64TileM, 8) + 7) / 8);
+      // complex arenas count elements of 16 bytes
+      need = std::max(need, (f64_bytes(schedule_gemm(p, op, kLanesTile, kLanesTile, false, true), kLanesTile, 16) + 15) / 16);
       // a chain's one launch holds the partial tiles of both its products at once
       if (static_cast<int32_t>(i) == p.chain_second)
       {
@@ -478,25 +483,41 @@ namespace ttg
     // FP64 / complex128
     // ---------------------------------------------------------------------------------------
 
-    // Persistent: kF64Workers workers of 128 threads, each computing 32 x 32 tiles over a K range
-    // with 2 x 4 entries per thread, K staged 16 at a time through its own shared memory (A padded
-    // to 33 columns so the k-fast, coalesced stores hit distinct banks).  FP64 retires about 0.44
-    // DFMA per clock per SM sub-partition on this part: the workers keep all four busy.
-    template <typename T>
+    // Persistent: kF64Workers workers of 128 threads, each computing 16 x 16 tiles over a K range on FP64
+    // FMA lanes.  A complex multiply-add is four FP64 ones and a warp's FP64 instruction takes 64 clocks
+    // on a quarter of an SM, so what counts is that no lane works on padding and none waits for copies:
+    //   - a tile's live entries times R phases of K (R a power of two, as many as fill the worker's 1024
+    //     slots, at most the 16 K of a step) are dealt to the threads, eight independent chains each at most,
+    //     and the phases of an entry summed at the end (a 10 x 10 block as 32 x 32 padded entries spent ten
+    //     times its multiply-adds); 32 x 32 tiles over 32 of K would hold an SM for 32 us and do not balance
+    //     (the Fibonacci recoupling of 16 multiplets, all full tiles, takes 3.97 ms with them and 3.85 with
+    //     16 x 16);
+    //   - K advances through two shared stages, the next one's cp.async in flight during a step.
+    // The three products of an environment update at bond 203 (13 charges) take 19, 42 and 26 us; with
+    // padded 32 x 32 tiles and one synchronous stage 70, 94 and 66.
+    constexpr int kLanesK = 16, kLanesPer = 8, kLanesPitch = kLanesTile + 1;
+    constexpr int kLanesSlots = kLanesPer * kWorkerThreads;
+    constexpr int kLanesBytes = kF64Workers * (2 * 2 * kLanesK * kLanesPitch + kLanesSlots) * 16;
+
+    __device__ __forceinline__ void copy16(double2 *dst, const double2 *src, bool in)
+    {
+      const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+    }
+
     __global__ void __launch_bounds__(kF64Workers * kWorkerThreads, 1)
-      gemm_f64_kernel(const T *__restrict__ A, const T *__restrict__ B, T *__restrict__ C,
-                      const DevBlock *__restrict__ blocks, const DevPair *__restrict__ pairs,
-                      const GemmItem *__restrict__ items, const int32_t *__restrict__ cta_begin, const GemmReduce *__restrict__ reduces,
-                      int64_t n_reduces, T *__restrict__ partial, int *__restrict__ tickets)
+      gemm_c128_kernel(const double2 *__restrict__ A, const double2 *__restrict__ B, double2 *__restrict__ C,
+                       const DevBlock *__restrict__ blocks, const DevPair *__restrict__ pairs,
+                       const GemmItem *__restrict__ items, const int32_t *__restrict__ cta_begin, const GemmReduce *__restrict__ reduces,
+                       int64_t n_reduces, double2 *__restrict__ partial, int *__restrict__ tickets)
     {
       dependent_entry();
-      constexpr int BM = kF64TileM, BN = kF64TileN, BK = 16, TM = 2, TN = 4;
+      constexpr int BM = kLanesTile, BN = kLanesTile, BK = kLanesK, P = kLanesPitch;
       extern __shared__ __align__(16) unsigned char smem_raw[];
       const int worker = threadIdx.x / kWorkerThreads, lt = threadIdx.x % kWorkerThreads;
-      T(*as)[BM + 1] = reinterpret_cast<T(*)[BM + 1]>(smem_raw + worker * 2 * BK * (BM + 1) * sizeof(T));
-      T(*bs)[BN + 1] = reinterpret_cast<T(*)[BN + 1]>(smem_raw + (worker * 2 + 1) * BK * (BM + 1) * sizeof(T));
+      double2 *stage_base = reinterpret_cast<double2 *>(smem_raw) + static_cast<int64_t>(worker) * (2 * 2 * BK * P + kLanesSlots);
+      double2 *slots = stage_base + 2 * 2 * BK * P;
       __shared__ int flags[kF64Workers];
-      const int tx = lt % (BN / TN), ty = lt / (BN / TN);
       // this CTA's list of items (dealt by the host, largest first, to balance the SMs); its
       // workers take them in order through a shared counter
       __shared__ int next[kF64Workers];
@@ -509,11 +530,39 @@ namespace ttg
       {
         const GemmItem it = items[idx];
         const DevBlock blk = blocks[it.block];
-        T acc[TM][TN];
+        const int rows = min(BM, blk.m - it.m0), cols = min(BN, blk.n - it.n0), live = rows * cols;
+        int shift = 0;
+        while ((1 << shift) < BK && (live << (shift + 1)) <= kLanesSlots) ++shift;
+        const int phases = 1 << shift, count = live << shift;
+        const int mine = count > lt ? (count - lt + kWorkerThreads - 1) / kWorkerThreads : 0;
+        // slot v: entry v >> shift, phase v & (phases - 1)
+        int pa[kLanesPer], pb[kLanesPer];
+        double2 acc[kLanesPer];
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = zero_t<T>();
+        for (int i = 0; i < kLanesPer; ++i)
+        {
+          const int v = min(lt + i * kWorkerThreads, count - 1), e = v >> shift, row = e / cols, k = v & (phases - 1);
+          pa[i] = k * P + row;
+          pb[i] = BK * P + k * P + (e - row * cols);
+          acc[i] = make_double2(0.0, 0.0);
+        }
+        const auto load = [&](int stage, const double2 *a, const double2 *b, int K, int k0, int hi)
+        {
+          double2 *as = stage_base + stage * 2 * BK * P, *bs = as + BK * P;
+          for (int i = lt; i < rows * BK; i += kWorkerThreads)
+          {
+            const int row = i / BK, kk = i % BK;
+            const bool in = k0 + kk < hi;
+            copy16(as + kk * P + row, in ? a + static_cast<int64_t>(it.m0 + row) * K + k0 + kk : a, in);
+          }
+          for (int i = lt; i < BK * cols; i += kWorkerThreads)
+          {
+            const int kk = i / cols, c = i - kk * cols;
+            const bool in = k0 + kk < hi;
+            copy16(bs + kk * P + c, in ? b + static_cast<int64_t>(k0 + kk) * blk.n + it.n0 + c : b, in);
+          }
+          copy_commit();
+        };
         int32_t kbase = 0;
         for (int32_t pi = 0; pi < blk.pair_count; ++pi)
         {
@@ -522,68 +571,63 @@ namespace ttg
           const int lo = max(it.k0 - kbase, 0), hi = min(it.k1 - kbase, K);
           kbase += K;
           if (lo >= hi) continue;
-          const T *a = A + pr.a;
-          const T *b = B + pr.b;
-          for (int k0 = lo; k0 < hi; k0 += BK)
+          load(0, A + pr.a, B + pr.b, K, lo, hi);
+          int stage = 0;
+          for (int k0 = lo; k0 < hi; k0 += BK, stage ^= 1)
           {
-            for (int i = lt; i < BM * BK; i += kWorkerThreads)
-            {
-              const int r = i / BK, kk = i % BK;
-              const int gm = it.m0 + r, gk = k0 + kk;
-              as[kk][r] = (gm < blk.m && gk < hi) ? a[static_cast<int64_t>(gm) * K + gk] : zero_t<T>();
-            }
-            for (int i = lt; i < BK * BN; i += kWorkerThreads)
-            {
-              const int kk = i / BN, cc = i % BN;
-              const int gk = k0 + kk, gn = it.n0 + cc;
-              bs[kk][cc] = (gk < hi && gn < blk.n) ? b[static_cast<int64_t>(gk) * blk.n + gn] : zero_t<T>();
-            }
+            if (k0 + BK < hi)
+              load(stage ^ 1, A + pr.a, B + pr.b, K, k0 + BK, hi);
+            else
+              copy_commit();  // an empty group keeps the count of the wait below
+            copy_wait_one();
             worker_sync(worker);
+            const double2 *base = stage_base + stage * 2 * BK * P;
+            const int steps = min(BK, hi - k0);  // entries of the stage past `hi` are zeros
+            for (int kk = 0; kk < steps; kk += phases)
 #pragma unroll
-            for (int kk = 0; kk < BK; ++kk)
-            {
-              T av[TM], bv[TN];
-#pragma unroll
-              for (int i = 0; i < TM; ++i) av[i] = as[kk][ty * TM + i];
-#pragma unroll
-              for (int j = 0; j < TN; ++j) bv[j] = bs[kk][tx * TN + j];
-#pragma unroll
-              for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fma_t(av[i], bv[j], acc[i][j]);
-            }
+              for (int i = 0; i < kLanesPer; ++i)
+                if (i < mine) acc[i] = cfma(base[kk * P + pa[i]], base[kk * P + pb[i]], acc[i]);
             worker_sync(worker);
           }
+        }
+        // the phases of each entry, summed in order
+        if (shift != 0)
+        {
+#pragma unroll
+          for (int i = 0; i < kLanesPer; ++i)
+            if (i < mine) slots[lt + i * kWorkerThreads] = acc[i];
+          worker_sync(worker);
+#pragma unroll
+          for (int i = 0; i < kLanesPer; ++i)
+          {
+            const int e = lt + i * kWorkerThreads;
+            double2 sum = make_double2(0.0, 0.0);
+            if (e < live)
+              for (int f = 0; f < phases; ++f) sum = add_t(sum, slots[(e << shift) + f]);
+            acc[i] = sum;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kLanesPer; ++i)
+        {
+          const int e = lt + i * kWorkerThreads;
+          if (e >= live) continue;
+          const int row = e / cols, c = e - row * cols;
+          if (it.slot >= 0) partial[static_cast<int64_t>(it.slot) * BM * BN + row * BN + c] = acc[i];
+          else C[blk.c + static_cast<int64_t>(it.m0 + row) * blk.n + it.n0 + c] = acc[i];
         }
         if (it.slot >= 0)
         {
-          T *out = partial + static_cast<int64_t>(it.slot) * BM * BN;
-#pragma unroll
-          for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) out[(ty * TM + i) * BN + tx * TN + j] = acc[i][j];
-          finish_partial<T, BM, BN>(worker, lt, flags + worker, tickets, reduces, it.reduce, blocks, partial, C);
+          finish_partial<double2, BM, BN>(worker, lt, flags + worker, tickets, reduces, it.reduce, blocks, partial, C);
           continue;
-        }
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-        {
-          const int gm = it.m0 + ty * TM + i;
-          if (gm >= blk.m) continue;
-#pragma unroll
-          for (int j = 0; j < TN; ++j)
-          {
-            const int gn = it.n0 + tx * TN + j;
-            if (gn < blk.n) C[blk.c + static_cast<int64_t>(gm) * blk.n + gn] = acc[i][j];
-          }
         }
         // the alignment pad after an odd-sized block reads as zero in arena-wide sums
         const int64_t entries = static_cast<int64_t>(blk.m) * blk.n;
-        if (lt == 0 && it.m0 + BM >= blk.m && it.n0 + BN >= blk.n && (entries & 1)) C[blk.c + entries] = zero_t<T>();
+        if (lt == 0 && it.m0 + BM >= blk.m && it.n0 + BN >= blk.n && (entries & 1)) C[blk.c + entries] = make_double2(0.0, 0.0);
       }
     }
 
-    // The float64 form of gemm_f64_kernel on the FP64 matrix instruction (mma m16n8k8 f64): each of
+    // The float64 products on the FP64 matrix instruction (mma m16n8k8 f64): each of
     // a worker's 4 warps owns a 16 x 16 quarter of the 32 x 32 tile as two m16n8 accumulators; per
     // 8 of K staged in shared memory a warp issues 2 DMMA.
     __global__ void __launch_bounds__(kF64Workers * kWorkerThreads, 1)
@@ -1051,12 +1095,14 @@ namespace ttg
   namespace
   {
     // The FP64 tables of a GEMM op, built on its first FP64 launch.
-    cudaError_t ensure_f64(const Program &p, DeviceTables &t, size_t op_index)
+    cudaError_t ensure_f64(const Program &p, DeviceTables &t, size_t op_index, bool complex)
     {
       std::lock_guard<std::mutex> lock(t.mutex);
-      DeviceTables::GemmTables &dst = t.gemm[op_index];
+      DeviceTables::GemmTables &dst = (complex ? t.gemm_complex : t.gemm)[op_index];
       if (dst.ready) return cudaSuccess;
-      const GemmSchedule s = schedule_gemm(p, p.ops[op_index], kF64TileM, kF64TileN, true);
+      const int tile = complex ? kLanesTile : kF64TileM;
+      const GemmSchedule s = schedule_gemm(p, p.ops[op_index], tile, tile, true, complex);
+
       dst.n_items = static_cast<int64_t>(s.items.size());
       dst.n_reduces = static_cast<int64_t>(s.reduces.size());
       dst.slots = s.slots;
@@ -1078,8 +1124,8 @@ namespace ttg
   cudaError_t launch_gemm_f64(const Program &p, DeviceTables &t, size_t op_index, const void *A, const void *B, void *C,
                               bool complex, void *scratch, int *ticket_region, cudaStream_t stream)
   {
-    if (const cudaError_t built = ensure_f64(p, t, op_index); built != cudaSuccess) return built;
-    const auto &sched = t.gemm[op_index];
+    if (const cudaError_t built = ensure_f64(p, t, op_index, complex); built != cudaSuccess) return built;
+    const auto &sched = (complex ? t.gemm_complex : t.gemm)[op_index];
     if (sched.n_items == 0) return cudaSuccess;
     const auto *blocks = reinterpret_cast<const DevBlock *>(t.blocks);
     const auto *pairs = reinterpret_cast<const DevPair *>(t.pairs);
@@ -1091,7 +1137,7 @@ namespace ttg
     cudaError_t e = cudaSuccess;
     if (sched.n_reduces > kTicketInts)
     {
-      tickets = reinterpret_cast<int *>(base + up256(sched.slots * kF64TileM * kF64TileN * 16));
+      tickets = reinterpret_cast<int *>(base + up256(sched.slots * (complex ? kLanesTile * kLanesTile * 16 : kF64TileM * kF64TileN * 8)));
       if ((e = cudaMemsetAsync(tickets, 0, static_cast<size_t>(sched.n_reduces) * 4, stream)) != cudaSuccess) return e;
     }
     // one CTA per list the schedule dealt, as many workers as its longest list needs (at most four)
@@ -1099,10 +1145,10 @@ namespace ttg
     const int workers = static_cast<int>(std::clamp<int64_t>(sched.longest, 1, kF64Workers));
     if (complex)
     {
-      const int bytes = std::max<int>(kF64Workers * 2 * 16 * (kF64TileM + 1) * 16, kPinBytes);
+      const int bytes = std::max<int>(kLanesBytes, kPinBytes);
       static std::once_flag once;
-      if ((e = configure(gemm_f64_kernel<double2>, bytes, once)) != cudaSuccess) return e;
-      e = launch_dependent(gemm_f64_kernel<double2>, grid, workers * kWorkerThreads, bytes, stream,
+      if ((e = configure(gemm_c128_kernel, bytes, once)) != cudaSuccess) return e;
+      e = launch_dependent(gemm_c128_kernel, grid, workers * kWorkerThreads, bytes, stream,
                            static_cast<const double2 *>(A), static_cast<const double2 *>(B), static_cast<double2 *>(C), blocks,
                            pairs, static_cast<const GemmItem *>(sched.items), static_cast<const int32_t *>(sched.cta_begin),
                            static_cast<const GemmReduce *>(sched.reduces), sched.n_reduces, static_cast<double2 *>(partial),
@@ -1278,6 +1324,7 @@ namespace ttg
   void stage_gemm(const Program &p, DeviceTables &t, TableStaging &staging)
   {
     t.gemm.assign(p.ops.size(), {});
+    t.gemm_complex.assign(p.ops.size(), {});
     t.split.assign(p.ops.size(), {});
     t.tc.assign(p.ops.size(), {});
     if (!p.gemm_plans) return;

@@ -91,6 +91,7 @@ namespace ttg
 
   // Tile sizes of the two kernels.
   constexpr int kF64TileM = 32, kF64TileN = 32;
+  constexpr int kLanesTile = 16;  // rows and columns of a complex128 tile
   constexpr int kDmmaStepK = 32;  // K staged per step (two stages in flight) in the DMMA kernel
   constexpr int kSplitTileM = 32, kSplitTileN = 32, kSplitStepK = 32;
   // Persistent launches: one CTA per SM (held there by its shared memory), several workers of 128
@@ -144,7 +145,8 @@ namespace ttg
 
   // The FP64 schedule of a GEMM op; with full = false only its sizes (items, partial slots,
   // reductions), for sizing the scratch: the items are dealt on the op's first FP64 launch.
-  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full = true);
+  // `lanes`: costed for the FMA-lane kernel (complex128) rather than DMMA fragments.
+  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full = true, bool lanes = false);
   // The partial tiles (32 x 32 doubles each) the one launch of a program's product chain may hold
   // (chain.cu; 0 without a chain).
   int64_t chain_partial_slots(const Program &p);

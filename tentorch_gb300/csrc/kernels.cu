@@ -199,8 +199,9 @@ namespace ttg
     if (base) cudaFree(base);
     if (chain.base) cudaFree(chain.base);
     if (chain.relabel_base) cudaFree(chain.relabel_base);
-    for (GemmTables &g : gemm)
-      if (g.base) cudaFree(g.base);
+    for (std::vector<GemmTables> *tables : {&gemm, &gemm_complex})
+      for (GemmTables &g : *tables)
+        if (g.base) cudaFree(g.base);
     for (SplitTables &g : split)
       if (g.base) cudaFree(g.base);
   }
