@@ -1507,6 +1507,13 @@ namespace ttg
     {
       const KeepEntry e = table[blockIdx.x];
       const double *sv = s + e.s_off;
+      // the pads after blocks of odd size (the bond's sector has first_ld multiplets)
+      if (blockIdx.y == 0 && threadIdx.x == 0)
+      {
+        const int64_t one = static_cast<int64_t>(e.rows) * e.first_ld, two = static_cast<int64_t>(e.first_ld) * e.cols;
+        if (e.column == 0 && (one & 1)) first[e.first_off + one] = 0.0;
+        if (e.row == 0 && (two & 1)) second[e.second_off + two] = 0.0;
+      }
       const int32_t at = static_cast<int32_t>(blockIdx.y * blockDim.x + threadIdx.x), step = static_cast<int32_t>(gridDim.y * blockDim.x);
       for (int32_t i = at; i < e.rows * e.kept; i += step)
       {

@@ -99,7 +99,7 @@ def lanczos_einsum(spec: str, tensors, vector: int, start: Tensor, n_iter: int =
     if wait and norm(start) == 0.0:
         raise ValueError('Lanczos needs a starting vector of non-zero norm.')
     from tentorch_gb300 import linalg
-    from tentorch_gb300._lib import check, f64, i32, i64, lib, pointers
+    from tentorch_gb300._lib import check, f64, i32, i64, lib
     operands = list(tensors)
     operands[vector] = start
     linalg._check_device(operands)
@@ -108,8 +108,8 @@ def lanczos_einsum(spec: str, tensors, vector: int, start: Tensor, n_iter: int =
         raise ValueError('the action has to map the vector to a tensor with the same legs')
     data = start._data
     device = data.device
-    stream = torch.cuda.current_stream(device).cuda_stream
-    capturing = torch.cuda.is_current_stream_capturing()
+    stream = linalg._raw_stream(data.get_device())
+    capturing = linalg._capturing()
     if capturing:
         linalg._note_capture()
     ws = linalg._workspace(plan, device, data.dtype, stream)
@@ -123,8 +123,8 @@ def lanczos_einsum(spec: str, tensors, vector: int, start: Tensor, n_iter: int =
     check(lib.tt_lanczos_scratch(start._space.size, n_iter, linalg._DTYPE[data.dtype], ctypes.byref(doubles)))
     scratch = torch.empty(doubles.value, dtype = torch.float64, device = device)
     result = torch.empty_like(data)
-    args = (plan.handle, linalg._DTYPE[data.dtype], linalg.get_precision(), pointers(t._data.data_ptr() for t in operands),
-            pointers((p.data_ptr() if p is not None else None) for p in prepared), vector, data.data_ptr(), n_iter, tol,
+    args = (plan.handle, linalg._DTYPE[data.dtype], linalg.get_precision(), linalg._addresses([t._data.data_ptr() for t in operands]),
+            linalg._addresses([p.data_ptr() if p is not None else None for p in prepared]), vector, data.data_ptr(), n_iter, tol,
             ws.data_ptr() if ws is not None else None, scratch.data_ptr(), result.data_ptr())
     if not wait:
         found = torch.empty(2, dtype = torch.float64, device = device)  # the energy, then the size (int32)

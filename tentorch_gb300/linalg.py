@@ -57,12 +57,33 @@ def precision(slices: int):
         set_precision(old)
 
 
+def _raw_stream(index: int) -> int:
+    '''The current stream of a CUDA device as a raw handle (without building a torch.cuda.Stream).'''
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+def _capturing() -> bool:
+    return torch._C._cuda_isCurrentStreamCapturing()
+
+
+# ctypes array types by length
+_vector_types = {}
+
+
+def _addresses(values):
+    '''A ctypes array of the addresses (None: null).'''
+    kind = _vector_types.get(len(values))
+    if kind is None:
+        kind = _vector_types[len(values)] = vp * len(values)
+    return kind(*values)
+
+
 class Plan:
     '''A compiled program: its output space, workspace and the size of each operand's prepared
     arena.  The engine owns the program; a wholesale clear of the plan caches frees it, and a Plan
     held across that clear compiles its program again on its next use (same key, same result).'''
     __slots__ = ('_handle', 'generation', 'key', 'build', 'cat', 'out_space', 'workspace', 'flops', 'moved', 'n_ops',
-                 'prepared', 'sizes', '__weakref__')
+                 'sizes', '__weakref__')
 
     def __init__(self, handle, cat, key = None, build = None):
         self._handle, self.cat, self.key, self.build = handle, cat, key, build
@@ -72,7 +93,6 @@ class Plan:
                                ctypes.byref(ops)))
         self.out_space = Space._load(cat, space.value)
         self.workspace, self.flops, self.moved, self.n_ops = ws.value, flops.value, moved.value, ops.value
-        self.prepared = []
         self.sizes = {}
 
     @property
@@ -134,6 +154,8 @@ def clear_plans() -> None:
     _batch_pools.clear()
     _superseded.clear()
     _qr_plans.clear()
+    _split_layouts.clear()
+    _split_writes.clear()
     check(lib.tt_plan_cache_clear())
 
 
@@ -206,7 +228,8 @@ def _prepared_arena(plan: Plan, operand: int, tensor: Tensor, ws, stream, force:
     data = tensor._data
     key = (plan.handle.value, operand, data.data_ptr())
     held = _prepared.get(key)
-    seen = held is not None and held[0]() is data and held[1] == data._version
+    mine = held is not None and held[0]() is data
+    seen = mine and held[1] == data._version
     if seen and held[2] is not None:
         return held[2]
     arena = None
@@ -214,7 +237,7 @@ def _prepared_arena(plan: Plan, operand: int, tensor: Tensor, ws, stream, force:
         arena = torch.empty(size, dtype = data.dtype, device = data.device)
         check(lib.tt_plan_prepare(plan.handle, _DTYPE[data.dtype], operand, data.data_ptr(), arena.data_ptr(),
                                   ws.data_ptr() if ws is not None else None, stream))
-    if held is None or held[0]() is not data:
+    if not mine:
         def forget(ref, key = key):
             entry = _prepared.get(key)
             if entry is not None and entry[0] is ref:
@@ -240,22 +263,36 @@ def _prepare_now(plan: Plan, operand: int, tensor: Tensor, ws, stream) -> Option
 
 def run(plan: Plan, tensors, out: Optional[Tensor] = None, reuse_prepared: bool = True) -> Tensor:
     """Execute a plan on the operands' device and return the output tensor."""
-    _check_device(tensors)
     data0 = tensors[0]._data
+    dtype, index = data0.dtype, data0.get_device()
+    for t in tensors:
+        if t._data.dtype != dtype or t._data.get_device() != index:
+            _check_device(tensors)
+    if index < 0:
+        _check_device(tensors)
     device = data0.device
     if out is None:
-        out = Tensor._wrap(plan.out_space, torch.empty(plan.out_space.size, dtype = data0.dtype, device = device))
-    stream = torch.cuda.current_stream(device).cuda_stream
+        out = Tensor._wrap(plan.out_space, torch.empty(plan.out_space.size, dtype = dtype, device = device))
+    stream = _raw_stream(index)
     # a captured CUDA graph reads every operand from its own buffer at each replay, never a prepared copy
-    if torch.cuda.is_current_stream_capturing():
+    if _capturing():
         _note_capture()
         reuse_prepared = False
-    ws = _workspace(plan, device, data0.dtype, stream)
-    prepared = [(_prepared_arena(plan, i, t, ws, stream) if reuse_prepared else None) for i, t in enumerate(tensors)]
-    inputs = pointers(t._data.data_ptr() for t in tensors)
-    prep = pointers((p.data_ptr() if p is not None else None) for p in prepared)
-    check(lib.tt_plan_execute(plan.handle, _DTYPE[data0.dtype], _precision, inputs, prep, out._data.data_ptr(),
-                              ws.data_ptr() if ws is not None else None, stream))
+    handle = plan.handle
+    ws = _workspace(plan, device, dtype, stream)
+    ws_at = ws.data_ptr() if ws is not None else None
+    if reuse_prepared:
+        prep = []
+        for i, t in enumerate(tensors):
+            arena = _prepared_arena(plan, i, t, ws, stream)
+            prep.append(arena.data_ptr() if arena is not None else None)
+        prep = _addresses(prep)
+    else:
+        prep = None
+    status = lib.tt_plan_execute(handle, _DTYPE[dtype], _precision, _addresses([t._data.data_ptr() for t in tensors]), prep,
+                                 out._data.data_ptr(), ws_at, stream)
+    if status:
+        check(status)
     return out
 
 
@@ -275,6 +312,10 @@ def place(tensor: Tensor, above, below = None) -> Tensor:
 
 def place_plan(space: Space, above, below) -> Plan:
     '''The compiled plan of `place` on a tensor of this space (legs already resolved).'''
+    key = ('place', space.id, tuple(above), tuple(below))
+    plan = _plans.get(key)
+    if plan is not None:
+        return plan
     above, below = [int(x) for x in above], [int(x) for x in below]
     a, na = ints32(above)
     b, nb = ints32(below)
@@ -303,9 +344,12 @@ def contract(left: Tensor, right: Tensor, left_legs, right_legs, charge = None) 
 
 def contract_plan(left: Space, right: Space, left_legs, right_legs, charge = None) -> Plan:
     '''The compiled plan of `contract` on tensors of these spaces.'''
-    left_legs, right_legs = [int(x) for x in left_legs], [int(x) for x in right_legs]
     has = charge is not None
     q = _label(charge) if has else 0
+    plan = _plans.get(('contract', left.id, right.id, tuple(left_legs), tuple(right_legs), has, q))
+    if plan is not None:
+        return plan
+    left_legs, right_legs = [int(x) for x in left_legs], [int(x) for x in right_legs]
     la, n = ints32(left_legs)
     ra, m = ints32(right_legs)
     if n != m:
@@ -323,11 +367,11 @@ def einsum(spec: str, *tensors: Tensor, **options) -> Tensor:
     outcharge = options.get('outcharge')
     if not tensors:
         raise ValueError('an einsum needs at least one operand')
-    cat = tensors[0].cat
+    cat = tensors[0]._space.cat
     for t in tensors:
-        if t.cat is not cat:
+        if t._space.cat is not cat:
             raise ValueError('an einsum needs every operand over one category')
-    return run(einsum_plan(spec, [t._space for t in tensors], outcharge), list(tensors))
+    return run(einsum_plan(spec, [t._space for t in tensors], outcharge), tensors)
 
 
 # per (device, stream, dtype, window): the workspace of one window of a batch (a batch's windows run
@@ -353,9 +397,9 @@ def einsum_batch(spec: str, operand_lists, outcharge = None) -> list:
         return []
     first = operand_lists[0][0]
     device, dtype = first._data.device, first._data.dtype
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = _raw_stream(first._data.get_device())
     # a captured CUDA graph reads every operand from its own buffer at each replay
-    capturing = torch.cuda.is_current_stream_capturing()
+    capturing = _capturing()
     if capturing:
         _note_capture()
     handles, outs, keep, inputs, prepared, workspaces = [], [], [], [], [], []
@@ -469,8 +513,12 @@ def einsum_plan(spec: str, spaces, outcharge = None) -> Plan:
     (from spaces a caller expects) fills the cache the call reads.'''
     has = outcharge is not None
     q = _label(outcharge) if has else 0
+    key = ('einsum', spec, tuple([s.id for s in spaces]), has, q)
+    plan = _plans.get(key)
+    if plan is not None:
+        return plan
     ids, n = ints32(s.id for s in spaces)
-    return _plan(('einsum', spec, tuple(s.id for s in spaces), has, q),
+    return _plan(key,
                  lambda out: lib.tt_plan_einsum(spec.encode(), n, ids, int(has), q, out), spaces[0].cat)
 
 
@@ -540,53 +588,160 @@ def _factor_blocks_per_block(arranged: Tensor, present, while_waiting = None):
     if while_waiting is not None:
         while_waiting()
     host = torch.cat([f[2] for f in factors]).to('cpu', torch.float64).tolist() if factors else []
-    return factors, host, None
+    return factors, host
 
 
-def _factor_blocks(arranged: Tensor, while_waiting = None):
-    """The thin SVD of every non-empty block.  float64 blocks on the GPU go through one launch of
-    the engine's Jacobi SVD (tt_svd_blocks), complex blocks, blocks beyond its size and the
-    per-block comparison form through at::linalg_svd one block at a time, as svd.cpp:57-62 does.
-    Returns [key, u, s, vh, kept, offset] per block (u, s, vh views of packed device arrays in the
-    first case) and the host copy of all singular values, block after block."""
-    space = arranged._space
-    present = [(i, key) for i, key in enumerate(arranged.keys()) if space.shapes[i][0] * space.shapes[i][1] > 0]
-    batched = (arranged.dtype == torch.float64 and arranged.device.type == 'cuda' and _precision != PER_BLOCK and
-               all(min(space.shapes[i]) <= 1024 for i, _ in present))
-    if not batched:
-        return _factor_blocks_per_block(arranged, present, while_waiting)
-    dims, count = ints64(x for i, _ in present for x in space.shapes[i])
-    places, total = (i64 * max(len(present), 1))(), i64()
-    check(lib.tt_svd_workspace(len(present), dims, places, ctypes.byref(total)))
-    ws_at = total.value
-    entries, shapes = [], []
-    u_at = s_at = vh_at = 0
-    for at, (i, key) in enumerate(present):
-        rows, cols = space.shapes[i]
-        k = min(rows, cols)
-        entries.append([space.offsets[i], rows, cols, u_at, s_at, vh_at, places[at]])
-        shapes.append((key, rows, cols, k, u_at, s_at, vh_at))
-        u_at, s_at, vh_at = u_at + rows * k, s_at + k, vh_at + k * cols
-    # the largest blocks first: the launch's clusters then finish together, small blocks last
-    entries.sort(key = lambda e: -min(e[1], e[2]) ** 2 * max(e[1], e[2]))
-    table = [x for e in entries for x in e]
-    largest = max((min(e[1], e[2]) for e in entries), default = 0)
-    device = arranged.device
-    # no wait for the stream's queued work (the window's Lanczos): the SVD is queued behind it
-    dev_table = _uploaded(table, torch.int64, device)
-    u = torch.empty(max(u_at, 1), dtype = torch.float64, device = device)
-    sv = torch.empty(max(s_at, 1), dtype = torch.float64, device = device)
-    vh = torch.empty(max(vh_at, 1), dtype = torch.float64, device = device)
-    ws = torch.empty(max(ws_at, 1), dtype = torch.float64, device = device)
-    info = torch.empty(max(len(present), 1), dtype = torch.int32, device = device)
-    stream = torch.cuda.current_stream(device).cuda_stream
-    check(lib.tt_svd_blocks(len(present), largest, dev_table.data_ptr(), arranged._data.data_ptr(), u.data_ptr(),
-                            sv.data_ptr(), vh.data_ptr(), ws.data_ptr(), info.data_ptr(), stream))
-    # the values stay on the device: the caller ranks them there and reads the sweep counts
-    # (info) with the per-block results in one wait
-    factors = [[key, (u_off, rows, k), (s_off, k), (vh_off, k, cols), 0, 0]
-               for key, rows, cols, k, u_off, s_off, vh_off in shapes]
-    return factors, None, (u, sv, vh, info[:max(len(present), 1)], s_at, present)
+class _SplitLayout:
+    '''What the batched SVD of the tensors of one space needs on a device, laid out once: the device table of its blocks
+    and of the ranking, the places of the packed factors and the workspace in one buffer.'''
+    __slots__ = ('present', 'count', 'largest', 'blocks', 'table', 'ranking', 'n_blocks', 'n_sectors', 'sv_at', 'vh_at', 'ws_at',
+                 'values', 'size')
+
+    def __init__(self, space: Space, device):
+        cat = space.cat
+        self.present = [(i, key) for i, key in enumerate(space.keys) if space.shapes[i][0] * space.shapes[i][1] > 0]
+        dims, _ = ints64(x for i, _ in self.present for x in space.shapes[i])
+        places, total = (i64 * max(len(self.present), 1))(), i64()
+        check(lib.tt_svd_workspace(len(self.present), dims, places, ctypes.byref(total)))
+        entries, self.blocks, ids = [], [], {}
+        u_at = s_at = vh_at = 0
+        for at, (i, key) in enumerate(self.present):
+            rows, cols = space.shapes[i]
+            k = min(rows, cols)
+            entries.append([space.offsets[i], rows, cols, u_at, s_at, vh_at, places[at]])
+            self.blocks.append((key, rows, cols, k, u_at, s_at, vh_at))
+            u_at, s_at, vh_at = u_at + rows * k, s_at + k, vh_at + k * cols
+            for sector in (key.domain, cat.dual(key.domain)):
+                ids.setdefault(sector, len(ids))
+        # the largest blocks first: the launch's clusters then finish together, small blocks last
+        entries.sort(key = lambda e: -min(e[1], e[2]) ** 2 * max(e[1], e[2]))
+        self.count = self.n_blocks = len(self.present)
+        self.largest = max((b[3] for b in self.blocks), default = 0)
+        self.n_sectors = len(ids)
+        self.values = s_at
+        # one buffer: U, the values, Vh, then the workspace, each from a multiple of 32 doubles
+        up = lambda n: (n + 31) // 32 * 32
+        self.sv_at = up(u_at)
+        self.vh_at = self.sv_at + up(s_at)
+        self.ws_at = self.vh_at + up(vh_at)
+        self.size = max(self.ws_at + total.value, 1)
+        # no wait for the stream's queued work (the window's Lanczos): the SVD is queued behind it
+        self.table = _uploaded([x for e in entries for x in e], torch.int64, device)
+        self.ranking = _uploaded([b[3] for b in self.blocks] + [ids[b[0].domain] for b in self.blocks] +
+                                 [ids[cat.dual(sector)] for sector in sorted(ids, key = ids.get)], torch.int32, device)
+
+
+class _SplitWrite:
+    '''Where the kept factors of one space's split go: the two output spaces, the bond's multiplets and the device table of
+    the kept blocks; `covered` when every entry of the outputs is written.'''
+    __slots__ = ('first', 'second', 'multiplets', 'table', 'count', 'covered')
+
+    def __init__(self, space: Space, layout: _SplitLayout, kept, absorb: int, device):
+        cat = space.cat
+        multiplicities, offsets = {}, []
+        for (key, *_), n in zip(layout.blocks, kept):
+            offsets.append(multiplicities.get(key.domain, 0))
+            if n:
+                multiplicities[key.domain] = offsets[-1] + n
+        placed, at = {}, 0
+        for sector in sorted(multiplicities):
+            placed[sector] = at
+            at += multiplicities[sector]
+        bond = Leg.from_blocks(cat, sorted((multiplicities or {cat.trivial(): 1}).items()))[0]
+        self.first = Space.of(cat, space.codomain, [bond], space.qtotal)
+        self.second = Space.of(cat, [bond], space.domain, cat.trivial())
+        self.multiplets = bond.multiplets()
+        table, written = [], [0, 0]
+        self.count = 0
+        for (key, rows, cols, k, u_at, s_at, vh_at), n, offset in zip(layout.blocks, kept, offsets):
+            if n == 0:
+                continue
+            fi = self.first.index[BlockKey(key.codomain, key.domain, key.copy)]
+            si = self.second.index[BlockKey(key.domain, key.domain, 0)]
+            table += [u_at, s_at, vh_at, self.first.offsets[fi], self.second.offsets[si], placed[key.domain] + offset,
+                      rows | cols << 32, k | n << 32, self.first.shapes[fi][1] | offset << 32, offset | absorb << 32]
+            written[0] += rows * n
+            written[1] += n * cols
+            self.count += 1
+        self.covered = (self.count > 0 and written[0] == sum(m * n for m, n in self.first.shapes) and
+                        written[1] == sum(m * n for m, n in self.second.shapes))
+        self.table = _uploaded(table, torch.int64, device)
+
+
+# (space, device) -> its split's layout (None: not for the batched SVD); (space, kept counts, absorb, device)
+# -> where its factors go
+_split_layouts = {}
+_split_writes = {}
+
+
+def _remembered(cache: dict, key, make):
+    found = cache.get(key, cache)
+    if found is cache:
+        found = make()
+        if len(cache) >= _PLAN_BUDGET:
+            cache.clear()
+        cache[key] = found
+    return found
+
+
+def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None):
+    """The split of float64 blocks on the GPU: one launch of the engine's Jacobi SVD for all blocks (tt_svd_blocks),
+    the ranking of the values on the device (tt_svd_rank), one read of each block's kept count with the
+    SVD's sweep counts, and one launch that writes the kept factors (tt_svd_keep).  None when the blocks are
+    not for it, False when one did not settle (then they go through at::linalg_svd one at a time)."""
+    global svd_fallbacks
+    space, data = arranged._space, arranged._data
+    if not (data.dtype == torch.float64 and data.is_cuda and _precision != PER_BLOCK):
+        return None
+    device, index = data.device, data.get_device()
+    layout = _remembered(_split_layouts, (space.id, index),
+                         lambda: _SplitLayout(space, device) if all(min(s) <= 1024 for s in space.shapes if s[0] * s[1]) else None)
+    if layout is None:
+        return None
+    buffer = torch.empty(layout.size, dtype = torch.float64, device = device)
+    counts = torch.empty(max(layout.count + layout.n_blocks, 1), dtype = torch.int32, device = device)
+    u = buffer.data_ptr()
+    sv, vh, ws = u + 8 * layout.sv_at, u + 8 * layout.vh_at, u + 8 * layout.ws_at
+    info, kept_at = counts.data_ptr(), counts.data_ptr() + 4 * layout.count
+    stream = _raw_stream(index)
+    check(lib.tt_svd_blocks(layout.count, layout.largest, layout.table.data_ptr(), data.data_ptr(), u, sv, vh, ws, info, stream))
+    ranking = layout.ranking.data_ptr()
+    # the host's ranking for splits too large for the kernel
+    status = lib.tt_svd_rank(sv, layout.values, ranking, ranking + 4 * layout.n_blocks, layout.n_blocks, ranking + 8 * layout.n_blocks,
+                             layout.n_sectors, float(tol), -1 if max_bond is None else int(max_bond), kept_at, stream)
+    if status not in (0, 1):
+        check(status)
+    if while_waiting is not None:
+        while_waiting()
+    host = counts.tolist() if layout.count else []
+    if layout.count and min(host[:layout.count]) < 0:
+        svd_fallbacks += 1
+        return False
+    if status == 0:
+        kept = tuple(host[layout.count:])
+    else:
+        kept = _ranked_on_host(arranged, layout, buffer[layout.sv_at:layout.sv_at + layout.values].tolist(), max_bond, tol)
+    write = _remembered(_split_writes, (space.id, kept, absorb, index), lambda: _SplitWrite(space, layout, kept, absorb, device))
+    # (the kernel writes the pads after odd blocks)
+    make = torch.empty if write.covered else torch.zeros
+    first, second, values = (make(n, dtype = torch.float64, device = device)
+                             for n in (write.first.size, write.second.size, write.multiplets))
+    if write.count:
+        check(lib.tt_svd_keep(write.count, write.table.data_ptr(), u, sv, vh, first.data_ptr(), second.data_ptr(), values.data_ptr(),
+                              stream))
+    return Tensor._wrap(write.first, first), values, Tensor._wrap(write.second, second)
+
+
+def _ranked_on_host(arranged: Tensor, layout: _SplitLayout, values, max_bond, tol):
+    '''The device ranking's kept counts, from the values on the host.'''
+    factors = [[b[0], None, None, None, 0, 0] for b in layout.blocks]
+    candidates, at = [], 0
+    for fi, b in enumerate(layout.blocks):
+        for i in range(b[3]):
+            candidates.append((values[at], fi, i))
+            at += 1
+    _rank_candidates(factors, candidates, max_bond, tol, arranged.cat)
+    return tuple(f[4] for f in factors)
 
 
 def _split_over(tensor: Tensor, left, max_bond, tol, absorb, while_waiting = None):
@@ -600,77 +755,20 @@ def _split_over(tensor: Tensor, left, max_bond, tol, absorb, while_waiting = Non
     if max_bond is not None and max_bond < 1:
         raise ValueError(f'a bond needs at least one multiplet, got {max_bond}')
     arranged = tensor.place(left) if left is not None else tensor
-    cat = arranged.cat
-    factors, host, packed = _factor_blocks(arranged, while_waiting)
-    if packed is not None:
-        ranked = _rank_on_device(arranged, factors, packed, max_bond, tol, while_waiting)
-        if ranked is None:
-            # a block the Jacobi sweeps did not settle within their cap: this split's blocks go
-            # through cuSOLVER one by one instead (QR iteration, gesvd), as the per-block form runs them
-            global svd_fallbacks
-            svd_fallbacks += 1
-            factors, host, packed = _factor_blocks_per_block(arranged, packed[5])
-        else:
-            multiplicities = ranked
-            return _split_finish(arranged, factors, packed, multiplicities, absorb)
+    batched = _split_batched(arranged, max_bond, tol, absorb, while_waiting)
+    if batched:
+        return batched
+    if batched is False:
+        while_waiting = None  # it has run
+    present = [(i, key) for i, key in enumerate(arranged.keys()) if arranged._space.shapes[i][0] * arranged._space.shapes[i][1] > 0]
+    factors, host = _factor_blocks_per_block(arranged, present, while_waiting)
     candidates, at = [], 0
     for fi, f in enumerate(factors):
         for index in range(f[2].numel()):
             candidates.append((host[at], fi, index))
             at += 1
-    multiplicities = _rank_candidates(factors, candidates, max_bond, tol, cat)
-    return _split_finish(arranged, factors, packed, multiplicities, absorb)
-
-
-def _rank_on_device(arranged: Tensor, factors, packed, max_bond, tol, while_waiting = None):
-    '''The ranking of the split's singular values on the device (tt_svd_rank): per block the values
-    it keeps, read with the SVD's sweep counts in one wait.  Returns the bond's multiplets per
-    domain sector (the blocks' f[4] set), or None when a block's Jacobi sweeps did not settle.
-    Where the values do not fit the ranking kernel, they are read and ranked on the host.'''
-    u, sv, vh, info, s_at, present = packed
-    cat = arranged.cat
-    ids = {}
-    for f in factors:
-        for sector in (f[0].domain, cat.dual(f[0].domain)):
-            ids.setdefault(sector, len(ids))
-    sectors = sorted(ids, key = ids.get)
-    table = ([f[2][1] for f in factors] + [ids[f[0].domain] for f in factors] +
-             [ids[cat.dual(sector)] for sector in sectors])
-    device = arranged.device
-    dev = _uploaded(table, torch.int32, device)
-    kept = torch.zeros(len(factors), dtype = torch.int32, device = device)
-    nb, ns = len(factors), len(sectors)
-    stream = torch.cuda.current_stream(device).cuda_stream
-    try:
-        check(lib.tt_svd_rank(sv.data_ptr(), s_at, dev.data_ptr(), dev.data_ptr() + 4 * nb, nb, dev.data_ptr() + 8 * nb, ns,
-                              float(tol), -1 if max_bond is None else int(max_bond), kept.data_ptr(), stream))
-    except ValueError:
-        if while_waiting is not None:
-            while_waiting()
-        return _rank_on_host(factors, sv[:s_at].cpu().tolist(), info, max_bond, tol, cat)
-    if while_waiting is not None:
-        while_waiting()
-    both = torch.cat([info.to(torch.int32), kept]).cpu()
-    if present and int(both[:info.numel()].min()) < 0:
-        return None
-    multiplicities = {}
-    for f, k in zip(factors, both[info.numel():].tolist()):
-        f[4] = k
-        if k:
-            multiplicities[f[0].domain] = multiplicities.get(f[0].domain, 0) + k
-    return multiplicities
-
-
-def _rank_on_host(factors, host, info, max_bond, tol, cat):
-    '''The same ranking on the host, for splits too large for the ranking kernel.'''
-    if factors and int(info.min()) < 0:
-        return None
-    candidates, at = [], 0
-    for fi, f in enumerate(factors):
-        for index in range(f[2][1]):
-            candidates.append((host[at], fi, index))
-            at += 1
-    return _rank_candidates(factors, candidates, max_bond, tol, cat)
+    multiplicities = _rank_candidates(factors, candidates, max_bond, tol, arranged.cat)
+    return _split_finish(arranged, factors, multiplicities, absorb)
 
 
 def _rank_candidates(factors, candidates, max_bond, tol, cat):
@@ -708,9 +806,9 @@ def _rank_candidates(factors, candidates, max_bond, tol, cat):
     return multiplicities
 
 
-def _split_finish(arranged: Tensor, factors, packed, multiplicities, absorb):
+def _split_finish(arranged: Tensor, factors, multiplicities, absorb):
     '''The bond of the split from its multiplets per domain sector, and the two factors and the
-    values written (one launch from the packed factors, else block by block).'''
+    values written block by block.'''
     cat = arranged.cat
     nxt = {}
     for f in factors:
@@ -726,27 +824,6 @@ def _split_finish(arranged: Tensor, factors, packed, multiplicities, absorb):
     first = Tensor(cat, arranged.codomain, [bond], arranged.qtotal, arranged.dtype, arranged.device)
     values = torch.zeros(bond.multiplets(), dtype = arranged.dtype, device = arranged.device)
     second = Tensor(cat, [bond], arranged.domain, cat.trivial(), arranged.dtype, arranged.device)
-    if packed is not None:
-        # one launch writes every kept block of both factors and the values
-        u, sv, vh = packed[:3]
-        table, count = [], 0
-        for key, (u_off, rows, k), (s_off, _), (vh_off, _, cols), kept, offset in factors:
-            if kept == 0:
-                continue
-            fi = first._space.index[BlockKey(key.codomain, key.domain, key.copy)]
-            si = second._space.index[BlockKey(key.domain, key.domain, 0)]
-            first_ld = first._space.shapes[fi][1]
-            table += [u_off, s_off, vh_off, first._space.offsets[fi], second._space.offsets[si],
-                      placed[key.domain] + offset, rows | cols << 32, k | kept << 32, first_ld | offset << 32,
-                      offset | absorb << 32]
-            count += 1
-        if count:
-            device = arranged.device
-            dev_table = _uploaded(table, torch.int64, device)
-            stream = torch.cuda.current_stream(device).cuda_stream
-            check(lib.tt_svd_keep(count, dev_table.data_ptr(), u.data_ptr(), sv.data_ptr(), vh.data_ptr(),
-                                  first._data.data_ptr(), second._data.data_ptr(), values.data_ptr(), stream))
-        return first, values, second
     for key, u, s, vh, kept, offset in factors:
         if kept == 0:
             continue
@@ -861,8 +938,8 @@ def _qr_blocks(arranged: Tensor, transposed: bool):
         return None
     count, first, second, table, total, ranks = plan
     data = arranged._data
-    stream = torch.cuda.current_stream(data.device).cuda_stream
-    if torch.cuda.is_current_stream_capturing():
+    stream = _raw_stream(data.get_device())
+    if _capturing():
         _note_capture()
     # zeros: what no block covers (and the pads after odd blocks) is part of the factors
     out = [torch.zeros(s.size, dtype = data.dtype, device = data.device) for s in (first, second)]

@@ -58,3 +58,21 @@ def test_factors_within_their_bounds(sizes, spectrum):
         for q in (u.T @ u, v @ v.T):
             assert np.abs(q - np.eye(count)).max() <= tol
         assert np.abs((u * s) @ v - b).max() <= tol * scale + 1e-13 * n
+
+
+def test_the_pads_after_odd_blocks_are_zero():
+    '''The factors are written into uninitialised memory when they cover their arenas: the alignment pads after
+    blocks of odd size, which arena-wide sums read, have to be written too.'''
+    rng = np.random.default_rng(3)
+    cat = tg.su2
+    sizes = [(3, 5), (7, 7), (5, 9)]
+    legs = [tg.Leg(cat, [(i,) for i in range(3)], [s[side] for s in sizes]) for side in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = torch.float64, device = 'cuda')
+    for i, (m, n) in enumerate(sizes):
+        t.block((i,), (i,)).copy_(torch.from_numpy(rng.standard_normal((m, n))))
+    for n in (64, 128, 256, 512, 1024):  # freed memory of the sizes the factors take, full of NaN
+        filled = [torch.full((n,), float('nan'), dtype = torch.float64, device = 'cuda') for _ in range(8)]
+        del filled
+    for factor in (tg.svd(t, None, 0.0)[0], tg.svd(t, None, 0.0)[2]):
+        blocks = sum(float(b.square().sum()) for b in factor.to_tuple()[3].values())
+        assert abs(float(factor.data.square().sum()) - blocks) <= 1e-12 * blocks
