@@ -13,7 +13,7 @@
 // three shuffled additions.  Q is formed from the unit vectors by the reflectors, the last first, each
 // rank its columns.  A block is scaled by a power of two first, so that no norm under- or overflows.
 //
-// The site of bond 256 (18 blocks, the largest 92 x 46): 236 us for the whole call, 4661 us with one cuSOLVER
+// The site of bond 256 (18 blocks, the largest 92 x 46): 242 us for the whole call, 4661 us with one cuSOLVER
 // factorisation per block.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -98,6 +98,16 @@ namespace ttg
     template <int G>
     __device__ __forceinline__ double2 lanes_sum(double2 v) { return make_double2(lanes_sum<G>(v.x), lanes_sum<G>(v.y)); }
 
+    // sqrt(x) and its reciprocal, each to half an ulp or so: an ulp of rsqrt in the first, largest columns
+    // doubled the error of Q R
+    __device__ __forceinline__ void root(double x, double &norm, double &inv)
+    {
+      inv = rsqrt(x);
+      norm = x * inv;
+      norm = fma(0.5 * inv, fma(-norm, norm, x), norm);
+      inv = fma(inv, fma(-norm, inv, 1.0), inv);
+    }
+
     // dlarfg / zlarfg: H = I - tau v v^H with v_0 = 1 takes (alpha, x) to (beta, 0), beta real; v's rest is
     // x scale, xn = |x|^2.
     __device__ __forceinline__ void make_reflector(double alpha, double xn, double &beta, double &tau, double &scale)
@@ -106,7 +116,8 @@ namespace ttg
       tau = scale = 0.0;
       if (xn > 0.0)
       {
-        const double norm2 = fma(alpha, alpha, xn), inv = rsqrt(norm2), norm = norm2 * inv;
+        double norm, inv;
+        root(fma(alpha, alpha, xn), norm, inv);
         const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
         beta = -copysign(norm, alpha);
         tau = fabs(d) * inv;                             // (beta - alpha) / beta
@@ -119,7 +130,8 @@ namespace ttg
       tau = scale = make_double2(0.0, 0.0);
       if (xn > 0.0 || alpha.y != 0.0)
       {
-        const double norm2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn)), inv = rsqrt(norm2), norm = norm2 * inv;
+        double norm, inv;
+        root(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn)), norm, inv);
         const double re = alpha.x + copysign(norm, alpha.x);  // alpha - beta, without cancellation
         const double side = copysign(inv, alpha.x);           // -1 / beta
         beta = make_double2(-copysign(norm, alpha.x), 0.0);

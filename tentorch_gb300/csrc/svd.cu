@@ -30,7 +30,7 @@
 // One launch, one block of 148 x 148 / 92 x 92 / 31 x 31 with singular values over twelve decades: 2782 / 1378 /
 // 466 us; with FP32 sweeps column by column that skipped the small columns and 3 to 6 FP64 sweeps 7557 /
 // 3783 / 2152 us.  Factors orthonormal to 1e-15 (3e-15 before; clusters of values 1e-9 apart 1e-11, 1e-7
-// before).  At 148 columns now: QR 0.56 ms, FP32 sweeps 1.16 (eight), refinement 0.73, U = Q J 0.27.
+// before).  At 148 columns now: QR 0.56 ms, FP32 sweeps 1.16 (eight), refinement 0.7, U = Q J 0.27.
 //
 // A thread-block cluster of up to 16 CTAs per block, which shares every step: QR by columns, FP32 sweeps
 // by pairs of column blocks in distributed shared memory, the products by tiles, the FP64 sweeps with
@@ -1097,8 +1097,8 @@ namespace ttg
       // idea of T. Ogita and K. Aishima, "Iterative refinement for symmetric eigenvalue decomposition",
       // Japan J. Indust. Appl. Math. 35 (2018), on the one-sided form, whose graded columns keep their
       // relative accuracy).  E has to be good only to FP32, so V E is an FP32 product.  Done when no
-      // cosine is above tol and V is orthonormal to it (or, from the fourth time on, both stand at the
-      // round-off of W = X V, within four times that).  Pairs whose angle is not small (close singular values
+      // cosine is above tol and V is orthonormal to it; once both are within four times that, a last step of
+      // that size leaves V as orthonormal as its rounding, and W = X V is formed again.  Pairs whose angle is not small (close singular values
       // that FP32 left mixed) are left out; when there are some after the first time, or it does not
       // settle, the FP64 sweeps below take over.  Against the 3 to 6 FP64 sweeps of 0.7 ms each that it
       // replaces, a step is about 0.1 ms at 148 columns.
@@ -1107,11 +1107,11 @@ namespace ttg
       float *em = reinterpret_cast<float *>(ws + lay.v_slices);
       void *small_stage = dynamic + kDynamicBytes - kSmallBytes;
       double *v_start = ws + lay.w32_slices;  // V as FP32 left it, for the sweeps should they run (k x k)
-      bool refined = false;
+      bool refined = false, last = false;
       int refinements = 0;
       for (int64_t i = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x; i < k * k; i += static_cast<int64_t>(ranks) * blockDim.x)
         v_start[i] = __ldcg(v_cur + i);
-      for (int it = 0; it < 7 && !refined; ++it)
+      for (int it = 0; it < 8 && !refined; ++it)
       {
         const double *vc = v_cur;
         const int64_t nrow = (xl + kSmallTile - 1) / kSmallTile, ncol = (k + kSmallTile - 1) / kSmallTile;
@@ -1129,6 +1129,11 @@ namespace ttg
             });
         }
         cluster.sync();
+        if (last)
+        {
+          refined = true;
+          break;
+        }
         int64_t turn = 0;
         for (int which = 0; which < 2; ++which)
           for (int64_t tr = 0; tr < ncol; ++tr)
@@ -1149,7 +1154,7 @@ namespace ttg
         cluster.sync();
         for (int64_t j = threadIdx.x; j < k; j += blockDim.x) norms_raw[j] = __ldcg(g + j * k + j);
         __syncthreads();
-        int status = 0;  // 1: a cosine above tol, 2: V off by more, 4: an angle that is not small, 8: either above four times tol
+        int status = 0;  // above four times tol: 1 a cosine, 2 V^T V - I; 8: either above tol; 4: an angle that is not small
         for (int64_t i = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x; i < k * k; i += static_cast<int64_t>(ranks) * blockDim.x)
         {
           const int64_t c = i / k, r = i - c * k;
@@ -1159,22 +1164,23 @@ namespace ttg
           {
             const double off = 1.0 - h;
             em[i] = static_cast<float>(0.5 * off);
-            if (!(fabs(off) <= tol + 1e-15)) status |= fabs(off) <= 4.0 * tol ? 2 : 10;
+            if (!(fabs(off) <= tol)) status |= fabs(off) <= 4.0 * tol ? 8 : 10;
             continue;
           }
           const double gamma = __ldcg(g + i), lr = norms_raw[r], lc = norms_raw[c];
-          if (!(fabs(h) <= tol + 1e-15)) status |= fabs(h) <= 4.0 * tol ? 2 : 10;
           const double limit = tol * tol * lr * lc, square = gamma * gamma;
-          if (!(square <= limit)) status |= square <= 16.0 * limit ? 1 : 9;
+          const bool open = !(square <= 16.0 * limit);
+          if (!(square <= limit)) status |= open ? 9 : 8;
+          if (!(fabs(h) <= tol)) status |= fabs(h) <= 4.0 * tol ? 8 : 10;
           const double st = fma(-0.5 * h, lr + lc, gamma);
           float cf, sf;
           double tangent = 0.0;
-          // (a pair at round-off is left: with equal values its angle is noise)
-          if (square > 0.25 * limit && angle(lr, lc, st, cf, sf))
+          if (angle(lr, lc, st, cf, sf))
           {
             const float tf = sf / cf;
-            if (fabsf(tf) > 0.1f) status |= 4;
-            else tangent = tf;
+            // (at round-off the angle of a pair of equal values is noise)
+            if (open && fabsf(tf) > 0.1f) status |= 4;
+            if (fabsf(tf) <= (open ? 0.1f : 1e-8f)) tangent = tf;
           }
           em[c * k + r] = static_cast<float>(fma(-0.5, h, tangent));
           em[r * k + c] = static_cast<float>(fma(-0.5, h, -tangent));
@@ -1186,12 +1192,10 @@ namespace ttg
         status = 0;
         for (unsigned r = 0; r < ranks; ++r) status |= cluster.map_shared_rank(flags, r)[2];
         refinements = it + 1;
-        if (!(status & 3) || (it >= 3 && !(status & 8)))
-        {
-          refined = true;
-          break;
-        }
-        if ((it >= 1 && (status & 4)) || it == 6) break;
+        refined = !(status & 8);
+        if (refined) break;
+        last = !(status & 3);
+        if (!last && ((it >= 1 && (status & 4)) || it >= 6)) break;
         for (int64_t tile = rank; tile < ncol * ncol; tile += ranks)
         {
           const int64_t tr = tile / ncol, tc = tile % ncol;
