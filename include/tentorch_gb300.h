@@ -276,6 +276,18 @@ int32_t tt_svd_rank(const double *values, int32_t n_values, const int32_t *block
 int32_t tt_svd_keep(int32_t count, const int64_t *table, const double *u, const double *s, const double *vh,
                     double *first, double *second, double *values, void *stream);
 
+/* The same for complex128 blocks of min(rows, cols) <= 160 (elements are complex numbers, the values doubles).
+ * tt_svd_complex_plan: from host pairs of rows and cols the place of each block's workspace and the
+ * elements in all, the table of the blocks' QR factorisations (8 int64 a block, to be copied to the device) and
+ * the cluster size for those (0: some block is not for this path, nothing else is set).
+ * tt_svd_complex_blocks: the 7 int64 a block of tt_svd_blocks and that table, both DEVICE arrays, in one order;
+ * info[i] is -1 where block i did not settle or has a zero singular value.  Asynchronous on `stream`. */
+int32_t tt_svd_complex_plan(int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int64_t *qr_table, int32_t *qr_ranks);
+int32_t tt_svd_complex_blocks(int32_t count, int64_t largest, int32_t qr_ranks, const int64_t *table, const int64_t *qr_table,
+                              const void *a, void *u, double *s, void *vh, void *workspace, int32_t *info, void *stream);
+int32_t tt_svd_complex_keep(int32_t count, const int64_t *table, const void *u, const double *s, const void *vh, void *first,
+                            void *second, void *values, void *stream);
+
 /* ---- Krylov arithmetic on arenas ----------------------------------------------------------- */
 
 /* out[2j], out[2j+1] = <a_j, b> (conjugating a_j) for j < count, on `stream`, with no host

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -881,6 +882,50 @@ extern "C"
       return fail(TT_EINVAL, "too many singular values to rank in one CTA's shared memory (" + std::to_string(n_values) + ")");
     const cudaError_t e = ttg::svd_rank(values, n_values, block_k, block_sector, n_blocks, dual, n_sectors, tol, max_bond,
                                         kept, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(TT_ECUDA, std::string("CUDA: ") + cudaGetErrorString(e));
+    return TT_OK;
+  }
+
+  int32_t tt_svd_complex_plan(int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int64_t *qr_table, int32_t *qr_ranks)
+  {
+    if (count < 0) return fail(TT_EINVAL, "a negative block count");
+    return guarded([&] {
+      *total = 0;
+      *qr_ranks = 0;
+      std::vector<int64_t> tall(2 * static_cast<size_t>(count));
+      for (int32_t i = 0; i < count; ++i)
+      {
+        const int64_t rows = shapes[2 * i], cols = shapes[2 * i + 1];
+        if (rows < 1 || cols < 1) throw ttg::InvalidArgument("a block of the batched SVD needs rows and columns");
+        if (!ttg::complex_svd_takes(rows, cols)) return;
+        tall[2 * i] = std::max(rows, cols);
+        tall[2 * i + 1] = std::min(rows, cols);
+        offsets[i] = *total;
+        ttg::complex_svd_qr_entry(rows, cols, *total, qr_table + 8 * i);
+        *total += ttg::complex_svd_workspace(rows, cols);
+      }
+      *qr_ranks = ttg::qr_cluster(count, tall.data(), true);
+    });
+  }
+
+  int32_t tt_svd_complex_blocks(int32_t count, int64_t largest, int32_t qr_ranks, const int64_t *table, const int64_t *qr_table,
+                                const void *a, void *u, double *s, void *vh, void *workspace, int32_t *info, void *stream)
+  {
+    if (count < 0) return fail(TT_EINVAL, "a negative block count");
+    if (!ttg::complex_svd_takes(largest, largest)) return fail(TT_EINVAL, "a block of the batched SVD is too large");
+    if (qr_ranks < 1 || qr_ranks > 16 || (qr_ranks & (qr_ranks - 1)))
+      return fail(TT_EINVAL, "the batched SVD takes the cluster size tt_svd_complex_plan gave");
+    const cudaError_t e = ttg::complex_svd_blocks(count, largest, qr_ranks, table, qr_table, a, u, s, vh, workspace, info,
+                                                  static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(TT_ECUDA, std::string("CUDA: ") + cudaGetErrorString(e));
+    return TT_OK;
+  }
+
+  int32_t tt_svd_complex_keep(int32_t count, const int64_t *table, const void *u, const double *s, const void *vh, void *first,
+                              void *second, void *values, void *stream)
+  {
+    if (count < 0) return fail(TT_EINVAL, "a negative block count");
+    const cudaError_t e = ttg::complex_svd_keep(count, table, u, s, vh, first, second, values, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(TT_ECUDA, std::string("CUDA: ") + cudaGetErrorString(e));
     return TT_OK;
   }

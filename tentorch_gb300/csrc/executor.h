@@ -228,6 +228,16 @@ namespace ttg
   cudaError_t qr_blocks(int32_t count, int32_t ranks, const void *table, const void *a, void *q, void *r, void *workspace, bool complex,
                         cudaStream_t stream);
 
+  // Thin SVDs of complex128 blocks (svd_complex.cu): whether a block fits, its workspace in elements, its entry in
+  // the table of the QR factorisations (8 int64), the launches (tables in device memory) and the kept factors.
+  bool complex_svd_takes(int64_t rows, int64_t cols);
+  int64_t complex_svd_workspace(int64_t rows, int64_t cols);
+  void complex_svd_qr_entry(int64_t rows, int64_t cols, int64_t ws_off, int64_t *entry);
+  cudaError_t complex_svd_blocks(int32_t count, int64_t largest, int32_t qr_ranks, const void *table, const void *qr_table, const void *a,
+                                 void *u, double *s, void *vh, void *workspace, int32_t *info, cudaStream_t stream);
+  cudaError_t complex_svd_keep(int32_t count, const void *table, const void *u, const double *s, const void *vh, void *first,
+                               void *second, void *values, cudaStream_t stream);
+
   // The Lanczos loop of a window (lanczos.cu): `base` carries the plan's operands (the vector
   // operand's pointer is replaced by each basis vector), prepared arenas and workspace; scratch holds
   // lanczos_scratch_doubles() doubles; the normalised Ritz vector goes to `result`, the lowest Ritz

@@ -594,15 +594,14 @@ def _factor_blocks_per_block(arranged: Tensor, present, while_waiting = None):
 class _SplitLayout:
     '''What the batched SVD of the tensors of one space needs on a device, laid out once: the device table of its blocks
     and of the ranking, the places of the packed factors and the workspace in one buffer.'''
-    __slots__ = ('present', 'count', 'largest', 'blocks', 'table', 'ranking', 'n_blocks', 'n_sectors', 'sv_at', 'vh_at', 'ws_at',
-                 'values', 'size')
+    __slots__ = ('present', 'count', 'largest', 'blocks', 'table', 'order', 'qr_ranks', 'ranking', 'n_blocks', 'n_sectors', 'sv_at',
+                 'vh_at', 'ws_at', 'values', 'size')
 
-    def __init__(self, space: Space, device):
+    def __init__(self, space: Space, device, present, places, total: int, width: int, qr = None):
+        '''`places` and `total`: each block's workspace and all of it in elements, of `width` doubles; `qr` (complex128): the
+        blocks' QR table (a row a block) and the cluster size.'''
         cat = space.cat
-        self.present = [(i, key) for i, key in enumerate(space.keys) if space.shapes[i][0] * space.shapes[i][1] > 0]
-        dims, _ = ints64(x for i, _ in self.present for x in space.shapes[i])
-        places, total = (i64 * max(len(self.present), 1))(), i64()
-        check(lib.tt_svd_workspace(len(self.present), dims, places, ctypes.byref(total)))
+        self.present = present
         entries, self.blocks, ids = [], [], {}
         u_at = s_at = vh_at = 0
         for at, (i, key) in enumerate(self.present):
@@ -614,21 +613,44 @@ class _SplitLayout:
             for sector in (key.domain, cat.dual(key.domain)):
                 ids.setdefault(sector, len(ids))
         # the largest blocks first: the launch's clusters then finish together, small blocks last
-        entries.sort(key = lambda e: -min(e[1], e[2]) ** 2 * max(e[1], e[2]))
+        self.order = sorted(range(len(entries)), key = lambda at: -min(entries[at][1:3]) ** 2 * max(entries[at][1:3]))
+        rows = [x for at in self.order for x in entries[at]]
+        self.qr_ranks = 0
+        if qr is not None:
+            rows += [x for at in self.order for x in qr[0][8 * at:8 * at + 8]]
+            self.qr_ranks = qr[1]
         self.count = self.n_blocks = len(self.present)
         self.largest = max((b[3] for b in self.blocks), default = 0)
         self.n_sectors = len(ids)
         self.values = s_at
         # one buffer: U, the values, Vh, then the workspace, each from a multiple of 32 doubles
         up = lambda n: (n + 31) // 32 * 32
-        self.sv_at = up(u_at)
+        self.sv_at = up(width * u_at)
         self.vh_at = self.sv_at + up(s_at)
-        self.ws_at = self.vh_at + up(vh_at)
-        self.size = max(self.ws_at + total.value, 1)
+        self.ws_at = self.vh_at + up(width * vh_at)
+        self.size = max(self.ws_at + width * total, 1)
         # no wait for the stream's queued work (the window's Lanczos): the SVD is queued behind it
-        self.table = _uploaded([x for e in entries for x in e], torch.int64, device)
+        self.table = _uploaded(rows, torch.int64, device)
         self.ranking = _uploaded([b[3] for b in self.blocks] + [ids[b[0].domain] for b in self.blocks] +
                                  [ids[cat.dual(sector)] for sector in sorted(ids, key = ids.get)], torch.int32, device)
+
+
+def _split_layout(space: Space, device, dtype):
+    '''The layout of the batched SVD, None when some block is too large for it.'''
+    present = [(i, key) for i, key in enumerate(space.keys) if space.shapes[i][0] * space.shapes[i][1] > 0]
+    count = len(present)
+    if any(min(space.shapes[i]) > 1024 for i, _ in present):
+        return None
+    dims, _ = ints64(x for i, _ in present for x in space.shapes[i])
+    places, total = (i64 * max(count, 1))(), i64()
+    if dtype == torch.float64:
+        check(lib.tt_svd_workspace(count, dims, places, ctypes.byref(total)))
+        return _SplitLayout(space, device, present, places, total.value, 1)
+    table, ranks = (i64 * max(8 * count, 1))(), i32()
+    check(lib.tt_svd_complex_plan(count, dims, places, ctypes.byref(total), table, ctypes.byref(ranks)))
+    if count and not ranks.value:
+        return None
+    return _SplitLayout(space, device, present, places, total.value, 2, (table, ranks.value))
 
 
 class _SplitWrite:
@@ -668,7 +690,7 @@ class _SplitWrite:
         self.table = _uploaded(table, torch.int64, device)
 
 
-# (space, device) -> its split's layout (None: not for the batched SVD); (space, kept counts, absorb, device)
+# (space, device, dtype) -> its split's layout (None: not for the batched SVD); (space, kept counts, absorb, device)
 # -> where its factors go
 _split_layouts = {}
 _split_writes = {}
@@ -685,17 +707,16 @@ def _remembered(cache: dict, key, make):
 
 
 def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None):
-    """The split of float64 blocks on the GPU: one launch of the engine's Jacobi SVD for all blocks (tt_svd_blocks),
+    """The split on the GPU: the engine's Jacobi SVD for all blocks (tt_svd_blocks; complex128 tt_svd_complex_blocks),
     the ranking of the values on the device (tt_svd_rank), one read of each block's kept count with the
-    SVD's sweep counts, and one launch that writes the kept factors (tt_svd_keep).  None when the blocks are
-    not for it, False when one did not settle (then they go through at::linalg_svd one at a time)."""
+    SVD's sweep counts, and one launch that writes the kept factors (tt_svd_keep).  Blocks that did not settle
+    go through at::linalg_svd before the values are ranked again.  None when the blocks are not for it."""
     global svd_fallbacks
-    space, data = arranged._space, arranged._data
-    if not (data.dtype == torch.float64 and data.is_cuda and _precision != PER_BLOCK):
+    space, data, dtype = arranged._space, arranged._data, arranged._data.dtype
+    if not (data.is_cuda and _precision != PER_BLOCK and dtype in (torch.float64, torch.complex128)):
         return None
     device, index = data.device, data.get_device()
-    layout = _remembered(_split_layouts, (space.id, index),
-                         lambda: _SplitLayout(space, device) if all(min(s) <= 1024 for s in space.shapes if s[0] * s[1]) else None)
+    layout = _remembered(_split_layouts, (space.id, index, dtype), lambda: _split_layout(space, device, dtype))
     if layout is None:
         return None
     buffer = torch.empty(layout.size, dtype = torch.float64, device = device)
@@ -703,20 +724,33 @@ def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None
     u = buffer.data_ptr()
     sv, vh, ws = u + 8 * layout.sv_at, u + 8 * layout.vh_at, u + 8 * layout.ws_at
     info, kept_at = counts.data_ptr(), counts.data_ptr() + 4 * layout.count
-    stream = _raw_stream(index)
-    check(lib.tt_svd_blocks(layout.count, layout.largest, layout.table.data_ptr(), data.data_ptr(), u, sv, vh, ws, info, stream))
+    stream, table = _raw_stream(index), layout.table.data_ptr()
+    if dtype == torch.float64:
+        check(lib.tt_svd_blocks(layout.count, layout.largest, table, data.data_ptr(), u, sv, vh, ws, info, stream))
+    elif layout.count:
+        check(lib.tt_svd_complex_blocks(layout.count, layout.largest, layout.qr_ranks, table, table + 56 * layout.count, data.data_ptr(),
+                                        u, sv, vh, ws, info, stream))
     ranking = layout.ranking.data_ptr()
-    # the host's ranking for splits too large for the kernel
-    status = lib.tt_svd_rank(sv, layout.values, ranking, ranking + 4 * layout.n_blocks, layout.n_blocks, ranking + 8 * layout.n_blocks,
-                             layout.n_sectors, float(tol), -1 if max_bond is None else int(max_bond), kept_at, stream)
-    if status not in (0, 1):
-        check(status)
+
+    def rank():
+        # the host's ranking for splits too large for the kernel
+        status = lib.tt_svd_rank(sv, layout.values, ranking, ranking + 4 * layout.n_blocks, layout.n_blocks,
+                                 ranking + 8 * layout.n_blocks, layout.n_sectors, float(tol), -1 if max_bond is None else int(max_bond),
+                                 kept_at, stream)
+        if status not in (0, 1):
+            check(status)
+        return status
+
+    status = rank()
     if while_waiting is not None:
         while_waiting()
     host = counts.tolist() if layout.count else []
-    if layout.count and min(host[:layout.count]) < 0:
+    unsettled = [layout.order[at] for at in range(layout.count) if host[at] < 0]
+    if unsettled:
         svd_fallbacks += 1
-        return False
+        _factor_into(arranged, layout, buffer, unsettled)
+        rank()
+        host = counts.tolist()
     if status == 0:
         kept = tuple(host[layout.count:])
     else:
@@ -724,12 +758,25 @@ def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None
     write = _remembered(_split_writes, (space.id, kept, absorb, index), lambda: _SplitWrite(space, layout, kept, absorb, device))
     # (the kernel writes the pads after odd blocks)
     make = torch.empty if write.covered else torch.zeros
-    first, second, values = (make(n, dtype = torch.float64, device = device)
+    first, second, values = (make(n, dtype = dtype, device = device)
                              for n in (write.first.size, write.second.size, write.multiplets))
     if write.count:
-        check(lib.tt_svd_keep(write.count, write.table.data_ptr(), u, sv, vh, first.data_ptr(), second.data_ptr(), values.data_ptr(),
-                              stream))
+        keep = lib.tt_svd_keep if dtype == torch.float64 else lib.tt_svd_complex_keep
+        check(keep(write.count, write.table.data_ptr(), u, sv, vh, first.data_ptr(), second.data_ptr(), values.data_ptr(), stream))
     return Tensor._wrap(write.first, first), values, Tensor._wrap(write.second, second)
+
+
+def _factor_into(arranged: Tensor, layout: _SplitLayout, buffer, blocks):
+    '''at::linalg_svd of these blocks of the layout, into the packed factors.'''
+    parts = [buffer[:layout.sv_at], buffer[layout.vh_at:layout.ws_at]]
+    if arranged.dtype == torch.complex128:
+        parts = [torch.view_as_complex(p.view(-1, 2)) for p in parts]
+    for at in blocks:
+        _, rows, cols, k, u_at, s_at, vh_at = layout.blocks[at]
+        u, sv, vh = torch.linalg.svd(arranged._view(layout.present[at][0]), full_matrices = False, driver = PER_BLOCK_SVD_DRIVER)
+        parts[0][u_at:u_at + rows * k].view(rows, k).copy_(u)
+        buffer[layout.sv_at + s_at:layout.sv_at + s_at + k].copy_(sv)
+        parts[1][vh_at:vh_at + k * cols].view(k, cols).copy_(vh)
 
 
 def _ranked_on_host(arranged: Tensor, layout: _SplitLayout, values, max_bond, tol):
@@ -756,10 +803,8 @@ def _split_over(tensor: Tensor, left, max_bond, tol, absorb, while_waiting = Non
         raise ValueError(f'a bond needs at least one multiplet, got {max_bond}')
     arranged = tensor.place(left) if left is not None else tensor
     batched = _split_batched(arranged, max_bond, tol, absorb, while_waiting)
-    if batched:
+    if batched is not None:
         return batched
-    if batched is False:
-        while_waiting = None  # it has run
     present = [(i, key) for i, key in enumerate(arranged.keys()) if arranged._space.shapes[i][0] * arranged._space.shapes[i][1] > 0]
     factors, host = _factor_blocks_per_block(arranged, present, while_waiting)
     candidates, at = [], 0

@@ -76,3 +76,55 @@ def test_the_pads_after_odd_blocks_are_zero():
     for factor in (tg.svd(t, None, 0.0)[0], tg.svd(t, None, 0.0)[2]):
         blocks = sum(float(b.square().sum()) for b in factor.to_tuple()[3].values())
         assert abs(float(factor.data.square().sum()) - blocks) <= 1e-12 * blocks
+
+
+def _complex(make):
+    def block(rng, m, n):
+        re, im = (make(rng, m, n) for _ in range(2))
+        return re + 1j * im
+    return block
+
+
+def _complex_graded(rng, m, n):
+    k = min(m, n)
+    u, v = (np.linalg.qr(rng.standard_normal((x, k)) + 1j * rng.standard_normal((x, k)))[0] for x in (m, n))
+    return (u * 10.0 ** (-12 * np.arange(k) / k)) @ v.conj().T
+
+
+COMPLEX_SPECTRA = {'graded': _complex_graded, 'unstructured': _complex(SPECTRA['unstructured']),
+                   'deficient': lambda rng, m, n: _complex_graded(rng, m, max(1, min(m, n) // 3)) @ _complex_graded(rng, max(1, min(m, n) // 3), n),
+                   'equal': lambda rng, m, n: 1e-40 * np.linalg.qr(rng.standard_normal((max(m, n),) * 2) + 1j)[0][:m, :n]}
+
+
+@pytest.mark.parametrize('spectrum', COMPLEX_SPECTRA)
+@pytest.mark.parametrize('sizes', [[(1, 1), (1, 5), (2, 2), (9, 2)], [(15, 15), (16, 40), (24, 24)], [(32, 33), (31, 7)], [(33, 64), (8, 9), (64, 65)],
+                                   [(97, 96), (65, 70)], [(128, 129)], [(300, 20), (20, 160), (160, 161)]])
+def test_complex_factors_within_their_bounds(sizes, spectrum):
+    '''The complex128 kernels: one CTA up to 32 columns, clusters of 8 and (from 96) of 16, one to five registers a
+    lane and column, the most columns (160); 'equal' a spectrum of ones at a scale whose squares vanish in FP32.
+    A complex multiply-add's error is at most sqrt(8) times a real one's: 24 n eps.'''
+    rng = np.random.default_rng(len(sizes) * 1000 + sizes[0][0])
+    blocks = [COMPLEX_SPECTRA[spectrum](rng, m, n) for m, n in sizes]
+    cat = tg.su2
+    legs = [tg.Leg(cat, [(i,) for i in range(len(sizes))], [s[side] for s in sizes]) for side in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = torch.complex128, device = 'cuda')
+    for i, b in enumerate(blocks):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    cut = 1e-13 * max(np.abs(b).max() for b in blocks)
+    first, values, second = tg.svd(t, None, cut)
+    bond = first.domain[0]
+    at = 0
+    kept = dict(zip(bond.sectors, bond.multiplicities))
+    for i, b in enumerate(blocks):
+        n = max(b.shape)
+        count = kept.get((i,), 0)
+        u, v = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+        s = values[at:at + count].cpu().numpy()
+        at += count
+        want = np.linalg.svd(b, compute_uv = False)
+        scale, tol = want[0], 24 * n * EPS
+        assert np.abs(s - want[:count]).max(initial = 0.0) <= tol * scale
+        assert want[count:].max(initial = 0.0) <= cut + tol * scale
+        for q in (u.conj().T @ u, v @ v.conj().T):
+            assert np.abs(q - np.eye(count)).max(initial = 0.0) <= tol
+        assert np.abs((u * s) @ v - b).max() <= tol * scale + cut * n
