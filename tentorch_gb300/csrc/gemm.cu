@@ -784,6 +784,7 @@ namespace ttg
       const int64_t at = group_begin + blockIdx.x;
       const SplitGroup g = groups[at];
       dependent_entry();
+      dependent_release();  // to the product, which sets up its barriers and tensor memory meanwhile
       const bool left = at < groups_a;
       const int line = threadIdx.x & 7, first = threadIdx.x >> 3, runs = blockDim.x >> 3;
       const bool live = line < g.lines;

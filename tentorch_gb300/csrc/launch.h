@@ -4,6 +4,13 @@
 // set-up overlap the previous kernel's tail) and holds at griddepcontrol.wait until the previous
 // grid has completed and its writes are visible.  Every kernel launched this way calls
 // dependent_entry() before it touches global memory.
+//
+// A kernel lets the next one in as its CTAs leave (what their exit does by itself).  Let in at a kernel's
+// start, the next one's CTAs took the first SMs that came free, several to an SM, and waited there for the
+// last: the 260 CTAs that slice the second operand of the matvec of bond 1001 then ran on some 40 SMs, and
+// the matvec took 178 us instead of 142 (bond 512: 65 and 50; an environment of bond 203, complex128:
+// 114 and 107).  Only a kernel that is short and whose follower has one CTA an SM lets it in early,
+// by dependent_release().
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,6 +22,10 @@ namespace ttg
   __device__ __forceinline__ void dependent_entry()
   {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  }
+
+  __device__ __forceinline__ void dependent_release()
+  {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   }
 

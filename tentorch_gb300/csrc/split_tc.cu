@@ -24,7 +24,7 @@
 // Measured on the SU(2) recoupling of bond 8 x 9 spins (85.9 GFLOP, S = 6: 1.80 PFLOP of slice products)
 // 1.16 ms, 1.55 PFLOP/s, 0.78 of the measured bf16 peak; as 21 products of 64 columns staged by cp.async
 // from slices a row apart it took 5.99 ms.  The matvec of bond 1001 (both products and their
-// slicing) takes 178 us, 425 on mma.sync.
+// slicing) takes 142 us, 425 on mma.sync.
 // The roles pass stages, level sums and free tensor memory through mbarriers.  Every wait gives up
 // after two seconds or once another has, and raises an error flag; on every path out the copies and
 // products in flight are waited for (again with a limit) and the tensor memory is freed.
@@ -251,7 +251,6 @@ namespace ttg
       __shared__ int failed_flag, last_flag;
       volatile int *failed = &failed_flag;
       const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-      asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
       if (warp == 0)
       {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_base)) : "memory");
@@ -620,6 +619,7 @@ namespace ttg
       __syncthreads();
       if (tid == 0 && failed_flag) atomicExch(a.error, 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      dependent_release();
       if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
     }
   } // namespace
