@@ -103,7 +103,7 @@ namespace ttg
       int64_t longest = 0, n_items = 0, n_reduces = 0, first_tiles = 0, slots = 0, moved_from = 0;
       std::vector<ChainItem> host_items;  // every item, first product first, before the deal (for batches)
       std::vector<double> host_work;      // their work estimates
-    } chain;
+    } chain, chain_batch;                 // chain_batch: with 32 x 32 tiles, for a launch of several programs
 
     cudaError_t ensure(const Program &p);
     ~DeviceTables();

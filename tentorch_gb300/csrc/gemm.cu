@@ -46,7 +46,7 @@ namespace ttg
     int64_t up256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
   } // namespace
 
-  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full, bool lanes)
+  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full, bool lanes, bool whole)
   {
     GemmSchedule s;
     // The workers of one SM share its FP64 pipe, so what has to balance is the work per SM: items
@@ -91,7 +91,7 @@ namespace ttg
         {
           const double rows = std::min(bm, blk.m - m0), cols = std::min(bn, blk.n - n0);
           const double work = cost(rows, cols, static_cast<double>(ktotal));
-          int64_t chunks = std::max<int64_t>(1, static_cast<int64_t>(std::ceil(work / target)));
+          int64_t chunks = whole ? 1 : std::max<int64_t>(1, static_cast<int64_t>(std::ceil(work / target)));
           int64_t kc = (ktotal + chunks - 1) / std::max<int64_t>(chunks, 1);
           kc = std::max<int64_t>(16, (kc + 15) / 16 * 16);
           chunks = ktotal > 0 ? (ktotal + kc - 1) / kc : 1;

@@ -145,8 +145,9 @@ namespace ttg
 
   // The FP64 schedule of a GEMM op; with full = false only its sizes (items, partial slots,
   // reductions), for sizing the scratch: the items are dealt on the op's first FP64 launch.
-  // `lanes`: costed for the FMA-lane kernel (complex128) rather than DMMA fragments.
-  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full = true, bool lanes = false);
+  // `lanes`: costed for the FMA-lane kernel (complex128) rather than DMMA fragments; `whole`: no tile is
+  // cut along K.
+  GemmSchedule schedule_gemm(const Program &p, const Op &op, int bm, int bn, bool full = true, bool lanes = false, bool whole = false);
   // The partial tiles (32 x 32 doubles each) the one launch of a program's product chain may hold
   // (chain.cu; 0 without a chain).
   int64_t chain_partial_slots(const Program &p);

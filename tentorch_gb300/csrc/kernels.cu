@@ -198,6 +198,7 @@ namespace ttg
   {
     if (base) cudaFree(base);
     if (chain.base) cudaFree(chain.base);
+    if (chain_batch.base) cudaFree(chain_batch.base);
     if (chain.relabel_base) cudaFree(chain.relabel_base);
     for (std::vector<GemmTables> *tables : {&gemm, &gemm_complex})
       for (GemmTables &g : *tables)
