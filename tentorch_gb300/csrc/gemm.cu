@@ -837,12 +837,18 @@ namespace ttg
       if (live && first == 0) (left ? exps_a : exps_b)[g.exp + line] = static_cast<int16_t>(e);
       const auto cut = [&](int run, const double (&x)[8])
       {
-        // the integer plus half a unit of each of the eight digits: digit t is then a field of seven bits,
-        // 64 too large but for the first (balanced digits with all their carries taken at once)
-        constexpr long long half = 0x0001020408102040ll;  // sum over t < 7 of 2^(48 - 7 t)
+        // The first t + 1 digits are the integer rounded to nearest, halves up, at that place, so that any
+        // number of slices is as near to the entry as it can be (fields of seven bits of the integer plus
+        // half a unit of each digit, -64 to 63, are off by up to 0.504 of the last kept one); digit t is what
+        // that prefix adds to the one before, of which 32 bits suffice.
         long long r[8];
+        uint32_t prefix[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) r[j] = scaled_integer(x[j], 56 - e) + half;
+        for (int j = 0; j < 8; ++j)
+        {
+          r[j] = scaled_integer(x[j], 56 - e);
+          prefix[j] = 0;
+        }
         uint16_t *out = dst + static_cast<int64_t>(run >> 2) * g.step_stride + (run & 3) * 64;
 #pragma unroll
         for (int t = 0; t < kMaxSlices; ++t)
@@ -852,7 +858,10 @@ namespace ttg
 #pragma unroll
           for (int j = 0; j < 8; ++j)
           {
-            const int q = t == 0 ? static_cast<int>(r[j] >> 49) : static_cast<int>((r[j] >> (49 - 7 * t)) & 127) - 64;
+            const int place = 49 - 7 * t;
+            const uint32_t now = static_cast<uint32_t>((r[j] + ((1ll << place) >> 1)) >> place);
+            const int q = static_cast<int>(now - (prefix[j] << 7));
+            prefix[j] = now;
             // |q| <= 128: the fp32 of 12582912 + q holds q in its last bits, and q is exact in bf16
             const uint32_t f = __float_as_uint(__int_as_float(0x4b400000 + q) - 12582912.0f) >> 16;
             word[j >> 1] = j & 1 ? word[j >> 1] | f << 16 : f;

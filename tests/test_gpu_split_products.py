@@ -58,3 +58,30 @@ def test_one_block_within_its_bound(size, slices):
                     assert worst.max() <= 1, (forms, float(worst.max()))
         finally:
             la.clear_tuning()
+
+
+def _digits(x, axis, slices):
+    '''The first digits of x over the power of two above its lines' largest entries: each prefix is x at that place
+    rounded to nearest, halves up (the rest after it is exact in FP64).'''
+    e = _exponents(np.abs(x).max(axis, keepdims = True))
+    rest, digits = np.ldexp(x, -e), []
+    for t in range(slices):
+        digits.append(np.floor(np.ldexp(rest, 7 * (t + 1)) + 0.5))
+        rest = rest - np.ldexp(digits[-1], -7 * (t + 1))
+    return digits, e
+
+
+@pytest.mark.parametrize('slices', [1, 2, 3, 4])
+@pytest.mark.parametrize('size', [(9, 10, 33), (130, 70, 600)])
+def test_the_digits_are_the_nearest_at_every_place(size, slices):
+    '''Up to four slices every sum is an integer below 2^53, so the product is that of the digits to the last bit;
+    half the entries have 30 bits, so that many lie half way between two digits.'''
+    m, n, k = size
+    rng = np.random.default_rng(slices)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    a[:, ::2], b[::2] = (np.ldexp(np.rint(np.ldexp(x, 27)), -27) for x in (a[:, ::2], b[::2]))
+    (da, ea), (db, eb) = _digits(a, 1, slices), _digits(b, 0, slices)
+    want = np.ldexp(sum(np.ldexp(da[t] @ db[u], -7 * (t + u + 2)) for t in range(slices) for u in range(slices - t)), ea + eb)
+    with tg.precision(slices):
+        got = tg.contract(_tensor(a), _tensor(b), [1], [0]).block((0,), (0,)).cpu().numpy()
+    assert np.array_equal(got, want)
