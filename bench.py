@@ -276,7 +276,7 @@ KIND_NAMES = {0: 'memset', 1: 'gather_kernel', 2: 'runs_kernel', 3: None, 4: 'ad
 
 
 def gemm_kernel_name(precision):
-    return {0: 'gemm_dmma_kernel', -1: 'cublas_dgemm'}.get(precision, 'gemm_split_kernel')
+    return {0: 'gemm_dmma_kernel', -1: 'cublas_dgemm'}.get(precision, 'gemm_split_tc_kernel')
 
 
 def launches_of(kind, precision):
@@ -536,7 +536,7 @@ def run_gpu(args, rank, world):
         achieved = bf16_flops / (gemm_ms / 1e3) / 1e12 if gemm_ms > 0 else 0.0
         peak = peaks['bf16_tflops']
         roofline = {'bound': 'tensor', 'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s', 'frac': achieved / peak,
-                    'traffic': ncu_traffic('gemm_split_kernel'), 'kernel': 'gemm_split_kernel',
+                    'traffic': ncu_traffic('gemm_split_tc_kernel'), 'kernel': 'gemm_split_tc_kernel',
                     'peak_source': f'{peak_kind} bf16_tflops', 'kernel_ms': gemm_ms,
                     'algorithmic': f'{bf16_flops:.4g} bf16 FLOP per step ({slices}({slices}+1)/2 slice products)'}
     roofline['op_ms'] = {k: round(v, 6) for k, v in by_kind.items()}

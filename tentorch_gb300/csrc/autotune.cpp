@@ -5,9 +5,9 @@
 //
 // The forms (ExecArgs::forms bits): kFormSeparate runs a product chain (two products with a leg
 // move between them) as separate launches instead of one; kFormNoTensorCores keeps split-precision
-// products of large blocks on the mma.sync kernel instead of the tcgen05 one.  The tile shapes and
-// schedules inside each form are fixed by the form's kernel (32 x 32 FP64 tiles with K cut to about
-// six items per SM, 32 x 32 split tiles, 128 x 64 tcgen05 tiles).
+// products on the mma.sync kernel instead of the tcgen05 one.  The tile shapes and schedules inside
+// each form are chosen by the form's kernel (FP64: up to 32 x 32, chain.cu chain_tile; mma.sync 32 x 32;
+// tcgen05 128 x 64 or 128 x 32).
 //
 // The histogram: per block product of the plan, in order, the multiply-adds of its block pairs
 // binned by (log2 m, log2 n, log2 K), each bin's sum kept to a quarter octave; plus whether the plan

@@ -10,7 +10,7 @@
 // Split precision (gemm.cu): every row of A and column of B is scaled by a power of two so that
 // its entries lie in [-1, 1], then cut into `s` slices of 7 bits held exactly as bf16 integers
 // (|q_1| <= 128, |q_t| <= 64).  The products of slices are sums of integers that fp32 accumulates
-// exactly over a K-chunk of up to 256, so the only rounding is the final FP64 combination and the
+// exactly over a K-chunk (kExactChunk), so the only rounding is the final FP64 combination and the
 // truncation after s slices (about 2^-7s of the row and column maxima): Ozaki's error-free
 // splitting (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59 (2012)) on bf16
 // tensor cores with fp32 accumulation.
@@ -160,7 +160,7 @@ namespace ttg
   // The slices of a GEMM operand that is an operand's prepared value (fixed while the arena is
   // unchanged: the head and tail of a Lanczos window) are cut once, when the arena is prepared,
   // into the arena after the prepared value: kMaxSlices slices (any fewer are a prefix of them)
-  // and the exponents, laid out as the launch's scratch lays them out.
+  // and the exponents, in the order of SplitPair.
   struct SliceCache
   {
     int32_t op;       // the GEMM op

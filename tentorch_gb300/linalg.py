@@ -11,7 +11,7 @@ cached against the operand's arena and its version counter, so a loop that appli
 operator to changing vectors (the Lanczos matvec) recouples the operator once.
 
 Block products run in FP64 by default; `precision(k)` switches them to split products on the
-tensor cores with k bf16 slices per operand (see gemm_split.cu).
+tensor cores with k bf16 slices per operand (see gemm.h).
 '''
 from __future__ import annotations
 
@@ -432,7 +432,7 @@ def einsum_batch(spec: str, operand_lists, outcharge = None) -> list:
 
 # the forms a plan's block products run in (tt_autotune): bits of the integer autotune returns
 FORM_SEPARATE = 1          # a product chain (the two-site matvec) as separate launches
-FORM_NO_TENSOR_CORES = 2   # split products of large blocks on mma.sync instead of tcgen05
+FORM_NO_TENSOR_CORES = 2   # split products on mma.sync instead of tcgen05
 
 
 def histogram_key(plan: Plan) -> int:
