@@ -190,6 +190,26 @@ def _uploaded(values, dtype, device) -> torch.Tensor:
     return torch.tensor(values, dtype = dtype).pin_memory().to(device, non_blocking = True)
 
 
+class _KeptTable:
+    '''A device table that later calls use too, on whichever stream they run: one of another stream than the upload's
+    waits for the upload and is recorded with the table's memory.  (Under capture neither is needed or possible: a
+    capture begins with the device idle, and what it uses is not dropped.)'''
+    __slots__ = ('table', 'stream', 'uploaded')
+
+    def __init__(self, values, dtype, device):
+        self.table = _uploaded(values, dtype, device)
+        self.stream = _raw_stream(self.table.get_device())
+        self.uploaded = torch.cuda.Event()
+        self.uploaded.record(torch.cuda.current_stream(device))
+
+    def address(self, stream: int) -> int:
+        if stream != self.stream and not _capturing():
+            current = torch.cuda.current_stream(self.table.device)
+            current.wait_event(self.uploaded)
+            self.table.record_stream(current)
+        return self.table.data_ptr()
+
+
 def _check_device(tensors) -> None:
     dtype, device = tensors[0].dtype, tensors[0].device
     for t in tensors:
@@ -630,9 +650,9 @@ class _SplitLayout:
         self.ws_at = self.vh_at + up(width * vh_at)
         self.size = max(self.ws_at + width * total, 1)
         # no wait for the stream's queued work (the window's Lanczos): the SVD is queued behind it
-        self.table = _uploaded(rows, torch.int64, device)
-        self.ranking = _uploaded([b[3] for b in self.blocks] + [ids[b[0].domain] for b in self.blocks] +
-                                 [ids[cat.dual(sector)] for sector in sorted(ids, key = ids.get)], torch.int32, device)
+        self.table = _KeptTable(rows, torch.int64, device)
+        self.ranking = _KeptTable([b[3] for b in self.blocks] + [ids[b[0].domain] for b in self.blocks] +
+                                  [ids[cat.dual(sector)] for sector in sorted(ids, key = ids.get)], torch.int32, device)
 
 
 def _split_layout(space: Space, device, dtype):
@@ -687,7 +707,7 @@ class _SplitWrite:
             self.count += 1
         self.covered = (self.count > 0 and written[0] == sum(m * n for m, n in self.first.shapes) and
                         written[1] == sum(m * n for m, n in self.second.shapes))
-        self.table = _uploaded(table, torch.int64, device)
+        self.table = _KeptTable(table, torch.int64, device)
 
 
 # (space, device, dtype) -> its split's layout (None: not for the batched SVD); (space, kept counts, absorb, device)
@@ -700,6 +720,8 @@ def _remembered(cache: dict, key, make):
     found = cache.get(key, cache)
     if found is cache:
         found = make()
+        if _capturing():  # its uploads are part of the graph: not for other calls
+            return found
         if len(cache) >= _PLAN_BUDGET:
             cache.clear()
         cache[key] = found
@@ -724,13 +746,14 @@ def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None
     u = buffer.data_ptr()
     sv, vh, ws = u + 8 * layout.sv_at, u + 8 * layout.vh_at, u + 8 * layout.ws_at
     info, kept_at = counts.data_ptr(), counts.data_ptr() + 4 * layout.count
-    stream, table = _raw_stream(index), layout.table.data_ptr()
+    stream = _raw_stream(index)
+    table = layout.table.address(stream)
     if dtype == torch.float64:
         check(lib.tt_svd_blocks(layout.count, layout.largest, table, data.data_ptr(), u, sv, vh, ws, info, stream))
     elif layout.count:
         check(lib.tt_svd_complex_blocks(layout.count, layout.largest, layout.qr_ranks, table, table + 56 * layout.count, data.data_ptr(),
                                         u, sv, vh, ws, info, stream))
-    ranking = layout.ranking.data_ptr()
+    ranking = layout.ranking.address(stream)
 
     def rank():
         # the host's ranking for splits too large for the kernel
@@ -762,7 +785,7 @@ def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None
                              for n in (write.first.size, write.second.size, write.multiplets))
     if write.count:
         keep = lib.tt_svd_keep if dtype == torch.float64 else lib.tt_svd_complex_keep
-        check(keep(write.count, write.table.data_ptr(), u, sv, vh, first.data_ptr(), second.data_ptr(), values.data_ptr(), stream))
+        check(keep(write.count, write.table.address(stream), u, sv, vh, first.data_ptr(), second.data_ptr(), values.data_ptr(), stream))
     return Tensor._wrap(write.first, first), values, Tensor._wrap(write.second, second)
 
 
@@ -940,6 +963,8 @@ def _qr_plan(arranged: Tensor, transposed: bool):
     key = (space.id, transposed, arranged.dtype, device.index)
     if key in _qr_plans:
         return _qr_plans[key]
+    if _capturing():  # a table uploaded now would be the graph's: the blocks go one by one
+        return None
     cat = space.cat
     present = [(i, k) for i, k in enumerate(space.keys) if space.shapes[i][0] * space.shapes[i][1] > 0]
     multiplicities, offsets = {}, []
@@ -966,7 +991,7 @@ def _qr_plan(arranged: Tensor, transposed: bool):
             else:
                 entry, strides = (space.offsets[i], head, tail), (rows, cols, cols, 1, ld, 1, cols, 1)
             table += [*entry, places[at], *(strides[s] | strides[s + 1] << 32 for s in range(0, 8, 2))]
-        plan = (len(present), first, second, _uploaded(table, torch.int64, device), total.value, ranks.value)
+        plan = (len(present), first, second, _KeptTable(table, torch.int64, device), total.value, ranks.value)
     if len(_qr_plans) >= _PLAN_BUDGET and not _captured:
         _qr_plans.clear()
     _qr_plans[key] = plan
@@ -991,7 +1016,7 @@ def _qr_blocks(arranged: Tensor, transposed: bool):
     if count:
         ws = torch.empty(total, dtype = data.dtype, device = data.device)
         q, r = (out[1], out[0]) if transposed else (out[0], out[1])
-        check(lib.tt_qr_blocks(_DTYPE[data.dtype], count, ranks, table.data_ptr(), data.data_ptr(), q.data_ptr(), r.data_ptr(),
+        check(lib.tt_qr_blocks(_DTYPE[data.dtype], count, ranks, table.address(stream), data.data_ptr(), q.data_ptr(), r.data_ptr(),
                                ws.data_ptr(), stream))
     return Tensor._wrap(first, out[0]), Tensor._wrap(second, out[1])
 
