@@ -247,7 +247,7 @@ int32_t tt_qr_blocks(int32_t dtype, int32_t count, int32_t ranks, const int64_t 
  * it writes U (rows x k, row-major) at u + u_off, the k singular values in descending order at
  * s + s_off and Vh (k x cols, row-major) at vh + vh_off.  ws_off places the block's working set in
  * `workspace` (from tt_svd_workspace).  info[i] (device int32) receives the FP64 refinements or sweeps block
- * i took, -1 when they did not converge (then its factors are not to be used).  Asynchronous on
+ * i took, -1 when they did not converge or a value is not finite (then its factors are not to be used).  Asynchronous on
  * `stream`. */
 int32_t tt_svd_blocks(int32_t count, int64_t largest, const int64_t *table, const double *a, double *u, double *s,
                       double *vh, double *workspace, int32_t *info, void *stream);

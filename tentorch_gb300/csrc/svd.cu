@@ -37,7 +37,8 @@
 // the rows of W and V dealt to the ranks and the dot products of each round summed over the cluster.
 // Each sweep runs the pairs in the round-robin (circle) order.  Working sets sit in shared memory
 // when they fit (227 KB per CTA), else in the global workspace (L2 resident).  At most kMaxSweeps
-// sweeps per phase; a block whose FP64 phase did not converge reports -1 in `info` (the host raises).
+// sweeps per phase; a block whose FP64 phase did not converge, or with a value that is not finite, reports -1
+// in `info` (the host hands it to at::linalg_svd, or raises on a NaN).
 // All loops are bounded and every CTA of a cluster passes the same sequence of cluster barriers: what
 // ends a loop is the same on every rank.
 //
@@ -854,7 +855,7 @@ namespace ttg
             const float x = static_cast<float>(entry_a(i, j));
             sum = fmaf(x, x, sum);
           }
-          cn[j] = sum;
+          cn[j] = sum >= 0.0f ? sum : INFINITY;  // a NaN sorts like an infinity: the order is a permutation
         }
         __syncthreads();
         for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
@@ -890,7 +891,7 @@ namespace ttg
           double *col = colp(j);
           const double alpha = col[j];
           double beta = alpha, tau = 0.0, scale = 0.0;
-          if (xn > 0.0)
+          if (!(xn == 0.0))  // (a NaN goes on into R)
           {
             const double norm2 = fma(alpha, alpha, xn), inv = rsqrt(norm2), norm = norm2 * inv;
             const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
@@ -1338,6 +1339,10 @@ namespace ttg
         norms[j] = sqrt(sum);
       }
       __syncthreads();
+      // a NaN or an infinity in the block is in every column of W
+      bool finite = true;
+      for (int64_t j = threadIdx.x; j < k; j += blockDim.x) finite = finite && norms[j] < INFINITY;
+      if (!__syncthreads_and(finite)) sweeps_taken = -1;
       for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
       {
         int r = 0;

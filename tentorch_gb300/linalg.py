@@ -796,7 +796,11 @@ def _factor_into(arranged: Tensor, layout: _SplitLayout, buffer, blocks):
         parts = [torch.view_as_complex(p.view(-1, 2)) for p in parts]
     for at in blocks:
         _, rows, cols, k, u_at, s_at, vh_at = layout.blocks[at]
-        u, sv, vh = torch.linalg.svd(arranged._view(layout.present[at][0]), full_matrices = False, driver = PER_BLOCK_SVD_DRIVER)
+        block = arranged._view(layout.present[at][0])
+        # (LAPACK refuses such a block, cuSOLVER from three columns on; below it hands NaN values to the ranking)
+        if not bool(torch.isfinite(block).all()):
+            raise torch.linalg.LinAlgError('linalg.svd: the input matrix contained non-finite values')
+        u, sv, vh = torch.linalg.svd(block, full_matrices = False, driver = PER_BLOCK_SVD_DRIVER)
         parts[0][u_at:u_at + rows * k].view(rows, k).copy_(u)
         buffer[layout.sv_at + s_at:layout.sv_at + s_at + k].copy_(sv)
         parts[1][vh_at:vh_at + k * cols].view(k, cols).copy_(vh)
