@@ -332,15 +332,14 @@ def place(tensor: Tensor, above, below = None) -> Tensor:
 
 def place_plan(space: Space, above, below) -> Plan:
     '''The compiled plan of `place` on a tensor of this space (legs already resolved).'''
-    key = ('place', space.id, tuple(above), tuple(below))
+    above, below = tuple([int(x) for x in above]), tuple([int(x) for x in below])
+    key = ('place', space.id, above, below)
     plan = _plans.get(key)
     if plan is not None:
         return plan
-    above, below = [int(x) for x in above], [int(x) for x in below]
     a, na = ints32(above)
     b, nb = ints32(below)
-    return _plan(('place', space.id, tuple(above), tuple(below)),
-                 lambda out: lib.tt_plan_place(space.id, na, a, nb, b, out), space.cat)
+    return _plan(key, lambda out: lib.tt_plan_place(space.id, na, a, nb, b, out), space.cat)
 
 
 def conj(tensor: Tensor) -> Tensor:
@@ -364,18 +363,18 @@ def contract(left: Tensor, right: Tensor, left_legs, right_legs, charge = None) 
 
 def contract_plan(left: Space, right: Space, left_legs, right_legs, charge = None) -> Plan:
     '''The compiled plan of `contract` on tensors of these spaces.'''
+    left_legs, right_legs = tuple([int(x) for x in left_legs]), tuple([int(x) for x in right_legs])
     has = charge is not None
     q = _label(charge) if has else 0
-    plan = _plans.get(('contract', left.id, right.id, tuple(left_legs), tuple(right_legs), has, q))
+    key = ('contract', left.id, right.id, left_legs, right_legs, has, q)
+    plan = _plans.get(key)
     if plan is not None:
         return plan
-    left_legs, right_legs = [int(x) for x in left_legs], [int(x) for x in right_legs]
     la, n = ints32(left_legs)
     ra, m = ints32(right_legs)
     if n != m:
         raise ValueError(f'the two legs of a contraction must be given in pairs, got {n} and {m}')
-    return _plan(('contract', left.id, right.id, tuple(left_legs), tuple(right_legs), has, q),
-                 lambda out: lib.tt_plan_contract(left.id, right.id, n, la, ra, int(has), q, out), left.cat)
+    return _plan(key, lambda out: lib.tt_plan_contract(left.id, right.id, n, la, ra, int(has), q, out), left.cat)
 
 
 def einsum(spec: str, *tensors: Tensor, **options) -> Tensor:

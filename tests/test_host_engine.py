@@ -386,3 +386,25 @@ def test_einsum_fold_order_is_the_reference_rule():
         assert got == orc.fold_order(labels, dims), spec
         checked += 1
     assert checked == 60
+
+
+@pytest.mark.parametrize('once', [iter, lambda legs: (x for x in legs), lambda legs: map(int, legs),
+                                  lambda legs: reversed(legs[::-1]), lambda legs: [np.array(x) for x in legs]])
+def test_legs_may_be_any_iterable(once):
+    '''Legs given as a one-shot iterable (or as numpy scalars) name the same plan as a list, on a first call and on a
+    later one.'''
+    leg = tg.Leg(tg.u1, [(-1,), (0,), (1,)], [2, 3, 2])
+    a, b = (tg.Tensor(tg.u1, [leg, leg], [leg, leg], (0,), device = 'cpu')._space for _ in range(2))
+    la = tg.linalg
+    for listed_first in (False, True):
+        la.clear_plans()
+        if listed_first:
+            la.contract_plan(a, b, [2, 3], [0, 1])
+            la.place_plan(a, [0, 2], [1, 3])
+        contracted, mixed = la.contract_plan(a, b, once([2, 3]), once([0, 1])), la.contract_plan(a, b, [2, 3], once([0, 1]))
+        placed = la.place_plan(a, once([0, 2]), once([1, 3]))
+        want = la.contract_plan(a, b, [2, 3], [0, 1])
+        assert contracted.out_space is want.out_space and mixed.out_space is want.out_space
+        assert placed.out_space is la.place_plan(a, [0, 2], [1, 3]).out_space
+    with pytest.raises(ValueError, match = 'in pairs, got 1 and 2'):
+        la.contract_plan(a, b, once([2]), once([0, 1]))
