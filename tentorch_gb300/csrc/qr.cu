@@ -114,7 +114,7 @@ namespace ttg
     {
       beta = alpha;
       tau = scale = 0.0;
-      if (xn > 0.0)
+      if (!(xn == 0.0))  // (a NaN goes on into R and Q)
       {
         double norm, inv;
         root(fma(alpha, alpha, xn), norm, inv);
@@ -128,7 +128,7 @@ namespace ttg
     {
       beta = alpha;
       tau = scale = make_double2(0.0, 0.0);
-      if (xn > 0.0 || alpha.y != 0.0)
+      if (!(xn == 0.0 && alpha.y == 0.0))
       {
         double norm, inv;
         root(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn)), norm, inv);

@@ -35,3 +35,36 @@ def test_a_split_of_a_nan_raises(where, wide, columns):
     _, values, _ = tg.svd(_tensor(clean, torch.float64), None, 0.0)
     want = np.concatenate([np.linalg.svd(b, compute_uv = False) for b in clean])
     assert np.abs(values.cpu().numpy() - want).max() <= 16 * (columns + 3) * 2.0 ** -52 * want.max()
+
+
+@pytest.mark.parametrize('columns', [2, 3, 24])
+@pytest.mark.parametrize('where', [[(0, 0)], [(1, 0)], [(-1, -1)], [(1, 0), (0, -1)]])
+def test_a_complex_split_of_a_nan_raises(where, columns):
+    '''Real numbers, so that a column's head has no imaginary part to reflect.'''
+    bad = np.random.default_rng(columns).standard_normal((columns + 3, columns)) + 0j
+    for at in where:
+        bad[at] = np.nan
+    for block in (bad, bad.T.copy()):
+        with pytest.raises(torch.linalg.LinAlgError):
+            tg.svd(_tensor([block], torch.complex128), None, 0.0)
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf])
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('side', ['qr', 'rq'])
+@pytest.mark.parametrize('shape', [(4, 3), (6, 9), (40, 33)])
+def test_qr_keeps_what_is_not_finite(shape, side, dtype, bad):
+    '''At any place of the block the factors are not finite, as LAPACK's are not; with nothing to reflect before it
+    too (the columns of an identity).  The block beside it is factored as ever (8 n eps of its columns' sums).'''
+    rng = np.random.default_rng(shape[0])
+    beside = rng.standard_normal(shape)
+    for start in (rng.standard_normal(shape), np.eye(*shape)):
+        for at in [(0, 0), (1, 0), (shape[0] - 1, 0), (2, 2), (0, 1), (shape[0] - 1, shape[1] - 1)]:
+            block = start.copy()
+            block[at] = bad
+            blocks = [block, beside] if side == 'qr' else [block.T.copy(), beside.T.copy()]
+            first, second = getattr(tg, side)(_tensor(blocks, dtype))
+            one, two = first.block((0,), (0,)), second.block((0,), (0,))
+            assert not (torch.isfinite(one.abs()).all() and torch.isfinite(two.abs()).all()), at
+            got = (first.block((1,), (1,)) @ second.block((1,), (1,))).cpu().numpy()
+            assert np.abs(got - blocks[1]).max() <= 8 * max(shape) * 2.0 ** -52 * np.abs(beside).sum(0).max()
