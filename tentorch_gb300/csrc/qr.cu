@@ -11,7 +11,8 @@
 // clocks on a quarter of an SM here): column j + 1 has warp 0 and its quarter to itself, the other columns
 // go four to a warp, eight lanes each, on the other quarters, so that four dot products share their
 // three shuffled additions.  Q is formed from the unit vectors by the reflectors, the last first, each
-// rank its columns.  A block is scaled by a power of two first, so that no norm under- or overflows.
+// rank its columns.  A block is scaled by a power of two first, so that no square overflows, and a column
+// whose squares underflow all the same by one of its own (reflector.cuh).
 //
 // The site of bond 256 (18 blocks, the largest 92 x 46): 242 us for the whole call, 4661 us with one cuSOLVER
 // factorisation per block.
@@ -25,6 +26,7 @@
 
 #include "executor.h"
 #include "launch.h"
+#include "reflector.cuh"
 
 namespace ttg
 {
@@ -34,6 +36,9 @@ namespace ttg
 
     constexpr int kQrThreads = 512;
     constexpr int64_t kQrSmem = 220 * 1024;
+    // Blocks are scaled down no further than to 2^400: the squares do not overflow, and columns far below the
+    // largest entry stay in the normal range.
+    constexpr int kQrLargest = 400;
     constexpr int kQrBatch = 16;  // reflectors staged at a time while Q is formed
 
     // Entry (i, j) of the len x columns matrix, entry (i, c) of Q and entry (c, j) of R in their arenas, and
@@ -98,49 +103,6 @@ namespace ttg
     template <int G>
     __device__ __forceinline__ double2 lanes_sum(double2 v) { return make_double2(lanes_sum<G>(v.x), lanes_sum<G>(v.y)); }
 
-    // sqrt(x) and its reciprocal, each to half an ulp or so: an ulp of rsqrt in the first, largest columns
-    // doubled the error of Q R
-    __device__ __forceinline__ void root(double x, double &norm, double &inv)
-    {
-      inv = rsqrt(x);
-      norm = x * inv;
-      norm = fma(0.5 * inv, fma(-norm, norm, x), norm);
-      inv = fma(inv, fma(-norm, inv, 1.0), inv);
-    }
-
-    // dlarfg / zlarfg: H = I - tau v v^H with v_0 = 1 takes (alpha, x) to (beta, 0), beta real; v's rest is
-    // x scale, xn = |x|^2.
-    __device__ __forceinline__ void make_reflector(double alpha, double xn, double &beta, double &tau, double &scale)
-    {
-      beta = alpha;
-      tau = scale = 0.0;
-      if (!(xn == 0.0))  // (a NaN goes on into R and Q)
-      {
-        double norm, inv;
-        root(fma(alpha, alpha, xn), norm, inv);
-        const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
-        beta = -copysign(norm, alpha);
-        tau = fabs(d) * inv;                             // (beta - alpha) / beta
-        scale = 1.0 / d;
-      }
-    }
-    __device__ __forceinline__ void make_reflector(double2 alpha, double xn, double2 &beta, double2 &tau, double2 &scale)
-    {
-      beta = alpha;
-      tau = scale = make_double2(0.0, 0.0);
-      if (!(xn == 0.0 && alpha.y == 0.0))
-      {
-        double norm, inv;
-        root(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, xn)), norm, inv);
-        const double re = alpha.x + copysign(norm, alpha.x);  // alpha - beta, without cancellation
-        const double side = copysign(inv, alpha.x);           // -1 / beta
-        beta = make_double2(-copysign(norm, alpha.x), 0.0);
-        tau = make_double2(fabs(re) * inv, alpha.y * side);   // (beta - alpha) / beta
-        const double over = 1.0 / fma(re, re, alpha.y * alpha.y);
-        scale = make_double2(re * over, -alpha.y * over);     // 1 / (alpha - beta)
-      }
-    }
-
     template <typename T>
     __global__ void __launch_bounds__(kQrThreads, 1)
       qr_kernel(const QrEntry *__restrict__ table, const T *__restrict__ a, T *__restrict__ q, T *__restrict__ r, T *__restrict__ workspace)
@@ -159,7 +121,8 @@ namespace ttg
       T *qf = workspace + e.ws, *qtau = qf + static_cast<int64_t>(k) * len;  // the reflectors and their scalars
       const auto colp = [&](int c) -> T * { return own + static_cast<int64_t>(c / ranks) * len; };
 
-      // this rank's columns, and the power of two that brings the block's largest entry below one
+      // this rank's columns, and the power of two that brings the block's largest entry to at most 2^kQrLargest, a
+      // block below one up to it
       double most = 0.0;
       for (int c = rank; c < columns; c += ranks)
         for (int i = threadIdx.x; i < len; i += blockDim.x)
@@ -181,6 +144,7 @@ namespace ttg
       for (int o = 0; o < ranks; ++o) most = fmax(o == 0 ? 0.0 : most, *cluster.map_shared_rank(&big, o));
       int shift = 0;
       if (most > 0.0 && most < 1.7976931348623157e308) frexp(most, &shift);
+      if (shift > 0) shift = max(shift - kQrLargest, 0);
       const double down = ldexp(1.0, -shift / 2), down2 = ldexp(1.0, -(shift - shift / 2));  // each in range
       for (int64_t i = threadIdx.x; i < static_cast<int64_t>(mine) * len; i += blockDim.x) own[i] = scaled_by(scaled_by(own[i], down), down2);
       cluster.sync();  // every rank has read the others' maxima
@@ -188,8 +152,32 @@ namespace ttg
       // column j's reflector by one warp, xn the squared norm below its diagonal
       const auto reflect = [&](int j, double xn) {
         T *col = colp(j);
-        T beta, tau, scale;
-        make_reflector(col[j], xn, beta, tau, scale);
+        T head = col[j], beta, tau, scale;
+        double norm2 = square(head, xn), up = 1.0;
+        if (norm2 < kTinySquare)
+        {
+          double big = 0.0;
+          for (int i = j + lane; i < len; i += 32) big = fmax(big, largest(col[i]));
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+          if (big > 0.0)
+          {
+            int ex;
+            frexp(big, &ex);
+            up = ldexp(1.0, min(-ex, 1000));
+            xn = 0.0;
+            for (int i = j + 1 + lane; i < len; i += 32) xn = square(scaled_by(col[i], up), xn);
+            xn = lanes_sum<32>(xn);
+            head = scaled_by(head, up);
+            norm2 = square(head, xn);
+          }
+        }
+        make_reflector(head, xn, norm2, beta, tau, scale);
+        if (up != 1.0)
+        {
+          beta = scaled_by(beta, 1.0 / up);
+          scale = scaled_by(scale, up);
+        }
         __syncwarp();
         T *slot = vst + static_cast<int64_t>(j & 1) * len;
         for (int i = j + 1 + lane; i < len; i += 32)

@@ -45,3 +45,33 @@ def test_factors_match_lapack(sizes, side, dtype, scale):
         assert np.abs((q @ (r / 2.0 ** scale)) - want / 2.0 ** scale).max() <= tol * norm
         assert np.abs((r - wr) / 2.0 ** scale).max() <= tol * 100 * n * norm
         assert np.abs(np.tril(r, -1)).max(initial = 0) == 0
+
+
+@pytest.mark.parametrize('small', [1e-140, 1e-155, 1e-158, 1e-160, 1e-161, 1e-170, 1e-300])
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('side', ['qr', 'rq'])
+@pytest.mark.parametrize('columns', [[0], [1], [1, 2]])
+def test_columns_far_below_the_largest(columns, side, dtype, small):
+    '''Columns whose squares vanish: Q is orthonormal, and Q R reproduces each column to 8 max(m, n) eps of its own
+    entries (columnwise backward stability), the block's largest entry near 1 and near 2^1000.'''
+    rng = np.random.default_rng(columns[0] + 7)
+    blocks = []
+    for m, n in [(5, 3), (40, 33), (20, 50)]:
+        b = rng.standard_normal((m, n)) + (1j * rng.standard_normal((m, n)) if dtype.is_complex else 0)
+        b[:, columns] *= small
+        blocks.append(b)
+    blocks.append(blocks[1] * 2.0 ** 1000)
+    given = [b if side == 'qr' else b.T.copy() for b in blocks]
+    cat = tg.su2
+    legs = [tg.Leg(cat, [(i,) for i in range(len(given))], [b.shape[at] for b in given]) for at in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = dtype, device = 'cuda')
+    for i, b in enumerate(given):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    first, second = getattr(tg, side)(t)
+    for i, b in enumerate(blocks):
+        one, two = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+        q, r = (one, two) if side == 'qr' else (two.T, one.T)
+        tol = 8 * max(b.shape) * EPS
+        assert np.abs(q.conj().T @ q - np.eye(q.shape[1])).max() <= tol
+        norms = np.abs(b).sum(0)  # each column over its norm: no product leaves the normal range
+        assert (np.abs(q @ (r / norms) - b / norms).max(0) <= tol).all()
