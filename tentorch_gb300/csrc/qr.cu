@@ -82,26 +82,10 @@ namespace ttg
     __device__ __forceinline__ double2 conj_of(double2 a) { return make_double2(a.x, -a.y); }
     __device__ __forceinline__ double plus(double a, double b) { return a + b; }
     __device__ __forceinline__ double2 plus(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-    __device__ __forceinline__ double scaled_by(double a, double s) { return a * s; }
-    __device__ __forceinline__ double2 scaled_by(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-    __device__ __forceinline__ double square(double a, double c) { return fma(a, a, c); }
-    __device__ __forceinline__ double square(double2 a, double c) { return fma(a.x, a.x, fma(a.y, a.y, c)); }
-    __device__ __forceinline__ double largest(double a) { return fabs(a); }
-    __device__ __forceinline__ double largest(double2 a) { return fmax(fabs(a.x), fabs(a.y)); }
     __device__ __forceinline__ bool is_zero(double a) { return a == 0.0; }
     __device__ __forceinline__ bool is_zero(double2 a) { return a.x == 0.0 && a.y == 0.0; }
     __device__ __forceinline__ double load_l2(const double *p) { return __ldcg(p); }
     __device__ __forceinline__ double2 load_l2(const double2 *p) { return __ldcg(p); }
-
-    template <int G>
-    __device__ __forceinline__ double lanes_sum(double v)
-    {
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
-      return v;
-    }
-    template <int G>
-    __device__ __forceinline__ double2 lanes_sum(double2 v) { return make_double2(lanes_sum<G>(v.x), lanes_sum<G>(v.y)); }
 
     template <typename T>
     __global__ void __launch_bounds__(kQrThreads, 1)
@@ -152,32 +136,8 @@ namespace ttg
       // column j's reflector by one warp, xn the squared norm below its diagonal
       const auto reflect = [&](int j, double xn) {
         T *col = colp(j);
-        T head = col[j], beta, tau, scale;
-        double norm2 = square(head, xn), up = 1.0;
-        if (norm2 < kTinySquare)
-        {
-          double big = 0.0;
-          for (int i = j + lane; i < len; i += 32) big = fmax(big, largest(col[i]));
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
-          if (big > 0.0)
-          {
-            int ex;
-            frexp(big, &ex);
-            up = ldexp(1.0, min(-ex, 1000));
-            xn = 0.0;
-            for (int i = j + 1 + lane; i < len; i += 32) xn = square(scaled_by(col[i], up), xn);
-            xn = lanes_sum<32>(xn);
-            head = scaled_by(head, up);
-            norm2 = square(head, xn);
-          }
-        }
-        make_reflector(head, xn, norm2, beta, tau, scale);
-        if (up != 1.0)
-        {
-          beta = scaled_by(beta, 1.0 / up);
-          scale = scaled_by(scale, up);
-        }
+        T beta, tau, scale;
+        column_reflector(col, j, len, xn, beta, tau, scale);
         __syncwarp();
         T *slot = vst + static_cast<int64_t>(j & 1) * len;
         for (int i = j + 1 + lane; i < len; i += 32)

@@ -54,6 +54,7 @@
 #include <mutex>
 
 #include "executor.h"
+#include "reflector.cuh"
 
 namespace ttg
 {
@@ -826,8 +827,25 @@ namespace ttg
       double *v_cur = ws + lay.v0, *v_next = ws + lay.v1, *g = ws + lay.g;
       double *stage = reinterpret_cast<double *>(dynamic + kDynamicBytes - kStageBytes);
       const double *src = a + e.a_off;
-      const auto entry_a = [&](int64_t row, int64_t col) -> double
+      const auto raw = [&](int64_t row, int64_t col) -> double
       { return wide ? src[col * n + row] : src[row * n + col]; };  // row < len, col < k
+      // The block is worked on times a power of two, when its largest entry is not within 2^-30 .. 2^30 already: FP32
+      // column sums and products of four of its values then neither overflow nor vanish.  From `high`, the largest of
+      // the high words this thread has seen (integers: exponents are compared).
+      int shift = 0;
+      double unit = 1.0;
+      const auto find_unit = [&](int high) {
+        high = __reduce_max_sync(0xffffffffu, high);
+        if ((threadIdx.x & 31) == 0) rank_of[threadIdx.x >> 5] = high;
+        __syncthreads();
+        for (int w = 0; w < kSvdThreads / 32; ++w) high = max(high, rank_of[w]);
+        __syncthreads();
+        const int ex = (high >> 20) - 1022;  // the largest entry is below 2^ex; not finite from 1025 on
+        if ((ex >= -30 && ex <= 30) || ex > 1024) return;
+        shift = min(max(ex, -1000), 1000);
+        unit = ldexp(1.0, -shift);
+      };
+      const auto entry_a = [&](int64_t row, int64_t col) -> double { return raw(row, col) * unit; };
 
       // 0. Preconditioning: the columns sorted by norm, largest
       // first, and factored A P = Q R by Householder reflections; the sweeps then run on X = R^T
@@ -847,16 +865,24 @@ namespace ttg
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
         // squared column norms in FP32 (the same on every rank) and the order they give
         float *cn = reinterpret_cast<float *>(partial_raw);
-        for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
-        {
-          float sum = 0.0f;
-          for (int64_t i = 0; i < len; ++i)
+        const auto column_norms = [&] {
+          int high = 0;
+          for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
           {
-            const float x = static_cast<float>(entry_a(i, j));
-            sum = fmaf(x, x, sum);
+            float sum = 0.0f;
+            for (int64_t i = 0; i < len; ++i)
+            {
+              const double entry = entry_a(i, j);
+              high = max(high, __double2hiint(entry) & 0x7fffffff);
+              const float x = static_cast<float>(entry);
+              sum = fmaf(x, x, sum);
+            }
+            cn[j] = sum >= 0.0f ? sum : INFINITY;  // a NaN sorts like an infinity: the order is a permutation
           }
-          cn[j] = sum >= 0.0f ? sum : INFINITY;  // a NaN sorts like an infinity: the order is a permutation
-        }
+          return high;
+        };
+        find_unit(column_norms());
+        if (shift != 0) column_norms();
         __syncthreads();
         for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
         {
@@ -881,24 +907,16 @@ namespace ttg
           if (threadIdx.x == 0) qorder[c] = from;
         }
         cluster.sync();
-        // Step j: the owner of column j has made its reflector (as LAPACK's dlarfg: H = I - tau v v^T, v_0 = 1,
-        // R_jj = beta) and pushed it into every rank's shared memory; a warp per column right of j
-        // applies it.  The warp that holds column j + 1 does that column first and makes its reflector
-        // at once, so a step is one cluster barrier and one warp's chain of a dot product, the update,
-        // the norm and the scalars (the columns are dealt in turn, so that every rank has columns to the end).
+        // Step j: the owner of column j has made its reflector (reflector.cuh) and pushed it into every rank's
+        // shared memory; a warp per column right of j applies it.  The warp that holds column j + 1 does that
+        // column first and makes its reflector at once, so a step is one cluster barrier and one warp's chain of a
+        // dot product, the update, the norm and the scalars (the columns are dealt in turn, so that every rank has
+        // columns to the end).
         const auto reflect = [&](int64_t j, double xn) {
           // by one warp, xn the squared norm of column j below its diagonal
           double *col = colp(j);
-          const double alpha = col[j];
-          double beta = alpha, tau = 0.0, scale = 0.0;
-          if (!(xn == 0.0))  // (a NaN goes on into R)
-          {
-            const double norm2 = fma(alpha, alpha, xn), inv = rsqrt(norm2), norm = norm2 * inv;
-            const double d = alpha + copysign(norm, alpha);  // alpha - beta, without cancellation
-            beta = -copysign(norm, alpha);
-            tau = fabs(d) * inv;                             // (beta - alpha) / beta
-            scale = 1.0 / d;
-          }
+          double beta, tau, scale;
+          column_reflector(col, static_cast<int>(j), static_cast<int>(len), xn, beta, tau, scale);
           __syncwarp();
           double *slot = vst + (j & 1) * len;
           for (int64_t i = j + 1 + lane; i < len; i += 32)
@@ -992,6 +1010,12 @@ namespace ttg
       }
       // rows of the swept matrix, and its entries: the block (W orientation) or X = R^T
       const int64_t xl = precond ? k : len;
+      if (!precond)
+      {
+        int high = 0;
+        for (int64_t i = threadIdx.x; i < m * n; i += blockDim.x) high = max(high, __double2hiint(src[i]) & 0x7fffffff);
+        find_unit(high);
+      }
       const auto entry = [&](int64_t row, int64_t col) -> double
       { return precond ? (col <= row ? __ldcg(qf + row * len + col) : 0.0) : entry_a(row, col); };  // row < xl
 
@@ -1349,7 +1373,7 @@ namespace ttg
         const double sj = norms[j];
         for (int64_t i = 0; i < k; ++i) r += (norms[i] > sj || (norms[i] == sj && i < j)) ? 1 : 0;
         rank_of[j] = r;
-        if (rank == 0) s[e.s_off + r] = sj;
+        if (rank == 0) s[e.s_off + r] = sj * ldexp(1.0, shift);
       }
       __syncthreads();
       double *uo = u + e.u_off, *vo = vh + e.vh_off;

@@ -128,3 +128,35 @@ def test_complex_factors_within_their_bounds(sizes, spectrum):
         for q in (u.conj().T @ u, v @ v.conj().T):
             assert np.abs(q - np.eye(count)).max(initial = 0.0) <= tol
         assert np.abs((u * s) @ v - b).max() <= tol * scale + cut * n
+
+
+@pytest.mark.parametrize('scale', [-1020, -700, -200, 200, 500, 1000])
+@pytest.mark.parametrize('spectrum', SPECTRA)
+def test_blocks_far_from_one(spectrum, scale):
+    '''Blocks whose squares under- or overflow, with 2, 9, 31, 40 and 1 columns, tall and wide: the same bounds (a
+    power of two takes them to the scale of the other tests; below the normal range half a unit, 2^-1075, more).'''
+    rng = np.random.default_rng(abs(scale))
+    blocks = [SPECTRA[spectrum](rng, m, n) for m, n in [(5, 2), (9, 12), (31, 33), (50, 40), (6, 1)]]
+    scaled = [np.ldexp(b, scale - int(np.frexp(np.abs(b).max())[1])) for b in blocks]
+    blocks = [np.ldexp(b, -scale) for b in scaled]  # what the kernel is given, near one
+    cat = tg.su2
+    legs = [tg.Leg(cat, [(i,) for i in range(len(blocks))], [b.shape[at] for b in blocks]) for at in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = torch.float64, device = 'cuda')
+    for i, b in enumerate(scaled):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    first, values, second = tg.svd(t, None, float(np.ldexp(1e-13, scale)))
+    bond = first.domain[0]
+    kept, at = dict(zip(bond.sectors, bond.multiplicities)), 0
+    for i, b in enumerate(blocks):
+        n = max(b.shape)
+        count = kept.get((i,), 0)
+        u, v = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+        s = np.ldexp(values[at:at + count].cpu().numpy(), -scale)
+        at += count
+        want = np.linalg.svd(b, compute_uv = False)
+        tol, flat = 8 * n * EPS * want[0], float(np.ldexp(1.0, -1075 - scale)) if scale < 0 else 0.0
+        assert np.abs(s - want[:count]).max() <= tol + flat
+        assert want[count:].max(initial = 0.0) <= 1e-13 + tol + flat
+        for q in (u.T @ u, v @ v.T):
+            assert np.abs(q - np.eye(count)).max() <= 8 * n * EPS
+        assert np.abs((u * s) @ v - b).max() <= tol + 1e-13 * n + flat * n
