@@ -247,8 +247,8 @@ int32_t tt_qr_blocks(int32_t dtype, int32_t count, int32_t ranks, const int64_t 
  * it writes U (rows x k, row-major) at u + u_off, the k singular values in descending order at
  * s + s_off and Vh (k x cols, row-major) at vh + vh_off.  ws_off places the block's working set in
  * `workspace` (from tt_svd_workspace).  info[i] (device int32) receives the FP64 refinements or sweeps block
- * i took, -1 when they did not converge or a value is not finite (then its factors are not to be used).  Asynchronous on
- * `stream`. */
+ * i took, -1 when they did not converge or a value is not finite or vanishes beside the block (then its
+ * factors are not to be used).  Asynchronous on `stream`. */
 int32_t tt_svd_blocks(int32_t count, int64_t largest, const int64_t *table, const double *a, double *u, double *s,
                       double *vh, double *workspace, int32_t *info, void *stream);
 /* The workspace of tt_svd_blocks: for `count` blocks (host array of rows, cols per block) the
@@ -281,7 +281,7 @@ int32_t tt_svd_keep(int32_t count, const int64_t *table, const double *u, const 
  * elements in all, the table of the blocks' QR factorisations (8 int64 a block, to be copied to the device) and
  * the cluster size for those (0: some block is not for this path, nothing else is set).
  * tt_svd_complex_blocks: the 7 int64 a block of tt_svd_blocks and that table, both DEVICE arrays, in one order;
- * info[i] is -1 where block i did not settle or has a zero singular value.  Asynchronous on `stream`. */
+ * info[i] is -1 where block i did not settle or a value vanishes beside the block.  Asynchronous on `stream`. */
 int32_t tt_svd_complex_plan(int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int64_t *qr_table, int32_t *qr_ranks);
 int32_t tt_svd_complex_blocks(int32_t count, int64_t largest, int32_t qr_ranks, const int64_t *table, const int64_t *qr_table,
                               const void *a, void *u, double *s, void *vh, void *workspace, int32_t *info, void *stream);

@@ -37,8 +37,8 @@
 // the rows of W and V dealt to the ranks and the dot products of each round summed over the cluster.
 // Each sweep runs the pairs in the round-robin (circle) order.  Working sets sit in shared memory
 // when they fit (227 KB per CTA), else in the global workspace (L2 resident).  At most kMaxSweeps
-// sweeps per phase; a block whose FP64 phase did not converge, or with a value that is not finite, reports -1
-// in `info` (the host hands it to at::linalg_svd, or raises on a NaN).
+// sweeps per phase; a block whose FP64 phase did not converge, or with a value that is not finite or
+// below 1e-128 of the block, reports -1 in `info` (the host hands it to at::linalg_svd, or raises on a NaN).
 // All loops are bounded and every CTA of a cluster passes the same sequence of cluster barriers: what
 // ends a loop is the same on every rank.
 //
@@ -63,6 +63,8 @@ namespace ttg
     namespace cg = cooperative_groups;
 
     constexpr int kSvdThreads = 512;
+    constexpr int kBlockExp = 200;              // blocks are worked on with their largest entry at about 2^200
+    constexpr double kLeastSquare = 0x1p-450;   // there: columns whose squared norm is below have no direction to be trusted
     constexpr int kMaxSweeps = 40;
     constexpr int kMaxCols = 1024;              // k = min(rows, cols) of a block
     constexpr int kSvdSmemBytes = 227 * 1024;
@@ -829,9 +831,10 @@ namespace ttg
       const double *src = a + e.a_off;
       const auto raw = [&](int64_t row, int64_t col) -> double
       { return wide ? src[col * n + row] : src[row * n + col]; };  // row < len, col < k
-      // The block is worked on times a power of two, when its largest entry is not within 2^-30 .. 2^30 already: FP32
-      // column sums and products of four of its values then neither overflow nor vanish.  From `high`, the largest of
-      // the high words this thread has seen (integers: exponents are compared).
+      // The block is worked on times the power of two that brings its largest entry to about 2^kBlockExp, so that the
+      // products of four of its values that decide whether a pair is orthogonal neither overflow nor vanish for
+      // values down to 1e-128 of the largest.  From `high`, the largest of the high words this thread has seen
+      // (integers: exponents are compared).
       int shift = 0;
       double unit = 1.0;
       const auto find_unit = [&](int high) {
@@ -841,9 +844,10 @@ namespace ttg
         for (int w = 0; w < kSvdThreads / 32; ++w) high = max(high, rank_of[w]);
         __syncthreads();
         const int ex = (high >> 20) - 1022;  // the largest entry is below 2^ex; not finite from 1025 on
-        if ((ex >= -30 && ex <= 30) || ex > 1024) return;
-        shift = min(max(ex, -1000), 1000);
+        if (ex > 1024) return 0;
+        shift = max(ex - kBlockExp, -1000);
         unit = ldexp(1.0, -shift);
+        return ex;
       };
       const auto entry_a = [&](int64_t row, int64_t col) -> double { return raw(row, col) * unit; };
 
@@ -865,14 +869,14 @@ namespace ttg
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
         // squared column norms in FP32 (the same on every rank) and the order they give
         float *cn = reinterpret_cast<float *>(partial_raw);
-        const auto column_norms = [&] {
+        const auto column_norms = [&](double by) {
           int high = 0;
           for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
           {
             float sum = 0.0f;
             for (int64_t i = 0; i < len; ++i)
             {
-              const double entry = entry_a(i, j);
+              const double entry = raw(i, j) * by;
               high = max(high, __double2hiint(entry) & 0x7fffffff);
               const float x = static_cast<float>(entry);
               sum = fmaf(x, x, sum);
@@ -881,8 +885,8 @@ namespace ttg
           }
           return high;
         };
-        find_unit(column_norms());
-        if (shift != 0) column_norms();
+        const int ex = find_unit(column_norms(1.0));
+        if (ex < -30 || ex > 30) column_norms(ldexp(1.0, -max(ex, -1000)));  // the squares in FP32's range
         __syncthreads();
         for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
         {
@@ -1356,17 +1360,16 @@ namespace ttg
         if (lane == 0) partial[j] = sum;
       }
       cluster.sync();
+      bool sound = true;
       for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
       {
         double sum = 0;
         for (unsigned r = 0; r < ranks; ++r) sum += cluster.map_shared_rank(partial, r)[j];
         norms[j] = sqrt(sum);
+        // (a NaN or an infinity in the block is in every column of W; zeros need no direction)
+        sound = sound && sum < INFINITY && (sum == 0.0 || sum >= kLeastSquare);
       }
-      __syncthreads();
-      // a NaN or an infinity in the block is in every column of W
-      bool finite = true;
-      for (int64_t j = threadIdx.x; j < k; j += blockDim.x) finite = finite && norms[j] < INFINITY;
-      if (!__syncthreads_and(finite)) sweeps_taken = -1;
+      if (!__syncthreads_and(sound)) sweeps_taken = -1;
       for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
       {
         int r = 0;

@@ -8,8 +8,8 @@
 //      rotation applies), V refined in FP64 by matrix products to cosines at round-off, and the factors:
 //      X V = W = U_x S, so B P = (Q V) S U_x^H.
 // Pairs that the refinement leaves open (columns at the block's round-off) go through FP64 sweeps.  A block
-// that does not settle or has a zero singular value reports -1 in `info`; the caller factors it by
-// itself.  See svd.cu for each step's reasons.
+// that does not settle or has a singular value below 1e-128 of its largest entry reports -1 in `info`; the caller
+// factors it by itself.  See svd.cu for each step's reasons.
 //
 // Bound by latency: the QR's chain (a column at a time), the rounds of the sweeps, and FP64 multiply-adds (64
 // clocks a warp instruction on a quarter of an SM), so a block has a cluster even where one CTA could
@@ -36,6 +36,11 @@ namespace ttg
 
     constexpr int kThreads = 512;
     constexpr int kMaxSweeps = 40;
+    // Blocks are worked on with their largest entry at about 2^200, and columns whose squared norm is then below
+    // kLeastSquare (1e-128 of the block) have no direction to be trusted: products of four values neither overflow
+    // nor vanish (svd.cu).
+    constexpr int kBlockExp = 200;
+    constexpr double kLeastSquare = 0x1p-450;
     // Up to so many columns one CTA does the FP32 sweeps, without cluster barriers and remote columns, while the
     // others wait: nine 48 x 48 blocks 1144 -> 1119 us, four 64 x 64 1497 -> 1484.
     constexpr int kOneSweeper = 64;
@@ -407,7 +412,7 @@ namespace ttg
       const int32_t *order = reinterpret_cast<const int32_t *>(ws + l.order);
       void *stage = dynamic + kDynamic - kStageBytes;
       // X(row, col) = conj(R(col, row)), lower triangular
-      double scale = 1.0;  // a power of two: no square under- or overflows
+      double scale = 1.0;  // a power of two: no product under- or overflows
       const auto entry = [&](int row, int col) {
         if (col > row) return make_double2(0.0, 0.0);
         const double2 x = load2(r + static_cast<int64_t>(col) * k + row);
@@ -433,8 +438,8 @@ namespace ttg
       __syncthreads();
       int shift = 0;
       if (big > 0.0 && big < 1.7976931348623157e308) frexp(big, &shift);
-      shift = max(-1000, min(1000, shift));
-      scale = ldexp(1.0, -shift);
+      shift = max(-800, min(1000, shift));
+      scale = ldexp(1.0, -shift);  // to about one for the FP32 sweeps, then to 2^kBlockExp
       const auto column_of = [&](int i) { return ((i / ld / 4) * sweepers + rank) * 4 + i / ld % 4; };
       int taken = 0;
       if (rank < sweepers)
@@ -465,6 +470,8 @@ namespace ttg
       cluster.sync();
       taken = cluster.map_shared_rank(flags, 0)[2];
       cluster.sync();
+      shift -= kBlockExp;
+      scale = ldexp(1.0, -shift);
 
       // the refinement (svd.cu): E_rc = t e^(i phase) - h_rc / 2 with the phase of the pair's product.  Where W's
       // columns are not orthogonal to round-off after it (rank-deficient blocks), FP64 sweeps follow; V alone
@@ -667,7 +674,7 @@ namespace ttg
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) lambda[j] = sqrt(sum);
-        if (!(sum > 0.0)) refined = false;  // no direction for a zero value
+        if (!(sum >= kLeastSquare && sum < INFINITY)) refined = false;
       }
       refined = __syncthreads_and(refined);
       for (int j = threadIdx.x; j < k; j += blockDim.x)

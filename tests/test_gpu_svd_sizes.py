@@ -160,3 +160,34 @@ def test_blocks_far_from_one(spectrum, scale):
         for q in (u.T @ u, v @ v.T):
             assert np.abs(q - np.eye(count)).max() <= 8 * n * EPS
         assert np.abs((u * s) @ v - b).max() <= tol + 1e-13 * n + flat * n
+
+
+@pytest.mark.parametrize('small', [1e-30, 1e-76, 1e-80, 1e-90, 1e-120, 1e-127, 1e-150, 1e-200])
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('sizes', [(3, 2), (10, 12), (20, 30)])
+def test_values_far_below_the_largest(sizes, dtype, small):
+    '''Two blocks on a diagonal, the second `small` times the first: the squares of its columns' products vanish, and
+    its vectors are orthonormal to the same bounds (below 1e-128 the block is at::linalg_svd's).'''
+    rng = np.random.default_rng(sizes[0])
+    p, q = sizes
+    b = np.zeros((p + q, p + q), dtype = np.complex128 if dtype.is_complex else np.float64)
+    for part, n, scale in ((slice(0, p), p, 1.0), (slice(p, p + q), q, small)):
+        b[part, part] = scale * (rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if dtype.is_complex else 0))
+    cat = tg.no_symmetry
+    leg = tg.Leg(cat, [(0,)], [p + q])
+    t = tg.Tensor(cat, [leg], [leg], (0,), dtype = dtype, device = 'cuda')
+    t.block((0,), (0,)).copy_(torch.from_numpy(b))
+    first, values, second = tg.svd(t, None, 0.0)
+    u, v = (f.block((0,), (0,)).cpu().numpy() for f in (first, second))
+    s = values.cpu().numpy().real
+    count, tol = len(s), (24 if dtype.is_complex else 8) * (p + q) * EPS
+    assert count == p + q
+    for x in (u.conj().T @ u, v @ v.conj().T):
+        assert np.abs(x - np.eye(count)).max() <= tol
+    want = np.linalg.svd(b[:p, :p], compute_uv = False)
+    assert np.abs(s[:p] - want).max() <= tol * want[0]
+    assert np.abs((u * s) @ v - b).max() <= tol * want[0]
+    # Jacobi's method on the sorted, factored columns keeps the second block's values to its own scale
+    if small >= 1e-120:
+        want = np.linalg.svd(b[p:, p:] / small, compute_uv = False)
+        assert np.abs(s[p:] / small - want).max() <= tol * want[0]
