@@ -849,6 +849,11 @@ namespace ttg
           r[j] = scaled_integer(x[j], 56 - e);
           prefix[j] = 0;
         }
+        if (56 - e > kSubnormalScale)  // a line below the normal range
+        {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) r[j] *= 1ll << (56 - e - kSubnormalScale);
+        }
         uint16_t *out = dst + static_cast<int64_t>(run >> 2) * g.step_stride + (run & 3) * 64;
 #pragma unroll
         for (int t = 0; t < kMaxSlices; ++t)

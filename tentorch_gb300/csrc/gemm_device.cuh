@@ -101,13 +101,16 @@ namespace ttg
     }
 
     // __double2ll_rn(ldexp(x, k)) for |x| < 2^(56 - k) on the bits of x: the significand shifted by the
-    // exponent, rounded to nearest with ties to even (no branch: the eight entries of a thread overlap).
+    // exponent, rounded to nearest with ties to even (no branch: the eight entries of a thread overlap).  A value below
+    // 2^56 shifts down, but for k above kSubnormalScale, where x is subnormal and has fewer digits: that is left to be
+    // multiplied by 2^(k - kSubnormalScale).
+    constexpr int kSubnormalScale = 1077;
     __device__ __forceinline__ long long scaled_integer(double x, int k)
     {
       const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(x));
       const int field = static_cast<int>((bits >> 52) & 0x7ff);
       const unsigned long long mant = ((bits & 0xfffffffffffffull) | (field != 0 ? 1ull << 52 : 0ull)) << 3;
-      // x 2^k = mant 2^-down; a value below 2^56 shifts down
+      // x 2^k = mant 2^-down
       const int down = min(max(1078 - k - (field != 0 ? field : 1), 0), 62);
       const unsigned long long half = (1ull << down) >> 1;
       const unsigned long long q = (mant + (down ? half - 1ull + ((mant >> down) & 1ull) : 0ull)) >> down;

@@ -85,3 +85,22 @@ def test_the_digits_are_the_nearest_at_every_place(size, slices):
     with tg.precision(slices):
         got = tg.contract(_tensor(a), _tensor(b), [1], [0]).block((0,), (0,)).cpu().numpy()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize('slices', [1, 3, 6, 8])
+def test_lines_below_the_normal_range(slices):
+    '''Rows (and columns) whose largest entry is subnormal or just above, against factors that bring the products
+    back: the bound of one block.'''
+    rng = np.random.default_rng(slices)
+    m, n, k = 12, 10, 33
+    small, large = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    small *= 2.0 ** -np.arange(1012, 1060, 4)[:, None]
+    small[:, 5] = 0.0
+    large *= 2.0 ** 600
+    for a, b in ((small, large), (large.T.copy(), small.T.copy())):
+        want = a.astype(np.longdouble) @ b.astype(np.longdouble)
+        scale = np.ldexp(np.longdouble(1), _exponents(np.abs(a).max(1))[:, None] + _exponents(np.abs(b).max(0))[None, :])
+        bound = k * scale * (2.0 ** (-7 * slices) * (1.02 + 0.26 * (slices - 1)) + 2.0 ** -48) + 2.0 ** -52 * np.abs(want)
+        with tg.precision(slices):
+            got = tg.contract(_tensor(a), _tensor(b), [1], [0]).block((0,), (0,)).cpu().numpy()
+        assert (np.abs(got.astype(np.longdouble) - want) / bound).max() <= 1
