@@ -454,7 +454,7 @@ namespace ttg
                                   reinterpret_cast<const double *>(ptr[static_cast<size_t>(first.src2)]),
                                   reinterpret_cast<double *>(ptr[static_cast<size_t>(move.dst)]), args.precision,
                                   static_cast<char *>(args.workspace) + p.scratch_offset * esize,
-                                  static_cast<int *>(args.workspace), args.prepared, args.stream, relabel);
+                                  static_cast<int *>(args.workspace), args.prepared, args.stream, relabel, tensor_cores);
             if (e != cudaSuccess) return e;
             if (args.events && (e = cudaEventRecord(args.events[2 * i + 1], args.stream)) != cudaSuccess) return e;
             done[static_cast<size_t>(p.chain_move)] = 1;
