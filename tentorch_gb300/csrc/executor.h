@@ -188,8 +188,7 @@ namespace ttg
   void clear_chain_batches();
   // Split products on the tensor cores (split_tc.cu): whether an op's blocks are large enough that the
   // autotuner times them on mma.sync too, and the launch (slices and exponents as launch_gemm_split
-  // lays them out; partial tiles in `partial`, tickets and at their end an error flag, raised when a
-  // wait gives up, in `tickets`).
+  // lays them out; partial tiles in `partial`, tickets in `tickets`; entries become NaN when a wait gives up).
   bool split_tc_large(const Program &p, const Op &op, int32_t slices);
   cudaError_t launch_split_tc(const DeviceTables &t, size_t op_index, int32_t slices,
                               const uint16_t *sa, const uint16_t *sb, const int16_t *exps_a, const int16_t *exps_b,

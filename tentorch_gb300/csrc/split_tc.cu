@@ -26,8 +26,11 @@
 // from slices a row apart it took 5.99 ms.  The matvec of bond 1001 (both products and their
 // slicing) takes 142 us, 425 on mma.sync.
 // The roles pass stages, level sums and free tensor memory through mbarriers.  Every wait gives up
-// after two seconds or once another has, and raises an error flag; on every path out the copies and
-// products in flight are waited for (again with a limit) and the tensor memory is freed.
+// after two seconds or once another has.  The entries whose sums did not come then become NaN: a warp that
+// gave up goes on through its CTA's items without waiting, so that every barrier is met and every ticket
+// taken (a lost part says so in its ticket, and the whole tile becomes NaN), and the ticket region is left zero.
+// On every path out the copies and products in flight are waited for (again with a limit) and the tensor
+// memory is freed.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -85,8 +88,8 @@ namespace ttg
       int32_t longest;
       double *partial;
       int *tickets;
-      int *error;
     };
+    constexpr int kTcLost = 1 << 16;  // in a ticket: a part of the tile was lost (a tile has fewer parts, at most one a CTA and one)
 
     __device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -143,6 +146,17 @@ namespace ttg
       return t;
     }
 
+    // whether the phase with parity `parity` of the mbarrier at `at` is over, looked at for a while by the hardware
+    __device__ __forceinline__ bool tc_try(uint32_t at, uint32_t parity)
+    {
+      uint32_t done;
+      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                   : "=r"(done)
+                   : "r"(at), "r"(parity)
+                   : "memory");
+      return done != 0;
+    }
+
     // Wait for the phase of `bar` with parity `parity`; false when two seconds passed first, or when
     // another wait of the CTA has given up (`failed`, null to wait regardless).
     __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *failed)
@@ -151,17 +165,31 @@ namespace ttg
       unsigned long long start = 0;
       while (true)
       {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(done)
-                     : "r"(at), "r"(parity)
-                     : "memory");
-        if (done) return true;
+        if (tc_try(at, parity)) return true;
         const unsigned long long now = tc_now();
         if (start == 0) start = now;
         if ((failed && *failed) || now - start > kTcWaitNs)
         {
           if (failed) *failed = 1;
+          return false;
+        }
+      }
+    }
+
+    // The same for a whole warp, whose lanes go on together either way (a vote in the loop costs nothing against its
+    // branch; one after it 0.5% of a long product).
+    __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, volatile int *failed)
+    {
+      const uint32_t at = smem_addr(bar);
+      unsigned long long start = 0;
+      while (true)
+      {
+        if (__all_sync(0xffffffffu, tc_try(at, parity))) return true;
+        const unsigned long long now = tc_now();
+        if (start == 0) start = now;
+        if (__any_sync(0xffffffffu, *failed || now - start > kTcWaitNs))
+        {
+          *failed = 1;
           return false;
         }
       }
@@ -424,7 +452,7 @@ namespace ttg
 #pragma unroll
           for (int j = 0; j < kCols; ++j) value[j] = 0;  // also 0.0
           bool some = false;
-          ok = tc_segments(a, it, [&](const TcPair &sp, int lo, int hi) {
+          ok = ok && tc_segments(a, it, [&](const TcPair &sp, int lo, int hi) {
             long long head[kCols];
             float tail[kCols];
 #pragma unroll
@@ -435,7 +463,7 @@ namespace ttg
             }
             for (int step = lo; step < hi; step += kTcChunkSteps)
             {
-              if (!tc_wait(&sums_full, sums, failed)) return false;
+              if (!tc_wait_warp(&sums_full, sums, failed)) return false;
               sums ^= 1u;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -493,7 +521,7 @@ namespace ttg
             some = true;
             return true;
           });
-          if (!ok) break;
+          bool lost = !ok;
           if (it.slot >= 0)
           {
             // a partial tile, columns of 128 rows so that a warp writes 256 contiguous bytes; the CTA
@@ -507,14 +535,16 @@ namespace ttg
             epilogue_sync();
             if (tid == 0)
             {
-              last_flag = atomicAdd(a.tickets + it.reduce, 1) == r.nslots - 1;
+              const int mine = *failed ? 1 + kTcLost : 1, sum = atomicAdd(a.tickets + it.reduce, mine) + mine;
+              last_flag = sum % kTcLost != r.nslots ? 0 : sum < kTcLost ? 1 : 2;
               // every other part of the tile has its ticket: left zero for the next launch
               if (last_flag) a.tickets[it.reduce] = 0;
             }
             epilogue_sync();
-            const bool last = last_flag;
+            const int last = last_flag;
             epilogue_sync();
-            if (!last) continue;
+            if (last == 0) continue;
+            lost = last == 2;
             __threadfence();
             const long long *from = reinterpret_cast<const long long *>(a.partial) + static_cast<int64_t>(r.slot0) * kTcM * N +
                                     col0 * kTcM + 32 * quarter + lane;
@@ -541,6 +571,18 @@ namespace ttg
                                          : __double_as_longlong(__longlong_as_double(value[c + j]) + __longlong_as_double(x[s][j]));
               }
             }
+          }
+          if (lost)
+          {
+#pragma unroll 1
+            for (int j = 0; j < kCols; ++j)
+            {
+              int64_t at = it.c + static_cast<int64_t>(row) * it.n + it.n0 + col0 + j;
+              if (row >= it.m || it.n0 + col0 + j >= it.n) continue;
+              if (a.relabel && (at = a.relabel[at]) < 0) continue;
+              a.c[at] = __longlong_as_double(0x7ff8000000000000ll);
+            }
+            continue;
           }
           if constexpr (N != 32)
             if (single) exponents(it.ea, it.eb, row_exp, col_exp);
@@ -617,7 +659,6 @@ namespace ttg
         }
       }
       __syncthreads();
-      if (tid == 0 && failed_flag) atomicExch(a.error, 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       dependent_release();
       if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
@@ -659,8 +700,8 @@ namespace ttg
     const int w = tiles[1] <= p.ctas ? 0 : 1;
     s.n = 32 << w;
     int64_t share = std::max<int64_t>(16, (total[w] + p.ctas - 1) / p.ctas);
-    // a ticket per cut tile, and the error flag after them
-    if (tiles[w] >= kTicketInts - 1) share = INT32_MAX;
+    // a ticket per cut tile
+    if (tiles[w] > kTicketInts) share = INT32_MAX;
     struct Sized
     {
       TcItem item;
@@ -756,7 +797,7 @@ namespace ttg
     const DeviceTables::TcTables &tc = t.tc[op_index];
     const TcArgs args{sa, sb, exps_a, exps_b, C, relabel,
                       static_cast<const DevSplitPair *>(spairs), static_cast<const TcItem *>(tc.items), tc.reduces, tc.longest,
-                      partial, tickets, tickets + kTicketInts - 1};
+                      partial, tickets};
     cudaError_t e = cudaSuccess;
     switch (slices * 128 + tc.n)
     {

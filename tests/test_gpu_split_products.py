@@ -104,3 +104,22 @@ def test_lines_below_the_normal_range(slices):
         with tg.precision(slices):
             got = tg.contract(_tensor(a), _tensor(b), [1], [0]).block((0,), (0,)).cpu().numpy()
         assert (np.abs(got.astype(np.longdouble) - want) / bound).max() <= 1
+
+
+def test_a_lost_part_of_a_tile_shows_and_leaves_no_trace():
+    '''A part of K whose wait gave up marks its tile's ticket.  The mark is set here by hand, as one of several parts'
+    would be: that tile's entries become NaN and no others, the tickets are zero afterwards, and the next product
+    is right.'''
+    rng = np.random.default_rng(6)
+    ta, tb = _tensor(rng.standard_normal((100, 4000))), _tensor(rng.standard_normal((4000, 70)))
+    with tg.precision(6):
+        want = tg.contract(ta, tb, [1], [0]).block((0,), (0,)).clone()
+        (pool,) = (p for key, p in la._pools.items() if key[1] == torch.cuda.current_stream().cuda_stream and key[2] == torch.float64)
+        tickets = pool.view(torch.int32)[:16384]
+        assert int(tickets.count_nonzero()) == 0
+        tickets[1] = 1 << 16  # the second of the three tiles of 32 columns
+        lost = tg.contract(ta, tb, [1], [0]).block((0,), (0,))
+        assert int(tickets.count_nonzero()) == 0
+        assert torch.isnan(lost[:, 32:64]).all()
+        assert torch.equal(lost[:, :32], want[:, :32]) and torch.equal(lost[:, 64:], want[:, 64:])
+        assert torch.equal(tg.contract(ta, tb, [1], [0]).block((0,), (0,)), want)
