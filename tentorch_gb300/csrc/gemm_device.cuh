@@ -37,8 +37,6 @@ namespace ttg
       c.y = fma(a.x, b.y, fma(a.y, b.x, c.y));
       return c;
     }
-    __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-    __device__ __forceinline__ double2 fma_t(double2 a, double2 b, double2 c) { return cfma(a, b, c); }
     template <typename T>
     __device__ __forceinline__ T zero_t();
     template <>
@@ -116,13 +114,6 @@ namespace ttg
       const unsigned long long q = (mant + (down ? half - 1ull + ((mant >> down) & 1ull) : 0ull)) >> down;
       const long long v = static_cast<long long>(q);
       return (bits >> 63) ? -v : v;
-    }
-
-    // 2^k as a double built from its bits (k in the normal range), else through ldexp
-    __device__ __forceinline__ double pow2(int k)
-    {
-      if (k > -1023 && k < 1024) return __longlong_as_double(static_cast<long long>(k + 1023) << 52);
-      return ldexp(1.0, k);
     }
 
     // x 2^e, rounded only where the result leaves the normal range.
