@@ -119,6 +119,10 @@ namespace ttg
     // Blocks of at least this many columns are preconditioned by QR (below 32 columns, on one CTA, it
     // costs little, and the refinement needs the graded columns it leaves).
     constexpr int64_t kQrMinCols = 2;
+    // The longest columns whose reflectors one warp makes ahead of the step; longer ones are made by their CTA (one
+    // block, us, one warp against the CTA: 148 x 148 2729 and 2954, 300 x 150 3344 and 3467, 600 x 100 both 2929,
+    // 1000 x 100 4060 and 3814, 1500 x 60 2827 and 2421).
+    constexpr int64_t kAheadRows = 600;
 
     // The circle method's pair t of a round (players even, round < players - 1, t < players / 2):
     // player players - 1 stays, the others turn; p < q.  In 32-bit arithmetic with one conditional
@@ -869,24 +873,36 @@ namespace ttg
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
         // squared column norms in FP32 (the same on every rank) and the order they give
         float *cn = reinterpret_cast<float *>(partial_raw);
-        const auto column_norms = [&](double by) {
-          int high = 0;
+        int high = 0;
+        for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
+        {
+          float sum = 0.0f;
+#pragma unroll 8
+          for (int64_t i = 0; i < len; ++i)
+          {
+            const double entry = raw(i, j);
+            high = max(high, __double2hiint(entry) & 0x7fffffff);
+            const float x = static_cast<float>(entry);
+            sum = fmaf(x, x, sum);
+          }
+          cn[j] = sum >= 0.0f ? sum : INFINITY;  // a NaN sorts like an infinity: the order is a permutation
+        }
+        const int ex = find_unit(high);
+        if ((ex < -30 && ex > -1022) || ex > 30)
+        {
+          // again with the squares in FP32's range
+          const double by = ldexp(1.0, -max(ex, -1000));
           for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
           {
             float sum = 0.0f;
             for (int64_t i = 0; i < len; ++i)
             {
-              const double entry = raw(i, j) * by;
-              high = max(high, __double2hiint(entry) & 0x7fffffff);
-              const float x = static_cast<float>(entry);
+              const float x = static_cast<float>(raw(i, j) * by);
               sum = fmaf(x, x, sum);
             }
-            cn[j] = sum >= 0.0f ? sum : INFINITY;  // a NaN sorts like an infinity: the order is a permutation
+            cn[j] = sum >= 0.0f ? sum : INFINITY;
           }
-          return high;
-        };
-        const int ex = find_unit(column_norms(1.0));
-        if (ex < -30 || ex > 30) column_norms(ldexp(1.0, -max(ex, -1000)));  // the squares in FP32's range
+        }
         __syncthreads();
         for (int64_t j = threadIdx.x; j < k; j += blockDim.x)
         {
@@ -900,8 +916,9 @@ namespace ttg
         // global factored matrix); each reflector goes to the global one as it is made
         const bool qr_smem = (cpr + 2) * len * 8 <= kDynamicBytes;
         double *own = reinterpret_cast<double *>(dynamic);
-        double *vst = qr_smem ? own + cpr * len : own;  // the reflectors of two steps in turn (when they fit)
-        const bool push = qr_smem || 2 * len * 8 <= kDynamicBytes;
+        double *vst = qr_smem ? own + cpr * len : own;  // the reflectors of two steps in turn; one when columns are global
+        const bool staged = len * 8 <= kDynamicBytes;
+        const bool ahead = qr_smem && len <= kAheadRows;
         const auto colp = [&](int64_t c) -> double * { return qr_smem ? own + (c / ranks) * len : qf + c * len; };
         for (int64_t c = rank; c < k; c += ranks)
         {
@@ -911,6 +928,61 @@ namespace ttg
           if (threadIdx.x == 0) qorder[c] = from;
         }
         cluster.sync();
+        if (!ahead)
+        {
+          // Long columns, or too long for shared memory: the CTA that owns column j makes its reflector with all its
+          // threads and the others read it from L2; a warp per column applies it.  (A block of 5000 x 64 takes 8.7 ms
+          // so, 20.5 by the chain of one warp below, 10.0 with no QR ahead at all.)
+          for (int64_t j = 0; j < k; ++j)
+          {
+            if (j % ranks == rank)
+            {
+              double *col = colp(j);
+              double part = 0.0;
+              for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x) part = fma(col[i], col[i], part);
+              part = warp_sum(part);
+              if (lane == 0) norms_raw[warp] = part;
+              __syncthreads();
+              if (warp == 0)
+              {
+                double beta, tau, scale;
+                column_reflector(col, static_cast<int>(j), static_cast<int>(len), warp_sum(lane < warps ? norms_raw[lane] : 0.0), beta, tau, scale);
+                __syncwarp();
+                if (lane == 0)
+                {
+                  col[j] = beta;
+                  qtau[j] = tau;
+                  big = scale;
+                }
+              }
+              __syncthreads();
+              const double scale = big;
+              if (scale != 0.0)
+                for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x) qf[j * len + i] = col[i] * scale;
+            }
+            cluster.sync();
+            const double tau = __ldcg(qtau + j);
+            const double *v = qf + j * len;
+            if (staged && tau != 0.0)
+            {
+              for (int64_t i = j + 1 + threadIdx.x; i < len; i += blockDim.x) vst[i] = __ldcg(v + i);
+              __syncthreads();
+            }
+            const auto vi = [&](int64_t i) { return staged ? vst[i] : __ldcg(v + i); };
+            if (tau != 0.0)
+              for (int64_t c = rank + ((j + ranks - rank) / ranks + warp) * ranks; c < k; c += warps * ranks)
+              {
+                double *fc = colp(c), dot = 0.0;
+                for (int64_t i = j + 1 + lane; i < len; i += 32) dot = fma(vi(i), fc[i], dot);
+                dot = warp_sum(dot);
+                const double wt = tau * (fc[j] + dot);
+                for (int64_t i = j + 1 + lane; i < len; i += 32) fc[i] = fma(-wt, vi(i), fc[i]);
+                __syncwarp();
+                if (lane == 0) fc[j] -= wt;
+              }
+            __syncthreads();
+          }
+        }
         // Step j: the owner of column j has made its reflector (reflector.cuh) and pushed it into every rank's
         // shared memory; a warp per column right of j applies it.  The warp that holds column j + 1 does that
         // column first and makes its reflector at once, so a step is one cluster barrier and one warp's chain of a
@@ -923,13 +995,11 @@ namespace ttg
           column_reflector(col, static_cast<int>(j), static_cast<int>(len), xn, beta, tau, scale);
           __syncwarp();
           double *slot = vst + (j & 1) * len;
-          for (int64_t i = j + 1 + lane; i < len; i += 32)
+          for (int64_t i = j + 1 + lane; tau != 0.0 && i < len; i += 32)
           {
             const double x = col[i] * scale;
-            col[i] = x;
             qf[j * len + i] = x;
-            if (push)
-              for (unsigned r = 0; r < ranks; ++r) cluster.map_shared_rank(slot, r)[i] = x;
+            for (unsigned r = 0; r < ranks; ++r) cluster.map_shared_rank(slot, r)[i] = x;
           }
           if (lane == 0)
           {
@@ -939,26 +1009,21 @@ namespace ttg
             for (unsigned r = 0; r < ranks; ++r) cluster.map_shared_rank(taus, r)[j & 1] = tau;
           }
         };
-        if (rank == 0 && warp == 0)
+        if (ahead && rank == 0 && warp == 0)
         {
           const double *col = colp(0);
           double xn = 0.0;
           for (int64_t i = 1 + lane; i < len; i += 32) xn = fma(col[i], col[i], xn);
           reflect(0, warp_sum(xn));
         }
-        for (int64_t j = 0; j < k; ++j)
+        for (int64_t j = 0; ahead && j < k; ++j)
         {
           cluster.sync();
           const double *v = vst + (j & 1) * len;
-          if (!push)
-          {
-            v = qf + j * len;  // too long for shared memory: read through L2
-          }
           const double tau = taus[j & 1];
           // FP64 issue is what a step is made of (a warp instruction in 64 clocks a quarter of the SM): column
           // j + 1 has warp 0 and its quarter to itself, the others go four to a warp, eight lanes a column
           // (three shuffled additions for the four dot products instead of five each), on the other quarters.
-          const auto vi = [&](int64_t i) { return push ? v[i] : __ldcg(v + i); };
           const int64_t first = (j + 1 + ranks - 1 - rank) / ranks;  // the first local column c with c ranks + rank > j
           const bool next = (j + 1) % ranks == rank;                 // it is column j + 1
           if (warp == 0)
@@ -969,12 +1034,12 @@ namespace ttg
               if (tau != 0.0)
               {
                 double dot = 0.0;
-                for (int64_t i = j + 1 + lane; i < len; i += 32) dot = fma(vi(i), fc[i], dot);
+                for (int64_t i = j + 1 + lane; i < len; i += 32) dot = fma(v[i], fc[i], dot);
                 dot = warp_sum(dot);
                 const double wt = tau * (fc[j] + dot);
                 for (int64_t i = j + 1 + lane; i < len; i += 32)
                 {
-                  const double x = fma(-wt, vi(i), fc[i]);
+                  const double x = fma(-wt, v[i], fc[i]);
                   fc[i] = x;
                   if (i > j + 1) xn = fma(x, x, xn);
                 }
@@ -995,12 +1060,12 @@ namespace ttg
               const int64_t c = (l0 + (lane >> 3)) * ranks + rank;
               const bool live = c < k;
               double *fc = colp(live ? c : l0 * ranks + rank), dot = 0.0;
-              for (int64_t i = j + 1 + lanes; i < len; i += 8) dot = fma(vi(i), fc[i], dot);
+              for (int64_t i = j + 1 + lanes; i < len; i += 8) dot = fma(v[i], fc[i], dot);
               dot = group_sum<double, 8>(dot);
               const double head = fc[j], wt = tau * (head + dot);
               __syncwarp();
               if (!live) continue;
-              for (int64_t i = j + 1 + lanes; i < len; i += 8) fc[i] = fma(-wt, vi(i), fc[i]);
+              for (int64_t i = j + 1 + lanes; i < len; i += 8) fc[i] = fma(-wt, v[i], fc[i]);
               if (lanes == 0) fc[j] = head - wt;
             }
           }

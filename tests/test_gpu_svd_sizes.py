@@ -191,3 +191,11 @@ def test_values_far_below_the_largest(sizes, dtype, small):
     if small >= 1e-120:
         want = np.linalg.svd(b[p:, p:] / small, compute_uv = False)
         assert np.abs(s[p:] / small - want).max() <= tol * want[0]
+
+
+@pytest.mark.parametrize('spectrum', SPECTRA)
+@pytest.mark.parametrize('sizes', [[(600, 20), (601, 20)], [(9, 700), (1300, 33)], [(3200, 64), (26500, 5)]])
+def test_long_columns(sizes, spectrum):
+    '''Columns whose reflectors one warp makes ahead (to 600 entries) and whose CTA makes them, in shared memory or (3200
+    x 64) in global memory, and one too long to be staged there (26500): the bounds of the other sizes.'''
+    test_factors_within_their_bounds(sizes, spectrum)
