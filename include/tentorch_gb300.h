@@ -230,7 +230,7 @@ int32_t tt_lanczos_async(const tt_plan *plan, int32_t dtype, int32_t precision, 
  * thread-block cluster per block; replaces the per-block at::linalg_qr of svd.cpp:203-257).
  * tt_qr_plan: from the blocks' lengths and columns (host pairs) the offset in elements of each block's
  * part of the workspace, the elements in all and the cluster size for the launch (0: some block does
- * not fit a cluster's shared memory, factor it elsewhere).  tt_qr_blocks: `table` is a DEVICE array of 8
+ * not fit a cluster's shared memory, or the blocks take less time one by one: factor them elsewhere).  tt_qr_blocks: `table` is a DEVICE array of 8
  * int64 per block: the offsets in elements of the matrix (in `a`), Q, R and the workspace part, then
  * len, columns and the element strides matrix row, matrix column, Q row, Q column, R row, R column as
  * eight int32.  With k = min(len, columns), Q (len x k) and R (k x columns, zeros below its diagonal)

@@ -944,6 +944,7 @@ extern "C"
         *total += ttg::qr_workspace(shapes[2 * i], shapes[2 * i + 1]);
       }
       *ranks = ttg::qr_cluster(count, shapes, dtype == TT_DTYPE_COMPLEX128);
+      if (*ranks && !ttg::qr_pays(count, shapes, *ranks, dtype == TT_DTYPE_COMPLEX128)) *ranks = 0;
     });
   }
 

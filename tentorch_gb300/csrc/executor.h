@@ -223,6 +223,8 @@ namespace ttg
   // lengths and columns (0: some block does not fit the shared memory of the largest cluster), the
   // workspace elements of one block, and the launch (`table` a device array of 64 bytes per block).
   int32_t qr_cluster(int32_t count, const int64_t *shapes, bool complex);
+  // whether the launch takes less time than the blocks one by one
+  bool qr_pays(int32_t count, const int64_t *shapes, int32_t ranks, bool complex);
   int64_t qr_workspace(int64_t len, int64_t columns);
   cudaError_t qr_blocks(int32_t count, int32_t ranks, const void *table, const void *a, void *q, void *r, void *workspace, bool complex,
                         cudaStream_t stream);

@@ -140,7 +140,7 @@ namespace ttg
         column_reflector(col, j, len, xn, beta, tau, scale);
         __syncwarp();
         T *slot = vst + static_cast<int64_t>(j & 1) * len;
-        for (int i = j + 1 + lane; i < len; i += 32)
+        for (int i = j + 1 + lane; !is_zero(tau) && i < len; i += 32)
         {
           const T x = times(col[i], scale);
           qf[static_cast<int64_t>(j) * len + i] = x;
@@ -279,7 +279,8 @@ namespace ttg
     }
 
     // The cluster for a launch: the fewest ranks that hold every block's columns, at least 8 from 16
-    // columns on (one CTA below that) and 16 from 96, as far as the GPU can hold such clusters.
+    // columns on (one CTA below that) and 16 from 96, as far as the GPU can hold such clusters.  (Columns, of wide
+    // blocks too: 5 x 3000 takes 103 us with 16 CTAs, 885 with one.)
     template <typename T>
     int qr_ranks(int32_t count, const int64_t *shapes)
     {
@@ -314,7 +315,7 @@ namespace ttg
         }
       });
       int64_t widest = 0;
-      for (int32_t i = 0; i < count; ++i) widest = std::max(widest, std::min(shapes[2 * i], shapes[2 * i + 1]));
+      for (int32_t i = 0; i < count; ++i) widest = std::max(widest, shapes[2 * i + 1]);
       const auto fits = [&](int ranks) {
         for (int32_t i = 0; i < count; ++i)
           if (qr_elements(shapes[2 * i], shapes[2 * i + 1], ranks) * static_cast<int64_t>(sizeof(T)) > kQrSmem) return false;
@@ -329,6 +330,28 @@ namespace ttg
   int32_t qr_cluster(int32_t count, const int64_t *shapes, bool complex)
   {
     return complex ? qr_ranks<double2>(count, shapes) : qr_ranks<double>(count, shapes);
+  }
+
+  // Whether the blocks together take less time here than one after another in cuSOLVER (us, from blocks of 2 x 1 to
+  // 1300 x 80 and 5 x 20000 measured one at a time; both within some 15%).  Here a reflector costs its column's chain,
+  // by the length that is left, and the passes of 48 columns over a rank; the blocks run side by side.  One block,
+  // here and there: 92 x 46 228 and 816, 300 x 150 1277 and 1986, 450 x 200 2288 and 2629, 600 x 300 4193 and 4095,
+  // 1000 x 100 2507 and 1464, 20 x 5000 303 and 365, 5 x 20000 524 and 294; complex 300 x 150 2871 and 3187,
+  // 400 x 200 4929 and 4463.
+  bool qr_pays(int32_t count, const int64_t *shapes, int32_t ranks, bool complex)
+  {
+    double longest = 0.0, sum = 0.0, others = 85.0;
+    for (int32_t i = 0; i < count; ++i)
+    {
+      const double len = static_cast<double>(shapes[2 * i]), columns = static_cast<double>(shapes[2 * i + 1]), k = std::min(len, columns);
+      const double left = len - k / 2, passes = (columns - k / 2) / (48.0 * ranks), share = k / ranks;
+      const double t = complex ? k * (0.065 * left + 4.0 * passes + 0.2 * share + 1.5)
+                               : k * (0.0255 * left + 2.1 * passes + 0.12 * share + ranks / 32.0);
+      longest = std::max(longest, t);
+      sum += t;
+      others += complex ? 85.0 + k * (17.5 + 0.018 * k + 0.0045 * (columns - k)) : std::min(215.0, 60.0 + 8.0 * k) + k * (8.3 + 0.014 * k);
+    }
+    return 30.0 + std::max(longest, sum * ranks / device_sms()) < others;
   }
 
   int64_t qr_workspace(int64_t len, int64_t columns) { return std::min(len, columns) * (len + 1); }

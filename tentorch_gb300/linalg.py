@@ -957,7 +957,8 @@ def _split_blocks(tensor: Tensor, pieces):
 
 
 # (space, rows or columns first, dtype, device) -> the batched QR of a tensor of that space: its two
-# output spaces, the device table, workspace elements and cluster size; None where a block does not fit
+# output spaces, the device table, workspace elements and cluster size; None where a block
+# does not fit or cuSOLVER, block by block, is faster (csrc/qr.cu qr_pays)
 _qr_plans = {}
 
 
@@ -1003,7 +1004,7 @@ def _qr_plan(arranged: Tensor, transposed: bool):
 
 def _qr_blocks(arranged: Tensor, transposed: bool):
     '''Every block factored in one launch straight into the two output arenas, or None when the tensor is not on
-    a CUDA device or a block does not fit (then the blocks are factored one by one).'''
+    a CUDA device or the plan is not to (then the blocks are factored one by one).'''
     if arranged.device.type != 'cuda' or _precision == PER_BLOCK:
         return None
     plan = _qr_plan(arranged, transposed)

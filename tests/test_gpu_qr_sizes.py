@@ -75,3 +75,18 @@ def test_columns_far_below_the_largest(columns, side, dtype, small):
         assert np.abs(q.conj().T @ q - np.eye(q.shape[1])).max() <= tol
         norms = np.abs(b).sum(0)  # each column over its norm: no product leaves the normal range
         assert (np.abs(q @ (r / norms) - b / norms).max(0) <= tol).all()
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('side', ['qr', 'rq'])
+@pytest.mark.parametrize('sizes,batched', [([(1300, 80)], False), ([(1000, 20)], False), ([(5, 20000)], None), ([(20, 5000)], True),
+                                           ([(3, 1000), (15, 17), (1, 96)], True), ([(500, 60)] * 6, True)])
+def test_long_and_wide_blocks(sizes, batched, side, dtype):
+    '''Blocks that are faster in cuSOLVER go there, several side by side and wide ones (a cluster by their columns) do
+    not; by either way the bounds of the other sizes, and R within them of LAPACK's.'''
+    la = tg.linalg
+    la.clear_plans()
+    test_factors_match_lapack(sizes, side, dtype, 0)
+    if batched is not None and side == 'qr':
+        (plan,) = la._qr_plans.values()
+        assert (plan is not None) == batched
