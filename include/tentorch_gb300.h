@@ -281,7 +281,8 @@ int32_t tt_svd_keep(int32_t count, const int64_t *table, const double *u, const 
  * elements in all, the table of the blocks' QR factorisations (8 int64 a block, to be copied to the device) and
  * the cluster size for those (0: some block is not for this path, nothing else is set).
  * tt_svd_complex_blocks: the 7 int64 a block of tt_svd_blocks and that table, both DEVICE arrays, in one order;
- * info[i] is -1 where block i did not settle or a value vanishes beside the block.  Asynchronous on `stream`. */
+ * info[i] is -1 where block i did not settle or a value vanishes beside the block, -2 where it is right but for zero
+ * values, whose vectors on the side of the columns sorted and factored are zero.  Asynchronous on `stream`. */
 int32_t tt_svd_complex_plan(int32_t count, const int64_t *shapes, int64_t *offsets, int64_t *total, int64_t *qr_table, int32_t *qr_ranks);
 int32_t tt_svd_complex_blocks(int32_t count, int64_t largest, int32_t qr_ranks, const int64_t *table, const int64_t *qr_table,
                               const void *a, void *u, double *s, void *vh, void *workspace, int32_t *info, void *stream);

@@ -8,8 +8,9 @@
 //      rotation applies), V refined in FP64 by matrix products to cosines at round-off, and the factors:
 //      X V = W = U_x S, so B P = (Q V) S U_x^H.
 // Pairs that the refinement leaves open (columns at the block's round-off) go through FP64 sweeps.  A block
-// that does not settle or has a singular value below 1e-128 of its largest entry reports -1 in `info`; the caller
-// factors it by itself.  See svd.cu for each step's reasons.
+// that does not settle or has a singular value below 1e-128 of its largest entry reports -1 in `info`, and -2 where all
+// is well but for values that are zero and have no direction on one side; the caller factors the first by itself, the
+// second only when it keeps zeros.  See svd.cu for each step's reasons.
 //
 // Bound by latency: the QR's chain (a column at a time), the rounds of the sweeps, and FP64 multiply-adds (64
 // clocks a warp instruction on a quarter of an SM), so a block has a cluster even where one CTA could
@@ -663,6 +664,7 @@ namespace ttg
         taken = kMaxSweeps - left;
       }
       // the values and their order, then the factors: U_x = W / sigma and L = Q V
+      bool zero = false;
       for (int j = warp; j < k; j += warps)
       {
         double sum = 0.0;
@@ -674,9 +676,11 @@ namespace ttg
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) lambda[j] = sqrt(sum);
-        if (!(sum >= kLeastSquare && sum < INFINITY)) refined = false;
+        if (sum == 0.0) zero = true;  // no direction, and none needed where the value is not kept
+        else if (!(sum >= kLeastSquare && sum < INFINITY)) refined = false;
       }
       refined = __syncthreads_and(refined);
+      zero = __syncthreads_or(zero);
       for (int j = threadIdx.x; j < k; j += blockDim.x)
       {
         int above = 0;
@@ -710,7 +714,7 @@ namespace ttg
             else u[e.u_off + static_cast<int64_t>(row) * k + rank_of[c]] = sum;
           });
       }
-      if (threadIdx.x == 0 && rank == 0) info[block] = refined ? taken : -1;
+      if (threadIdx.x == 0 && rank == 0) info[block] = !refined ? -1 : zero ? -2 : taken;
       // no CTA leaves while another may still read its shared memory
       cluster.sync();
     }

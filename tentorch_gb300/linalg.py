@@ -767,7 +767,8 @@ def _split_batched(arranged: Tensor, max_bond, tol, absorb, while_waiting = None
     if while_waiting is not None:
         while_waiting()
     host = counts.tolist() if layout.count else []
-    unsettled = [layout.order[at] for at in range(layout.count) if host[at] < 0]
+    # (-2: complete but for the vectors of zero values, which a tolerance below zero alone keeps)
+    unsettled = [layout.order[at] for at in range(layout.count) if host[at] < 0 and not (host[at] == -2 and tol >= 0)]
     if unsettled:
         svd_fallbacks += 1
         _factor_into(arranged, layout, buffer, unsettled)

@@ -199,3 +199,43 @@ def test_long_columns(sizes, spectrum):
     '''Columns whose reflectors one warp makes ahead (to 600 entries) and whose CTA makes them, in shared memory or (3200
     x 64) in global memory, and one too long to be staged there (26500): the bounds of the other sizes.'''
     test_factors_within_their_bounds(sizes, spectrum)
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.complex128])
+@pytest.mark.parametrize('sizes', [[(2, 2), (1, 3)], [(16, 31), (24, 24)], [(64, 65), (100, 90)]])
+def test_zero_values_need_no_second_factorisation(sizes, dtype):
+    '''Blocks of zeros but for a corner, and zero blocks: the kernels' own factors, none handed on, with the bounds of
+    the other sizes; a tolerance below zero keeps the zeros, with orthonormal vectors in complex128 as at::linalg_svd
+    gives them.'''
+    rng = np.random.default_rng(sizes[0][0])
+    blocks, cat = [], tg.su2
+    for m, n in sizes:
+        b = np.zeros((m, n), dtype = np.complex128 if dtype.is_complex else np.float64)
+        h = min(m, n) // 2
+        b[:h, :h] = rng.standard_normal((h, h)) + (1j * rng.standard_normal((h, h)) if dtype.is_complex else 0)
+        blocks.append(b)
+    legs = [tg.Leg(cat, [(i,) for i in range(len(sizes))], [s[side] for s in sizes]) for side in (0, 1)]
+    t = tg.Tensor(cat, [legs[0]], [legs[1]], (0,), dtype = dtype, device = 'cuda')
+    for i, b in enumerate(blocks):
+        t.block((i,), (i,)).copy_(torch.from_numpy(b))
+    before = tg.linalg.svd_fallbacks
+    for tol in (0.0, -1.0) if dtype.is_complex else (0.0,):
+        first, values, second = tg.svd(t, None, tol)
+        kept = dict(zip(first.domain[0].sectors, first.domain[0].multiplicities))
+        at = 0
+        for i, b in enumerate(blocks):
+            count, bound = kept.get((i,), 0), (24 if dtype.is_complex else 8) * max(b.shape) * EPS
+            want = np.linalg.svd(b, compute_uv = False)
+            assert count == (min(b.shape) if tol < 0 else min(b.shape) // 2)
+            if count == 0:
+                continue
+            u, v = first.block((i,), (i,)).cpu().numpy(), second.block((i,), (i,)).cpu().numpy()
+            s = values[at:at + count].cpu().numpy().real
+            at += count
+            scale = max(want[0], 1e-300)
+            assert np.abs(s - want[:count]).max() <= bound * scale
+            for q in (u.conj().T @ u, v @ v.conj().T):
+                assert np.abs(q - np.eye(count)).max() <= bound
+            assert np.abs((u * s) @ v - b).max() <= bound * scale
+        if tol >= 0:
+            assert tg.linalg.svd_fallbacks == before
