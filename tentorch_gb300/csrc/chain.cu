@@ -107,7 +107,10 @@ namespace ttg
     // 96/9 44.0 and 21.5, 128/17 43.8 and 25.4, 160/13 52.4 and 31.1, 200/17 54.1 and 44.7, 230/17 56.3 and
     // 54.1; from bond 256 (67.6) on smaller tiles are level (16 x 16 whole for the first product: 68.7, bond 240
     // 1.6 faster) or slower.  The lines lie where two neighbours' gains cross (53e3: 16 x 32 cut for the
-    // second product gains 1.9 us at 52.5e3 and loses 8.2 at 58.3e3).  The windows of a
+    // second product gains 1.9 us at 52.5e3 and loses 8.2 at 58.3e3).  A product that has tiles enough, two of 32 x 32
+    // an SM, or hardly any K, whose tiles are all staging and storing, only gets more of them from smaller ones: the
+    // environments' first product, with the site (K of 1 to 3), took the update of bond 512/5 from 393 to 522 us with
+    // 8 x 16, and takes 388 so; 256/9 135, 195 and 130; 110/9 65, 69 and 60.  The windows of a
     // batch fill the SMs together and keep 32 x 32 (64 of them 6.35 ms, 6.45 with these).
     struct ChainTile
     {
@@ -118,7 +121,7 @@ namespace ttg
     {
       if (batch) return {kChainTile, kChainTile, false};
       double work = 0;
-      int64_t longest = 0;
+      int64_t longest = 0, tiles = 0;
       for (int64_t b = op.begin; b < op.begin + op.count; ++b)
       {
         const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
@@ -126,8 +129,10 @@ namespace ttg
         for (int32_t q = 0; q < blk.pair_count; ++q) k += p.gemm_pairs[static_cast<size_t>(blk.pair_begin + q)].k;
         work += static_cast<double>(blk.m) * blk.n * static_cast<double>(k);
         longest = std::max(longest, k);
+        tiles += static_cast<int64_t>((blk.m + kChainTile - 1) / kChainTile) * ((blk.n + kChainTile - 1) / kChainTile);
       }
       work /= p.ctas;
+      if (longest < 8 || tiles > 2 * static_cast<int64_t>(p.ctas)) return {kChainTile, kChainTile, false};
       if (work < 4e3) return {8, 8, longest <= 80};
       if (longest <= 128)
       {
