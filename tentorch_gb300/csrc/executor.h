@@ -83,6 +83,7 @@ namespace ttg
       void *items = nullptr;
       GemmReduce *reduces = nullptr;
       int32_t n_ctas = 0, longest = 0, n = 0;
+      bool padding[2] = {};  // the tiles are mostly padding, for mma.sync: up to six slices, seven and eight
     };
     std::vector<GemmTables> gemm, gemm_complex;
     std::vector<SplitTables> split;

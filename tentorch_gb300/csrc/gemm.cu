@@ -1220,6 +1220,23 @@ namespace ttg
       tc.n_ctas = ts.ctas;
       tc.longest = ts.longest;
       tc.n = ts.n;
+      // Products of one step of K whose tiles do not go by it but by their end: a 128 x 64 tile takes an SM about
+      // 10.5 us (22 with the FP64 sums of seven and eight slices), a 32 x 32 one on mma.sync 3.65 (3.1), so blocks of
+      // few rows and many columns, a tile mostly padding, run there: 8 x 30000 x 3 with six slices 36 us, 51 on
+      // tcgen05 (eight: 38 and 86); 30000 x 8 x 3 44 and 32, 4000 x 4000 x 16 375 and 141 (eight: 313 and 295).
+      // Up to a tile an SM both are latency.
+      int64_t tiles = 0, small = 0;
+      for (int64_t b = op.begin; b < op.begin + op.count; ++b)
+      {
+        const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
+        tiles += static_cast<int64_t>((blk.m + kSliceTileA - 1) / kSliceTileA) * ((blk.n + ts.n - 1) / ts.n);
+        small += static_cast<int64_t>((blk.m + kSplitTileM - 1) / kSplitTileM) * ((blk.n + kSplitTileN - 1) / kSplitTileN);
+      }
+      if (s.longest_line <= kSplitStepK && tiles > p.ctas)
+      {
+        tc.padding[0] = 3.65 * small < 10.5 * tiles;
+        tc.padding[1] = 3.1 * small < 22.0 * tiles;
+      }
       const cudaError_t e = staging.commit(&dst.base);
       if (e != cudaSuccess) return e;
       dst.ready = true;
@@ -1307,7 +1324,7 @@ namespace ttg
       const char *v = std::getenv("TENTORCH_GB300_TCGEN05");
       return !(v && v[0] == '0');
     }();
-    if (tc_enabled && tensor_cores)
+    if (tc_enabled && tensor_cores && !t.tc[op_index].padding[slices > 6])
       return launch_split_tc(t, op_index, slices, sa, sb, exps_a, exps_b, sched.pairs, C, partial, ticket_region, relabel,
                              stream);
     int *tickets = ticket_region;

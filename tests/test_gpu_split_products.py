@@ -123,3 +123,10 @@ def test_a_lost_part_of_a_tile_shows_and_leaves_no_trace():
         assert torch.isnan(lost[:, 32:64]).all()
         assert torch.equal(lost[:, :32], want[:, :32]) and torch.equal(lost[:, 64:], want[:, 64:])
         assert torch.equal(tg.contract(ta, tb, [1], [0]).block((0,), (0,)), want)
+
+
+@pytest.mark.parametrize('slices', [1, 6, 7, 8])
+@pytest.mark.parametrize('size', [(8, 20001, 3), (20001, 8, 3), (33, 11000, 32), (2100, 2100, 5), (8, 20001, 33)])
+def test_products_of_one_step_of_K(size, slices):
+    '''Many tiles of one step of K, on either kernel by their shape: the bound of one block.'''
+    test_one_block_within_its_bound(size, slices)
