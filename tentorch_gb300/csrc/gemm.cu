@@ -320,6 +320,24 @@ namespace ttg
       return up256(2 * s.slice_a) + up256(2 * s.slice_b) + up256(2 * s.exps) + split_partial_bytes(s, tc) +
              up256(4 * (static_cast<int64_t>(s.reduces.size()) + 1));
     }
+    // The complex128 tile of an op: 32 x 32 where such tiles are many beside their K.  A tile has its first copies, its
+    // sums' meeting and its claim for itself, which with a short K is most of its time; with a long K and few tiles an
+    // SM's share is too coarse.  Measured (us, 16 x 16 and 32 x 32): 4000 x 4000 x 4 879 and 498, x 16 2117 and 1668, x 128
+    // 13391 and 13084; 1000 x 1000 x 16 135 and 121, x 32 241 and 233, x 64 443 and 454; 30000 x 8 x 3 32 and 20;
+    // 300 x 300 x 16 19 and 24; the environment of bond 256/17 144, 144 and 135 by this line.
+    int lanes_tile(const Program &p, const Op &op)
+    {
+      int64_t tiles = 0, longest = 0;
+      for (int64_t b = op.begin; b < op.begin + op.count; ++b)
+      {
+        const GemmBlock &blk = p.gemm_blocks[static_cast<size_t>(b)];
+        int64_t k = 0;
+        for (int32_t q = 0; q < blk.pair_count; ++q) k += p.gemm_pairs[static_cast<size_t>(blk.pair_begin + q)].k;
+        longest = std::max(longest, k);
+        tiles += static_cast<int64_t>((blk.m + 2 * kLanesTile - 1) / (2 * kLanesTile)) * ((blk.n + 2 * kLanesTile - 1) / (2 * kLanesTile));
+      }
+      return tiles >= p.ctas * std::max<int64_t>(10, longest) / 5 ? 2 * kLanesTile : kLanesTile;
+    }
     // bytes of FP64 scratch: partial tiles (`entry` bytes an entry), tickets
     int64_t f64_bytes(const GemmSchedule &s, int tile, int entry)
     {
@@ -365,7 +383,8 @@ namespace ttg
       // here only its scratch
       need = std::max(need, (f64_bytes(plans->f64[i], kF64TileM, 8) + 7) / 8);
       // complex arenas count elements of 16 bytes
-      need = std::max(need, (f64_bytes(schedule_gemm(p, op, kLanesTile, kLanesTile, false, true), kLanesTile, 16) + 15) / 16);
+      const int lanes = lanes_tile(p, op);
+      need = std::max(need, (f64_bytes(schedule_gemm(p, op, lanes, lanes, false, true), lanes, 16) + 15) / 16);
       // a chain's one launch holds the partial tiles of both its products at once
       if (static_cast<int32_t>(i) == p.chain_second)
       {
@@ -483,21 +502,21 @@ namespace ttg
     // FP64 / complex128
     // ---------------------------------------------------------------------------------------
 
-    // Persistent: kF64Workers workers of 128 threads, each computing 16 x 16 tiles over a K range on FP64
+    // Persistent: kF64Workers workers of 128 threads, each computing 16 x 16 (lanes_tile: or 32 x 32) tiles over a K range on FP64
     // FMA lanes.  A complex multiply-add is four FP64 ones and a warp's FP64 instruction takes 64 clocks
     // on a quarter of an SM, so what counts is that no lane works on padding and none waits for copies:
     //   - a tile's live entries times R phases of K (R a power of two, as many as fill the worker's 1024
     //     slots, at most the 16 K of a step) are dealt to the threads, eight independent chains each at most,
     //     and the phases of an entry summed at the end (a 10 x 10 block as 32 x 32 padded entries spent ten
-    //     times its multiply-adds); 32 x 32 tiles over 32 of K would hold an SM for 32 us and do not balance
+    //     times its multiply-adds); 32 x 32 tiles over 32 of K hold an SM for 32 us, and few do not balance
     //     (the Fibonacci recoupling of 16 multiplets, all full tiles, takes 3.97 ms with them and 3.85 with
     //     16 x 16);
     //   - K advances through two shared stages, the next one's cp.async in flight during a step.
     // The three products of an environment update at bond 203 (13 charges) take 19, 42 and 26 us; with
     // padded 32 x 32 tiles and one synchronous stage 70, 94 and 66.
-    constexpr int kLanesK = 16, kLanesPer = 8, kLanesPitch = kLanesTile + 1;
+    constexpr int kLanesK = 16, kLanesPer = 8;
     constexpr int kLanesSlots = kLanesPer * kWorkerThreads;
-    constexpr int kLanesBytes = kF64Workers * (2 * 2 * kLanesK * kLanesPitch + kLanesSlots) * 16;
+    constexpr int lanes_bytes(int tile) { return kF64Workers * (2 * 2 * kLanesK * (tile + 1) + kLanesSlots) * 16; }
 
     __device__ __forceinline__ void copy16(double2 *dst, const double2 *src, bool in)
     {
@@ -505,6 +524,7 @@ namespace ttg
       asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
     }
 
+    template <int Tile>
     __global__ void __launch_bounds__(kF64Workers * kWorkerThreads, 1)
       gemm_c128_kernel(const double2 *__restrict__ A, const double2 *__restrict__ B, double2 *__restrict__ C,
                        const DevBlock *__restrict__ blocks, const DevPair *__restrict__ pairs,
@@ -512,7 +532,7 @@ namespace ttg
                        int64_t n_reduces, double2 *__restrict__ partial, int *__restrict__ tickets)
     {
       dependent_entry();
-      constexpr int BM = kLanesTile, BN = kLanesTile, BK = kLanesK, P = kLanesPitch;
+      constexpr int BM = Tile, BN = Tile, BK = kLanesK, P = Tile + 1;
       extern __shared__ __align__(16) unsigned char smem_raw[];
       const int worker = threadIdx.x / kWorkerThreads, lt = threadIdx.x % kWorkerThreads;
       double2 *stage_base = reinterpret_cast<double2 *>(smem_raw) + static_cast<int64_t>(worker) * (2 * 2 * BK * P + kLanesSlots);
@@ -1115,7 +1135,8 @@ namespace ttg
       std::lock_guard<std::mutex> lock(t.mutex);
       DeviceTables::GemmTables &dst = (complex ? t.gemm_complex : t.gemm)[op_index];
       if (dst.ready) return cudaSuccess;
-      const int tile = complex ? kLanesTile : kF64TileM;
+      const int tile = complex ? lanes_tile(p, p.ops[op_index]) : kF64TileM;
+      dst.tile = tile;
       const GemmSchedule s = schedule_gemm(p, p.ops[op_index], tile, tile, true, complex);
 
       dst.n_items = static_cast<int64_t>(s.items.size());
@@ -1152,7 +1173,7 @@ namespace ttg
     cudaError_t e = cudaSuccess;
     if (sched.n_reduces > kTicketInts)
     {
-      tickets = reinterpret_cast<int *>(base + up256(sched.slots * (complex ? kLanesTile * kLanesTile * 16 : kF64TileM * kF64TileN * 8)));
+      tickets = reinterpret_cast<int *>(base + up256(sched.slots * sched.tile * sched.tile * (complex ? 16 : 8)));
       if ((e = cudaMemsetAsync(tickets, 0, static_cast<size_t>(sched.n_reduces) * 4, stream)) != cudaSuccess) return e;
     }
     // one CTA per list the schedule dealt, as many workers as its longest list needs (at most four)
@@ -1160,10 +1181,12 @@ namespace ttg
     const int workers = static_cast<int>(std::clamp<int64_t>(sched.longest, 1, kF64Workers));
     if (complex)
     {
-      const int bytes = std::max<int>(kLanesBytes, kPinBytes);
-      static std::once_flag once;
-      if ((e = configure(gemm_c128_kernel, bytes, once)) != cudaSuccess) return e;
-      e = launch_dependent(gemm_c128_kernel, grid, workers * kWorkerThreads, bytes, stream,
+      const bool large = sched.tile != kLanesTile;
+      const auto kernel = large ? gemm_c128_kernel<2 * kLanesTile> : gemm_c128_kernel<kLanesTile>;
+      const int bytes = std::max<int>(lanes_bytes(sched.tile), kPinBytes);
+      static std::once_flag once[2];
+      if ((e = configure(kernel, bytes, once[large])) != cudaSuccess) return e;
+      e = launch_dependent(kernel, grid, workers * kWorkerThreads, bytes, stream,
                            static_cast<const double2 *>(A), static_cast<const double2 *>(B), static_cast<double2 *>(C), blocks,
                            pairs, static_cast<const GemmItem *>(sched.items), static_cast<const int32_t *>(sched.cta_begin),
                            static_cast<const GemmReduce *>(sched.reduces), sched.n_reduces, static_cast<double2 *>(partial),
