@@ -1,6 +1,6 @@
 // Grouped block-pair GEMM for sm_103a: balanced work schedules, the persistent FP64 / complex128
 // kernels, the slicing pass of split precision, and its mma.sync kernel, the form beside the tcgen05 one
-// (split_tc.cu) that the autotuner may pick.  See gemm.h for the numerical scheme.
+// (split_tc.cu) for blocks whose tiles there would be padding, and one that the autotuner may pick.  See gemm.h for the numerical scheme.
 //
 // Both GEMM kernels are persistent: one CTA per SM, held there by its shared-memory request, split
 // into independent workers of 128 threads that claim work items from a list sorted largest first
